@@ -225,20 +225,53 @@ __device__ __forceinline__ float3 fg_walls(const FgScene &S, float3 p, float3 v)
  * One candidate of ProcessCellForcesD (K_DeviceFunctions.cu:82-100):
  * contact when |q - p| < mind, force (k*lg - kd*dot(n, vq - vp)) * n with
  * n = (q - p)/lg. */
+__device__ __forceinline__ bool fg_contact_near(float3 p, float4 q, float mind, float3 &r, float &lg)
+{
+    r = make_float3(q.x - p.x, q.y - p.y, q.z - p.z);
+    lg = sqrtf(r.x * r.x + r.y * r.y + r.z * r.z);
+    return lg < mind;
+}
+/* the force of a candidate in contact: c n */
+__device__ __forceinline__ float fg_contact_force(float3 r, float lg, float3 vp, float4 vq, float k, float kd,
+                                                  float3 &n)
+{
+    const float inv = 1.0f / lg;
+    n = make_float3(r.x * inv, r.y * inv, r.z * inv);
+    return k * lg - kd * (n.x * (vq.x - vp.x) + n.y * (vq.y - vp.y) + n.z * (vq.z - vp.z));
+}
 __device__ __forceinline__ void fg_contact(float3 &acc, float3 p, float3 vp, float4 q, float4 vq, float mind,
                                            float k, float kd)
 {
-    float rx = q.x - p.x, ry = q.y - p.y, rz = q.z - p.z;
-    float lg = sqrtf(rx * rx + ry * ry + rz * rz);
-    if (lg < mind) {
-        float inv = 1.0f / lg;
-        float nx = rx * inv, ny = ry * inv, nz = rz * inv;
-        float c = k * lg - kd * (nx * (vq.x - vp.x) + ny * (vq.y - vp.y) + nz * (vq.z - vp.z));
-        acc.x += c * nx;
-        acc.y += c * ny;
-        acc.z += c * nz;
+    float3 r, n;
+    float lg;
+    if (fg_contact_near(p, q, mind, r, lg)) {
+        const float c = fg_contact_force(r, lg, vp, vq, k, kd, n);
+        acc.x += c * n.x;
+        acc.y += c * n.y;
+        acc.z += c * n.z;
     }
 }
+
+/* Cells marked near a rigid sphere: a hashed bit table over cells 1.25
+ * contact distances wide.  A sphere marks its own and the 26 cells around, so
+ * a particle in an unmarked cell is out of contact with every sphere (bits
+ * shared by hashing only mark more).  The quarter cell to spare covers the
+ * rounding of cell indices below 2^20; beyond, everything counts as near. */
+__device__ __forceinline__ bool fg_near_cell(float x, float y, float z, float inv, int &cx, int &cy, int &cz)
+{
+    const float a = x * inv, b = y * inv, c = z * inv;
+    cx = __float2int_rd(a);
+    cy = __float2int_rd(b);
+    cz = __float2int_rd(c);
+    return fabsf(a) < 1048576.f && fabsf(b) < 1048576.f && fabsf(c) < 1048576.f;
+}
+__device__ __forceinline__ uint32_t fg_near_bit(int cx, int cy, int cz, uint32_t scene, uint32_t mask)
+{
+    uint32_t h = (uint32_t)cx * FG_PX ^ (uint32_t)cy * FG_PY ^ (uint32_t)cz * FG_PZ ^ scene * 0x9e3779b1u;
+    h ^= h >> 15;
+    return h & mask;
+}
+__device__ __forceinline__ float fg_near_inv(float mind) { return 1.0f / (1.25f * mind); }
 
 /* float atomics on the ordered-int encoding (for bounding boxes) */
 __device__ __forceinline__ int fg_float_ord(float f)

@@ -232,6 +232,14 @@ bool Capacity::too_large() const
            rb_buckets >= 0x7fffffffULL;
 }
 
+/* Bits of the near-sphere table for a number of spheres: a body's surface
+ * marks about one cell per two to four spheres, so at 64 bits a sphere some
+ * 1% of them are set. */
+static uint32_t near_bits(uint64_t spheres)
+{
+    return 1u << std::min<uint32_t>(24u, std::max<uint32_t>(15u, ceil_log2(std::max<uint64_t>(spheres, 1) * 64)));
+}
+
 /* Device bytes reserve(c) allocates (list capacity `list_cap` slots). */
 size_t World::footprint(const Capacity &c, uint32_t list_cap)
 {
@@ -247,6 +255,7 @@ size_t World::footprint(const Capacity &c, uint32_t list_cap)
     b += sizeof(FgWork) * (std::max<uint64_t>(c.work, 1) + std::max<uint64_t>(c.work_sph, 1));
     if (c.bodies) {
         b += P * 16; /* the fluid side of the contact */
+        b += near_bits(c.spheres) / 8;
         b += S * (16 * 6 + 12);
         b += 8 * std::max<uint64_t>(c.rb_buckets, 1);
         b += c.bodies * (32 * 6 + 16 * 3 + 8 + 72 + 12 + 8 * 8 * FG_BODY_CHUNKS);
@@ -314,6 +323,8 @@ int World::reserve(const Capacity &c)
         const size_t S = std::max<uint64_t>(c.spheres, 1), B = c.bodies;
         const size_t RB = std::max<uint64_t>(c.rb_buckets, 1);
         if ((r = A((void **)&fcontact, 16 * N))) return r;
+        near_mask = near_bits(c.spheres) - 1u;
+        if ((r = A((void **)&near, (near_mask + 1u) / 8u))) return r;
         if ((r = A((void **)&rb_local, 16 * S))) return r;
         if ((r = A((void **)&rb_world, 16 * S))) return r;
         if ((r = A((void **)&rb_keys_u, 4 * S))) return r;
@@ -597,12 +608,14 @@ Launch World::sphere_launch() const
     return L;
 }
 
-/* Ordered-int AABB reset: mins to +big, maxes to -big. */
-__global__ void k_aabb_reset(int *aabb, uint32_t ns)
+/* Ordered-int AABB reset: mins to +big, maxes to -big; near-sphere bits to 0. */
+__global__ void k_aabb_reset(int *aabb, uint32_t ns, uint32_t *near, uint32_t words)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < 6 * ns) aabb[i] = (i % 6) < 3 ? fg_float_ord(3.0e38f) : fg_float_ord(-3.0e38f);
+    if (i < words) near[i] = 0u;
 }
+
 
 /* Rigid-sphere grid of every scene: AABB, world positions and keys, sort,
  * start/end (the stage bit FG_STAGE_RB_GRID). */
@@ -612,8 +625,9 @@ void World::enqueue_rb_grid(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches
     if (ev) cudaEventRecord(ev[8], st);
     Launch Ls = sphere_launch();
     Ls.stream = st;
-    k_aabb_reset<<<(6 * nscenes + 127) / 128, 128, 0, st>>>(aabb, nscenes);
-    launch_hash_with_offset(Ls, rb_local, bxf, bqf, rb_world, rb_keys_u, nullptr, aabb);
+    const uint32_t words = (near_mask + 1u) / 32u;
+    k_aabb_reset<<<(std::max(6 * nscenes, words) + 127) / 128, 128, 0, st>>>(aabb, nscenes, near, words);
+    launch_hash_with_offset(Ls, rb_local, bxf, bqf, rb_world, rb_keys_u, nullptr, aabb, near, near_mask);
     if (rb_small_scenes) {
         launch_rb_sort_ranges(single ? nullptr : scenes_d, &scenes_h[0], nscenes, rb_keys_u, rb_world, rb_keys,
                               rb_ids, rb_spos, rb_start, rb_end, st);
@@ -639,6 +653,8 @@ RigidGrid World::body_grid() const
     G.end = rb_end;
     G.body_vel = bvf;
     G.aabb = aabb;
+    G.near = near;
+    G.near_mask = near_mask;
     return G;
 }
 

@@ -112,6 +112,8 @@ struct World {
     bool order_refresh_due(uint64_t s) const;
     /* rigid */
     float4 *rb_local = nullptr, *rb_world = nullptr, *rb_spos = nullptr, *rb_force = nullptr, *rb_torque = nullptr;
+    uint32_t *near = nullptr; /* bit table of the cells near a sphere */
+    uint32_t near_mask = 0;   /* its bits - 1 */
     float4 *fcontact = nullptr; /* per sorted fluid particle: its contact with the bodies' spheres */
     uint32_t *rb_keys_u = nullptr, *rb_keys = nullptr, *rb_ids = nullptr, *rb_start = nullptr, *rb_end = nullptr;
     int *aabb = nullptr;

@@ -82,7 +82,7 @@ void launch_hash(const Launch &L, const float4 *pos, uint32_t *keys, uint32_t *i
 /* CalcHashKeyWithOffsetK (K_HashGrid.cu:43-63): world = conj(q)*p*q + cm of
  * the sphere's body (w = body index), key of the world position in the
  * rigid grid.  Optionally grows the per-scene AABB of sphere centres (six
- * ordered ints: min xyz, max xyz). */
+ * ordered ints: min xyz, max xyz) and marks the cells near each sphere. */
 __global__ void __launch_bounds__(FG_CHUNK) k_hash_offset(const FgWork *__restrict__ work, uint32_t nwork,
                                                          uint32_t n_single, const FgScene *__restrict__ table,
                                                          const __grid_constant__ FgScene single,
@@ -90,7 +90,8 @@ __global__ void __launch_bounds__(FG_CHUNK) k_hash_offset(const FgWork *__restri
                                                          const float4 *__restrict__ cm,
                                                          const float4 *__restrict__ q, float4 *__restrict__ world,
                                                          uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
-                                                         int *__restrict__ aabb)
+                                                         int *__restrict__ aabb, uint32_t *__restrict__ near,
+                                                         uint32_t near_mask)
 {
     for (uint32_t w = blockIdx.x; w < nwork; w += gridDim.x) {
         FgWork it = fg_work(work, w, n_single);
@@ -110,6 +111,24 @@ __global__ void __launch_bounds__(FG_CHUNK) k_hash_offset(const FgWork *__restri
             world[i] = a;
             keys[i] = S->rb_bucket_base + fg_hash(a.x, a.y, a.z, S->rb_cell, S->rb_nb, S->rb_nb_mask);
             if (ids) ids[i] = i;
+            if (near) {
+                int cx, cy, cz;
+                const float mind = S->fluid_radius + S->rb_radius + S->fluid_eps;
+                fg_near_cell(a.x, a.y, a.z, fg_near_inv(mind), cx, cy, cz);
+                /* neighbouring spheres mark the same cells: look, a plane of
+                 * nine at once, before the atomics (a stale look costs one) */
+                for (int z = -1; z <= 1; z++) {
+                    uint32_t h[9], old[9];
+#pragma unroll
+                    for (int o = 0; o < 9; o++) {
+                        h[o] = fg_near_bit(cx + o % 3 - 1, cy + o / 3 - 1, cz + z, it.scene, near_mask);
+                        old[o] = __ldcg(near + (h[o] >> 5));
+                    }
+#pragma unroll
+                    for (int o = 0; o < 9; o++)
+                        if (!(old[o] >> (h[o] & 31u) & 1u)) atomicOr(near + (h[o] >> 5), 1u << (h[o] & 31u));
+                }
+            }
         }
         if (aabb) {
             /* warp-reduce then one atomic per warp per bound */
@@ -135,11 +154,11 @@ __global__ void __launch_bounds__(FG_CHUNK) k_hash_offset(const FgWork *__restri
 }
 
 void launch_hash_with_offset(const Launch &L, const float4 *local, const float4 *cm, const float4 *q, float4 *world,
-                             uint32_t *keys, uint32_t *ids, int *aabb)
+                             uint32_t *keys, uint32_t *ids, int *aabb, uint32_t *near, uint32_t near_mask)
 {
     if (!L.nwork) return;
     k_hash_offset<<<grid_for(L.nwork, 16), FG_CHUNK, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, local,
-                                                                    cm, q, world, keys, ids, aabb);
+                                                                    cm, q, world, keys, ids, aabb, near, near_mask);
 }
 
 /* ----------------------------------------------------------- radix sort

@@ -31,7 +31,9 @@ uint32_t grid_for(uint32_t nwork, int ctas_per_sm);
 void launch_hash(const Launch &L, const float4 *pos, uint32_t *keys, uint32_t *ids, uint32_t *cnt = nullptr,
                  uint32_t *off = nullptr);
 void launch_hash_with_offset(const Launch &L, const float4 *local, const float4 *cm, const float4 *q,
-                             float4 *world, uint32_t *keys, uint32_t *ids, int *aabb /* 6 ints per scene or null */);
+                             float4 *world, uint32_t *keys, uint32_t *ids, int *aabb /* 6 ints per scene or null */,
+                             uint32_t *near = nullptr /* bit table to mark, zeroed by the caller */,
+                             uint32_t near_mask = 0);
 
 /* keys per radix tile (one CTA of the upsweep/downsweep); the histogram
  * holds 256 counts per tile plus 256 digit totals */
@@ -142,11 +144,14 @@ struct RigidGrid {
     const uint32_t *end;
     const float4 *body_vel; /* per-body velocity (float); null = static grid */
     const int *aabb;        /* per scene ordered-int AABB of sphere centres, or null */
+    const uint32_t *near;   /* bit table of the cells near a sphere (fg_near_bit), or null */
+    uint32_t near_mask;     /* its bits - 1 */
     int own_geometry;       /* 1: bucket count below (bucket base 0); 0: the scene's rigid grid */
     uint32_t nb, mask;
     /* the force pass: each fluid particle's contact with this grid, by
      * particle id, written by launch_fluid_contact for the particles inside
-     * the bodies' grown AABB; null = the force pass walks the grid itself */
+     * the bodies' grown AABB and marked near a sphere; null = the force pass
+     * walks the grid itself */
     const float4 *pre;
 };
 
@@ -162,8 +167,9 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
 
 /* The fluid side of the fluid/rigid contact as its own pass, over the
  * unsorted particles: for every active fluid particle of a scene with bodies
- * that lies inside the bodies' AABB grown by the contact distance, out[id] =
- * its contact with grid G (ProcessCollisionForcesD).  The force pass then
+ * that lies inside the bodies' AABB grown by the contact distance and in a
+ * cell marked near a sphere (G.near), out[id] = its contact with grid G
+ * (ProcessCollisionForcesD).  The force pass then
  * reads it (G.pre). */
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out);
 

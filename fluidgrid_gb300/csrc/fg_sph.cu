@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces(const FgWork *__r
                 float3 c = make_float3(0.f, 0.f, 0.f);
                 if (!R.dyn.pre) {
                     c = fg_fluid_rigid_contact(S, it.scene, p, v, R.dyn, true);
-                } else if (!fg_contact_outside(S, it.scene, p, R.dyn)) {
+                } else if (!fg_contact_outside(S, it.scene, p, R.dyn) && fg_contact_marked(S, it.scene, p, R.dyn)) {
                     const float4 q = R.dyn.pre[ord.tord ? pid : __ldg(ids + i)];
                     c = make_float3(q.x, q.y, q.z);
                 }
@@ -345,11 +345,18 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
 /* The fluid side of the fluid/rigid contact ahead of the force pass, by
  * particle id from the step's unsorted positions and velocities (the sorted
  * copies hold the same bits), so it runs right after the rigid-sphere grid
- * beside the fluid hash and sort.  Inside the force pass, the few particles
- * near a body walked (2r+1)^3 rigid buckets while the rest of their warps and
- * CTAs waited at 80 registers a thread.  The force pass adds the stored sum
- * where it added the walked one: the same bits. */
-__global__ void __launch_bounds__(FG_CHUNK) k_fluid_contact(const FgWork *__restrict__ work, uint32_t nwork,
+ * beside the fluid hash and sort.  The particles inside the bodies' AABB and
+ * in a cell marked near a sphere (a shell around the bodies' surfaces) search
+ * the rigid grid, a warp each: the pass is bound by the latency of those
+ * searches, and a lane's own chain of 25 bucket rows and about 55 spheres,
+ * diverging from its neighbours', takes as long as dozens of searches by
+ * warp.  The CTA's eight warps share the searches of its 128 particles, which
+ * ids along a surface may all need.  4M particles, eight bodies whose AABB is
+ * the whole scene: 1007 -> 151 us (a lane each inside the AABB -> here; a lane
+ * each in marked cells only: 399; a warp per eight particles: 235).  The force
+ * pass adds the stored sum where it would add the walked one: the same bits. */
+#define FG_CONTACT_THREADS 256u
+__global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWork *__restrict__ work, uint32_t nwork,
                                                            uint32_t n_single, const FgScene *__restrict__ table,
                                                            const __grid_constant__ FgScene single,
                                                            const float4 *__restrict__ pos,
@@ -357,24 +364,42 @@ __global__ void __launch_bounds__(FG_CHUNK) k_fluid_contact(const FgWork *__rest
                                                            const __grid_constant__ RigidGrid G,
                                                            float4 *__restrict__ out)
 {
+    __shared__ uint32_t s_id[FG_CHUNK], s_n;
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t w = blockIdx.x; w < nwork; w += gridDim.x) {
         const FgWork it = fg_work(work, w, n_single);
-        if (threadIdx.x >= it.count) continue;
         const FgScene *S = fg_scene(table, &single, it.scene);
-        if (!(S->flags & FG_SCENE_HAS_RB)) continue;
-        const uint32_t id = it.first + threadIdx.x;
-        const float4 p = pos[id];
-        if (!(p.w > 0.0f) || fg_contact_outside(S, it.scene, p, G)) continue;
-        const float3 c = fg_fluid_rigid_contact(S, it.scene, p, vel[id], G, true);
-        out[id] = make_float4(c.x, c.y, c.z, 0.0f);
+        if (!(S->flags & FG_SCENE_HAS_RB)) continue; /* uniform over the CTA */
+        if (threadIdx.x == 0) s_n = 0u;
+        __syncthreads();
+        if (threadIdx.x < FG_CHUNK) {
+            const uint32_t id = it.first + threadIdx.x;
+            bool walk = false;
+            if (threadIdx.x < it.count) {
+                const float4 p = __ldg(pos + id);
+                walk = p.w > 0.0f && !fg_contact_outside(S, it.scene, p, G) && fg_contact_marked(S, it.scene, p, G);
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, walk);
+            uint32_t base = 0u;
+            if (lane == 0u && m) base = atomicAdd(&s_n, (uint32_t)__popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (walk) s_id[base + __popc(m & ((1u << lane) - 1u))] = id;
+        }
+        __syncthreads();
+        for (uint32_t k = threadIdx.x >> 5; k < s_n; k += FG_CONTACT_THREADS / 32u) {
+            const uint32_t id = s_id[k];
+            const float3 c = fg_contact_warp(S, __ldg(pos + id), __ldg(vel + id), G, true);
+            if (lane == 0u) out[id] = make_float4(c.x, c.y, c.z, 0.0f);
+        }
+        __syncthreads();
     }
 }
 
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out)
 {
     if (!L.nwork) return;
-    k_fluid_contact<<<grid_for(L.nwork, 16), FG_CHUNK, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos,
-                                                                     vel, G, out);
+    k_fluid_contact<<<grid_for(L.nwork, 8), FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table,
+                                                                              *L.single, pos, vel, G, out);
 }
 
 /* SPHIntegrateK (K_FluidSim.cu:418-438): pos += vel*(dt/scale) for active

@@ -241,8 +241,14 @@ __device__ __forceinline__ float3 fg_fluid_rigid_contact(const FgScene *S, uint3
     auto visit = [&](uint32_t st, uint32_t en) {
         for (uint32_t j = st; j < en; j++) {
             const float4 q = __ldg(G.spos + j);
+            float3 r, n;
+            float lg;
+            if (!fg_contact_near(P, q, mind, r, lg)) continue;
             const float4 vq = dynamic ? __ldg(G.body_vel + (int)q.w) : make_float4(0.f, 0.f, 0.f, 0.f);
-            fg_contact(acc, P, V, q, vq, mind, S->ck, S->ckd);
+            const float c = fg_contact_force(r, lg, V, vq, S->ck, S->ckd, n);
+            acc.x += c * n.x;
+            acc.y += c * n.y;
+            acc.z += c * n.z;
         }
     };
     if (rx >= 0 && rx <= FG_CONTACT_ROW_MAX) {
@@ -285,6 +291,102 @@ __device__ __forceinline__ float3 fg_fluid_rigid_contact(const FgScene *S, uint3
                 const uint32_t b = bucket(fg_axis_hash_rel(p.x, S->rb_cell[0], x, FG_PX), hy, hz);
                 const uint32_t st = __ldg(G.start + b);
                 if (st != FG_EMPTY) visit(st, __ldg(G.end + b));
+            }
+        }
+    }
+    return acc;
+}
+
+/* Whether a particle's cell is marked near a sphere (G.near). */
+__device__ __forceinline__ bool fg_contact_marked(const FgScene *S, uint32_t scene, float4 p, const RigidGrid &G)
+{
+    int cx, cy, cz;
+    const float mind = S->fluid_radius + S->rb_radius + S->fluid_eps;
+    if (!fg_near_cell(p.x, p.y, p.z, fg_near_inv(mind), cx, cy, cz)) return true;
+    const uint32_t h = fg_near_bit(cx, cy, cz, scene, G.near_mask);
+    return __ldg(G.near + (h >> 5)) >> (h & 31u) & 1u;
+}
+
+/* fg_fluid_rigid_contact of one particle by a whole warp (converged, p and v
+ * the same in every lane): the lanes look four buckets each up at once, then
+ * test a sphere each, and the contacts, a few, are added in the walk's order:
+ * the same bits in two or three memory latencies instead of one per bucket
+ * row and sphere (about 55 spheres at the default half-width of 2). */
+__device__ __forceinline__ float3 fg_contact_warp(const FgScene *S, float4 p, float4 v, const RigidGrid &G,
+                                                  bool dynamic)
+{
+    const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
+    float3 acc = make_float3(0.f, 0.f, 0.f);
+    const float mind = S->fluid_radius + S->rb_radius + S->fluid_eps;
+    const float3 P = make_float3(p.x, p.y, p.z), V = make_float3(v.x, v.y, v.z);
+    const int rx = S->f2r_rel[0], ry = S->f2r_rel[1], rz = S->f2r_rel[2];
+    const uint32_t nx = 2u * rx + 1u, ny = 2u * ry + 1u, total = nx * ny * (2u * rz + 1u);
+    for (uint32_t b0 = 0; b0 < total; b0 += 128u) {
+        uint32_t st[4], cnt[4], sum = 0u;
+#pragma unroll
+        for (uint32_t u = 0; u < 4u; u++) {
+            const uint32_t q = b0 + 4u * lane + u, row = q / nx;
+            st[u] = cnt[u] = 0u;
+            if (q < total) {
+                const uint32_t hx = fg_axis_hash_rel(p.x, S->rb_cell[0], (int)(q - row * nx) - rx, FG_PX),
+                               hy = fg_axis_hash_rel(p.y, S->rb_cell[1], (int)(row % ny) - ry, FG_PY),
+                               hz = fg_axis_hash_rel(p.z, S->rb_cell[2], (int)(row / ny) - rz, FG_PZ);
+                const uint32_t b = G.own_geometry ? fg_bucket(hx, hy, hz, G.nb, G.mask)
+                                                  : S->rb_bucket_base + fg_bucket(hx, hy, hz, S->rb_nb, S->rb_nb_mask);
+                const uint32_t a = __ldg(G.start + b), e = __ldg(G.end + b);
+                if (a != FG_EMPTY && e > a) {
+                    st[u] = a;
+                    cnt[u] = e - a;
+                }
+            }
+            sum += cnt[u];
+        }
+        uint32_t incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(full, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        const uint32_t all = __shfl_sync(full, incl, 31);
+        for (uint32_t c0 = 0; c0 < all; c0 += 32u) {
+            /* candidate pos: the lane whose buckets hold it, then the bucket */
+            const uint32_t pos = c0 + lane;
+            uint32_t k = 0u;
+#pragma unroll
+            for (uint32_t o = 16u; o; o >>= 1) {
+                const uint32_t y = __shfl_sync(full, incl, (int)(k + o - 1u));
+                if (y <= pos) k += o;
+            }
+            uint32_t r = pos - __shfl_sync(full, incl - sum, (int)k), j = 0u;
+            bool found = false;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t n = __shfl_sync(full, cnt[u], (int)k), a = __shfl_sync(full, st[u], (int)k);
+                if (!found && r < n) {
+                    j = a + r;
+                    found = true;
+                }
+                if (!found) r -= n;
+            }
+            bool in = false;
+            float c = 0.f;
+            float3 n = make_float3(0.f, 0.f, 0.f);
+            if (pos < all) {
+                const float4 q = __ldg(G.spos + j);
+                float3 d;
+                float lg;
+                in = fg_contact_near(P, q, mind, d, lg);
+                if (in) {
+                    const float4 vq = dynamic ? __ldg(G.body_vel + (int)q.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    c = fg_contact_force(d, lg, V, vq, S->ck, S->ckd, n);
+                }
+            }
+            for (uint32_t m = __ballot_sync(full, in); m; m &= m - 1u) {
+                const int b = __ffs(m) - 1;
+                const float cb = __shfl_sync(full, c, b);
+                acc.x += cb * __shfl_sync(full, n.x, b);
+                acc.y += cb * __shfl_sync(full, n.y, b);
+                acc.z += cb * __shfl_sync(full, n.z, b);
             }
         }
     }
