@@ -94,6 +94,18 @@ __device__ __forceinline__ void fg_st_list2(uint32_t *p, uint32_t a, uint32_t b)
     asm volatile("st.global.cs.v2.b32 [%0], {%1, %2};" ::"l"(p), "r"(a), "r"(b));
 }
 
+/* Four (16-byte aligned) and eight (32-byte aligned, one sector) list entries,
+ * as fg_st_list2. */
+__device__ __forceinline__ void fg_st_list4(uint32_t *p, uint4 a)
+{
+    asm volatile("st.global.cs.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w));
+}
+__device__ __forceinline__ void fg_st_list8(uint32_t *p, uint4 a, uint4 b)
+{
+    asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+                 "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w));
+}
+
 /* select one of three register values without local-memory indexing */
 __device__ __forceinline__ uint32_t fg_sel3(uint32_t a0, uint32_t a1, uint32_t a2, int k)
 {

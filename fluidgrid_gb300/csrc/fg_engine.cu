@@ -858,7 +858,7 @@ uint32_t World::enqueue_step(cudaEvent_t *ev)
                               end, dp, nbr.rec, n, stream, cc_warps);
         else
             launch_density(L, spos, start, end, dp, 0.f, 0.f, 0.f, 0, svel, use_list ? &nbr : nullptr,
-                           density_order(), pair_counter);
+                           pair_counter);
         mark(3, 1);
         launches++;
     }
@@ -1263,7 +1263,7 @@ int World::run_stage(int stage, int flags)
                               end, dp, nbr.rec, n, stream, cc_warps);
         else
             launch_density(L, spos, start, end, dp, 0.f, 0.f, 0.f, 0, svel, use_list ? &nbr : nullptr,
-                           density_order(), pair_counter);
+                           pair_counter);
         break;
     case FG_RUN_RB_GRID: {
         if (!rb) break;

@@ -98,16 +98,11 @@ struct World {
     uint64_t kernels_enqueued = 0; /* kernel launches enqueued or replayed so far */
     bool order_valid = false;
     void enqueue_order_refresh();
-    /* the target order of the force pass, and of the density pass unless
-     * the Morton order is the force pass's only; the neighbour lists are
-     * indexed by sorted particle, so the two passes may differ */
+    /* the target order of the force pass; the density pass takes its targets
+     * in bucket order, and the neighbour lists are indexed by sorted particle */
     TargetOrder target_order() const
     {
         return (use_order && order_valid) ? TargetOrder{tord, inv} : TargetOrder{nullptr, nullptr};
-    }
-    TargetOrder density_order() const
-    {
-        return order_forces_only ? TargetOrder{nullptr, nullptr} : target_order();
     }
     bool order_refresh_due(uint64_t s) const;
     /* rigid */

@@ -136,7 +136,7 @@ struct NbrList {
 void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, const uint32_t *end, float2 *dp,
                     float gas_override, float rest_override, float mass_override, int use_override,
                     const float4 *svel = nullptr, const NbrList *list = nullptr,
-                    TargetOrder ord = TargetOrder{nullptr, nullptr}, unsigned long long *pairs = nullptr);
+                    unsigned long long *pairs = nullptr);
 
 struct RigidGrid {
     const float4 *spos;     /* sorted sphere positions, w = body index */

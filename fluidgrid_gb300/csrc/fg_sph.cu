@@ -16,84 +16,167 @@
  * agree with the reference arithmetic to the tolerances the parity tests
  * state.
  *
- * One thread per particle in sorted order: neighbouring lanes share cells,
- * so neighbour loads broadcast from L1 and sorted float4 loads coalesce.
- * In the world pipeline the density pass is the only one that walks the
+ * In the world pipeline the density pass is the only one that looks at the
  * ~216 candidates of the 27 buckets (~1,000 once the block compresses): it
  * records each particle's in-range visits (in visit order, duplicates and
- * the particle itself included) in the particle's own list, buffered in
- * registers and stored two entries at a time, together with a packed
- * 32-byte record per particle.  The force pass then loops over the ~30-110
- * listed neighbours per particle with all lanes busy, one 256-bit record
- * load each, instead of re-walking the candidates where almost every warp
- * iteration would run the pair math for a few lanes. */
+ * the particle itself included) in the particle's own list, together with a
+ * packed 32-byte record per particle.  The force pass then loops over the
+ * ~30-110 listed neighbours per particle with all lanes busy, one 256-bit
+ * record load each, instead of going over the candidates again. */
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
 #include "fg_device.cuh"
 #include "fg_kernels.h"
 #include "fg_sph_common.cuh"
+#include "fg_stage.cuh"
 
 namespace fg {
 
-/* 16 CTAs of 128 threads per SM (32 registers): the walk's per-row state
- * spills to L1, but the candidate loop keeps its values in registers, and
- * the full 64 warps per SM hide the candidate loads and the in-range
- * branch's divergence better than 8 CTAs at 64 registers (0.85 -> 0.71 ms
- * on the 1M-particle dam break). */
-/* Work items are FG_CHUNK particles whatever the block size: a CTA of
- * BLOCK < FG_CHUNK threads takes an item in FG_CHUNK / BLOCK passes, one of
- * BLOCK > FG_CHUNK threads takes BLOCK / FG_CHUNK items at once.  Every
- * particle's arithmetic is the same for every block size. */
-#define FG_ITEMS_PER_CTA(B) ((B) >= FG_CHUNK ? (B) / FG_CHUNK : 1u)
-#define FG_PASSES(B) ((B) >= FG_CHUNK ? 1u : FG_CHUNK / (B))
+/* The density pass, by warp: fg_stage.cuh's staging, then a lane per target
+ * over its staged candidates.  Bound by instruction issue (about 180 warp
+ * instructions a target at 0.5 h spacing, of which 100 are staging, and 620 at
+ * 0.32 h; the walk by thread took 237 and 700).  524,288 particles with lists,
+ * ncu, walk by thread -> here: 180 -> 139 us at 0.5 h, 249 -> 253 at 0.45 h
+ * (cells of 8 to 27 targets fill a warp badly), 366 -> 311 at 0.36 h, 506 ->
+ * 447 at 0.32 h; 4,194,304 particles 1790 -> 1182 us; 16,384 particles, where
+ * a thread's chain of 216 candidate loads was the pass, 37 -> 14 us.
+ *
+ * Staged candidates of a warp: its targets lie in four or five groups of some
+ * 90 (60-100 candidates kept of a cell's 216).  384 leave ten CTAs an SM;
+ * 512 (nine CTAs): 1509 against 1192 us at 4M, 275 against 246 at 1M. */
+#ifndef FG_DENSITY_STAGE
+#define FG_DENSITY_STAGE 384u
+#endif
+#ifndef FG_DENSITY_CTAS
+#define FG_DENSITY_CTAS 10
+#endif
+#define FG_STAGE_GROUPS 9u /* a warp whose targets lie in more groups walks by thread */
+#define FG_DENSITY_THREADS 64u
 
-template <bool LIST, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 2048 / BLOCK) k_density(const FgWork *__restrict__ work, uint32_t nwork,
-                                                     uint32_t n_single, const FgScene *__restrict__ table,
-                                                     const __grid_constant__ FgScene single,
-                                                     const float4 *__restrict__ spos,
-                                                     const float4 *__restrict__ svel,
-                                                     const uint32_t *__restrict__ start,
-                                                     const uint32_t *__restrict__ end, float2 *__restrict__ dp,
-                                                     float gas_o, float rest_o, float mass_o, int use_o,
-                                                     const __grid_constant__ NbrList list, TargetOrder ord,
-                                                     unsigned long long *__restrict__ pairs)
+template <bool LIST>
+struct DensityShared {
+    float4 cand[FG_DENSITY_STAGE]; /* x, y, z, sorted index as bits */
+    uint32_t idx[FG_STAGE_WINDOW];
+    uint32_t ring[LIST ? 16 : 1][32]; /* each lane's newest list entries */
+};
+
+/* One lane's list entries on their way to its list: collected in a ring of
+ * sixteen in shared memory, stored a sector of eight at a time.  Lists are far
+ * apart, so every store is a wavefront of its own a lane; and written in range
+ * or not, kept by the count, an entry costs no divergent branch (0.32 h, 1M:
+ * 855 us with two entries a store in a branch, 767 us so). */
+struct ListRing {
+    uint32_t cnt, done; /* entries; entries stored, a multiple of 8 */
+
+    /* j if it is in range */
+    __device__ __forceinline__ void push(uint32_t (*ring)[32], uint32_t lane, uint32_t j, bool in)
+    {
+        ring[cnt & 15u][lane] = j;
+        cnt += in ? 1u : 0u;
+    }
+    __device__ __forceinline__ uint4 four(const uint32_t (*ring)[32], uint32_t lane, uint32_t k) const
+    {
+        const uint32_t b = k & 15u; /* a multiple of 4 */
+        return make_uint4(ring[b][lane], ring[b + 1u][lane], ring[b + 2u][lane], ring[b + 3u][lane]);
+    }
+    /* after at most eight pushes since the last call */
+    __device__ __forceinline__ void spill(const uint32_t (*ring)[32], uint32_t lane, uint32_t *lp, uint32_t cap)
+    {
+        if (cnt - done >= 8u) {
+            if (done + 8u <= cap)
+                fg_st_list8(lp + done, four(ring, lane, done), four(ring, lane, done + 4u));
+            else if (done + 4u <= cap)
+                fg_st_list4(lp + done, four(ring, lane, done));
+            done += 8u;
+        }
+    }
+    /* the rest, padded to a whole group of four with the target itself, which
+     * the force pass skips, so it reads only whole groups */
+    __device__ __forceinline__ void finish(uint32_t (*ring)[32], uint32_t lane, uint32_t *lp, uint32_t cap, uint32_t self)
+    {
+        if (cnt > cap) return;
+        for (uint32_t k = cnt; k & 3u; k++) ring[k & 15u][lane] = self;
+        for (; done < cnt; done += 4u) fg_st_list4(lp + done, four(ring, lane, done));
+    }
+};
+
+template <bool LIST, bool COUNT>
+__global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density(
+    const FgWork *__restrict__ work, uint32_t nwork, uint32_t n_single, const FgScene *__restrict__ table,
+    const __grid_constant__ FgScene single, uint32_t range, const float4 *__restrict__ spos,
+    const float4 *__restrict__ svel, const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+    float2 *__restrict__ dp, float gas_o, float rest_o, float mass_o, int use_o, const __grid_constant__ NbrList list,
+    unsigned long long *__restrict__ pairs)
 {
-    constexpr uint32_t IPC = FG_ITEMS_PER_CTA(BLOCK), PASSES = FG_PASSES(BLOCK);
-    const uint32_t sub = IPC > 1u ? threadIdx.x / FG_CHUNK : 0u;
-    const uint32_t lt = IPC > 1u ? threadIdx.x % FG_CHUNK : threadIdx.x;
+    __shared__ DensityShared<LIST> shared[FG_DENSITY_THREADS / 32];
+    DensityShared<LIST> &sm = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t cap = LIST ? __ldg(list.cap) : 0u;
     unsigned long long pc = 0; /* in-range density visits of this thread */
     uint32_t mx = 0;           /* largest list count of this thread */
     uint32_t ovf = 0;          /* targets of this thread with more entries than slots */
-    for (uint32_t w = blockIdx.x * IPC + sub; w < nwork; w += gridDim.x * IPC)
-#pragma unroll 1
-    for (uint32_t ps = 0; ps < PASSES; ps++) {
-        const uint32_t tid = lt + ps * BLOCK;
-        FgWork it = fg_work(work, w, n_single);
-        const bool valid = tid < it.count;
+    const uint32_t per = FG_CHUNK / range; /* warps per work item */
+    for (uint32_t warp = blockIdx.x * (FG_DENSITY_THREADS / 32u) + (threadIdx.x >> 5); warp < nwork * per;
+         warp += gridDim.x * (FG_DENSITY_THREADS / 32u)) {
+        const FgWork it = fg_work(work, warp / per, n_single);
+        const uint32_t q0 = (warp % per) * range;
+        if (q0 >= it.count) continue; /* uniform over the warp */
         const FgScene *S = fg_scene(table, &single, it.scene);
-        const uint32_t tpos = it.first + tid; /* target slot */
-        const uint32_t i = (ord.tord && valid) ? __ldg(ord.inv + __ldg(ord.tord + tpos)) : tpos;
-        const float4 p = valid ? spos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const uint32_t lo = table ? S->pbase : 0u, hi = table ? S->pbase + S->n : n_single;
+        const float scale = S->scale, h2 = S->h2;
+        uint32_t next, stop;
+        const StageGrid G(S);
+        fg_stage_range(it.first + q0, range, lo, hi, G, spos, next, stop);
+        while (next < stop) {
+        const uint32_t i = next + lane; /* sorted index */
+        uint32_t n = min(32u, stop - next);
+        float4 p = lane < n ? spos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const StageSig sig = fg_stage_sig(p, G);
+        if (stop - next > 32u) n = fg_stage_trim(sig, __ldg(spos + next + 32u), G);
+        next += n;
+        const bool valid = lane < n;
         const bool active = valid && p.w > 0.0f; /* inactive: density not written */
+        const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
         DensityAcc acc;
         acc.init();
+        ListRing ring = {0u, 0u};
         /* lists by sorted index: the force pass may visit the targets in another order */
         uint32_t *lp = LIST ? list.idx + (size_t)i * list.stride : nullptr;
-        if (active) {
-            const float scale = S->scale, h2 = S->h2;
-            const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
+        uint32_t lead, leads;
+        const bool staged = fg_stage_groups(sig, __ballot_sync(FG_FULL, active), FG_STAGE_GROUPS, lead, leads) &&
+                            !__any_sync(FG_FULL, active && sig.odd);
+        if (staged) {
+            fg_stage_rounds<FG_DENSITY_STAGE>(
+                sig, lead, leads, px, py, pz, G, spos, start, end, sm.idx,
+                [&](uint32_t slot, uint32_t j, float4 c) {
+                    sm.cand[slot] = make_float4(c.x, c.y, c.z, __uint_as_float(j));
+                },
+                [&](uint32_t first, uint32_t stop, uint32_t) {
+                    for (uint32_t k = first; k < stop; k += 8u) {
+#pragma unroll
+                        for (uint32_t e = 0; e < 8u; e++) {
+                            const float4 q = sm.cand[k + e];
+                            const bool in = acc.term(q, px, py, pz, scale, h2);
+                            if (LIST) ring.push(sm.ring, lane, __float_as_uint(q.w), in);
+                            else if (COUNT) ring.cnt += in ? 1u : 0u;
+                        }
+                        if (LIST) ring.spill(sm.ring, lane, lp, cap);
+                    }
+                });
+            if (LIST && active) ring.finish(sm.ring, lane, lp, cap, i);
+            acc.cnt = ring.cnt;
+        } else if (active) {
             fg_walk27(
                 p.x, p.y, p.z, S, start, end,
-                [&](uint32_t j) { acc.visit<LIST>(__ldg(spos + j), j, px, py, pz, scale, h2, lp, cap); },
-                [&] { acc.end_bucket(); });
+                [&](uint32_t j) { acc.visit<LIST, COUNT>(__ldg(spos + j), j, px, py, pz, scale, h2, lp, cap); });
             if (LIST) acc.flush(lp, cap, i);
+        }
+        if (active) {
             const float mass = use_o ? mass_o : S->mass;
             const float gas = use_o ? gas_o : S->gas;
             const float rest = use_o ? rest_o : S->rest;
-            const float2 d = fg_density_out(mass, S->kpoly6, gas, rest, acc.s);
+            const float2 d = fg_density_out(mass, S->kpoly6, gas, rest, acc.sum());
             dp[i] = d;
             if (LIST) {
                 const float4 v = __ldg(svel + i);
@@ -107,16 +190,15 @@ __global__ void __launch_bounds__(BLOCK, 2048 / BLOCK) k_density(const FgWork *_
             list.rec[2 * i] = make_float4(p.x, p.y, p.z, d.x);
             list.rec[2 * i + 1] = make_float4(v.x, v.y, v.z, d.y);
         }
-        const uint32_t cnt = acc.cnt, dcnt = LIST ? acc.cnt : acc.dcnt;
-        if (LIST && valid) list.cnt[i] = cnt;
-        pc += dcnt;
-        mx = max(mx, cnt);
-        ovf += (LIST && cnt > cap) ? 1u : 0u;
+        if (LIST && valid) list.cnt[i] = acc.cnt;
+        pc += acc.cnt;
+        mx = max(mx, acc.cnt);
+        ovf += (LIST && acc.cnt > cap) ? 1u : 0u;
+        }
     }
     /* once per warp: in-range pair visits (self included) for reporting, and
      * the largest list count for the capacity check */
-    const uint32_t lane = threadIdx.x & 31u;
-    if (pairs) {
+    if (COUNT && pairs) {
 #pragma unroll
         for (int o = 16; o; o >>= 1) pc += __shfl_xor_sync(0xffffffffu, pc, o);
         if (lane == 0 && pc) atomicAdd(pairs, pc);
@@ -131,32 +213,45 @@ __global__ void __launch_bounds__(BLOCK, 2048 / BLOCK) k_density(const FgWork *_
     }
 }
 
+/* Targets of a warp: 32, or fewer where that leaves the SMs short of warps
+ * (16 each): a group's lookups and staging are a chain of some ten memory
+ * latencies, and a warp goes through its groups one after another. */
+static uint32_t stage_range(uint32_t nwork)
+{
+    const uint64_t want = 16ull * (uint64_t)sm_count();
+    uint32_t range = 32u;
+    while (range > 8u && (uint64_t)nwork * (FG_CHUNK / range) < want) range >>= 1;
+    return range;
+}
+
 void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, const uint32_t *end, float2 *dp,
                     float gas_o, float rest_o, float mass_o, int use_o, const float4 *svel, const NbrList *list,
-                    TargetOrder ord, unsigned long long *pairs)
+                    unsigned long long *pairs)
 {
     if (!L.nwork) return;
     NbrList none;
     memset(&none, 0, sizeof(none));
     const NbrList &nl = list ? *list : none;
-    const uint32_t B = L.block ? L.block : FG_CHUNK;
-    const uint32_t ipc = FG_ITEMS_PER_CTA(B);
-    /* ctas_per_sm counts CTAs of FG_CHUNK threads: the same threads per SM
-     * for every block size */
-    const int per_sm = (int)(((L.ctas_per_sm ? L.ctas_per_sm : 64u) * FG_CHUNK) / B);
-    const uint32_t g = grid_for((L.nwork + ipc - 1u) / ipc, per_sm > 0 ? per_sm : 1);
-#define FG_DENSITY(LI, BL)                                                                                        \
-    k_density<LI, BL><<<g, BL, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, spos, svel, start, end, dp, \
-                                              gas_o, rest_o, mass_o, use_o, nl, ord, pairs)
-    if (B == 64u) {
-        if (list) FG_DENSITY(true, 64); else FG_DENSITY(false, 64);
-    } else if (B == 256u) {
-        if (list) FG_DENSITY(true, 256); else FG_DENSITY(false, 256);
-    } else {
-        if (list) FG_DENSITY(true, 128); else FG_DENSITY(false, 128);
-    }
+    const uint32_t range = stage_range(L.nwork);
+    /* ctas_per_sm counts CTAs of FG_CHUNK threads for 32 targets a warp */
+    const uint32_t per = FG_CHUNK / range * 32u / FG_DENSITY_THREADS;
+    const uint32_t g = grid_for(L.nwork * per, (int)((L.ctas_per_sm ? L.ctas_per_sm : 64u) * per));
+#define FG_DENSITY(LI, CO)                                                                                         \
+    k_density<LI, CO><<<g, FG_DENSITY_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, range, spos, \
+                                                              svel, start, end, dp, gas_o, rest_o, mass_o, use_o,  \
+                                                              nl, pairs)
+    if (list) FG_DENSITY(true, true);
+    else if (pairs) FG_DENSITY(false, true);
+    else FG_DENSITY(false, false);
 #undef FG_DENSITY
 }
+
+/* Work items are FG_CHUNK particles whatever the block size: a CTA of
+ * BLOCK < FG_CHUNK threads takes an item in FG_CHUNK / BLOCK passes, one of
+ * BLOCK > FG_CHUNK threads takes BLOCK / FG_CHUNK items at once.  Every
+ * particle's arithmetic is the same for every block size. */
+#define FG_ITEMS_PER_CTA(B) ((B) >= FG_CHUNK ? (B) / FG_CHUNK : 1u)
+#define FG_PASSES(B) ((B) >= FG_CHUNK ? 1u : FG_CHUNK / (B))
 
 struct RigidArgs {
     RigidGrid dyn;
@@ -386,9 +481,10 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
             if (walk) s_id[base + __popc(m & ((1u << lane) - 1u))] = id;
         }
         __syncthreads();
+        const ContactShape C(S);
         for (uint32_t k = threadIdx.x >> 5; k < s_n; k += FG_CONTACT_THREADS / 32u) {
             const uint32_t id = s_id[k];
-            const float3 c = fg_contact_warp(S, __ldg(pos + id), __ldg(vel + id), G, true);
+            const float3 c = fg_contact_warp(S, C, __ldg(pos + id), __ldg(vel + id), G, true);
             if (lane == 0u) out[id] = make_float4(c.x, c.y, c.z, 0.0f);
         }
         __syncthreads();
@@ -398,8 +494,10 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out)
 {
     if (!L.nwork) return;
-    k_fluid_contact<<<grid_for(L.nwork, 8), FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table,
-                                                                              *L.single, pos, vel, G, out);
+    /* a CTA per item: most have nothing to search and leave their SM to the
+     * kernels beside this one */
+    k_fluid_contact<<<L.nwork, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos, vel,
+                                                                  G, out);
 }
 
 /* SPHIntegrateK (K_FluidSim.cu:418-438): pos += vel*(dt/scale) for active

@@ -57,50 +57,47 @@ __device__ __forceinline__ void fg_walk27(float px, float py, float pz, const Fg
 /* One target's state in a density pass: the sum of (h^2 - l^2)^3 over the
  * candidates with l <= h (an exact 0 at l = h, so the sum equals the
  * reference's l < h sum) and the force pass's neighbour list (every visit
- * with l <= h, the target's own entries included: testing j != i in the
- * force pass, which waits on memory, is cheaper than in this issue-bound
- * branch), stored two entries (8 bytes) at a time.  The terms of one bucket
- * (a few in range) are added plainly; each bucket's partial is then added to
- * the total with Kahan compensation, which keeps the hot in-range branch to
- * one addition.  Every operation is rounded on its own, so any kernel that
- * visits the same candidates in the same order produces the same bits. */
+ * with l <= h, the target's own entries included, which the force pass
+ * skips), stored two entries (8 bytes) at a time.  Every addition's rounding
+ * error is collected beside the sum; a candidate out of range adds an exact 0
+ * to both.  So the result depends on the in-range candidates and their order
+ * alone: however they are found, a target gets the same bits. */
 struct DensityAcc {
-    float s, c;          /* Kahan sum and compensation over bucket partials */
-    float b;             /* plain sum of the current bucket's terms */
-    uint32_t dcnt, cnt;  /* density visits (without a list), list entries */
-    uint32_t q2, q3;     /* the last two list entries (q3 the newest) */
+    float s, c;      /* sum and compensation */
+    uint32_t cnt;    /* in-range visits, the list's entries */
+    uint32_t q2, q3; /* the last two list entries (q3 the newest) */
 
     __device__ __forceinline__ void init()
     {
-        s = c = b = 0.0f;
-        dcnt = cnt = 0;
+        s = c = 0.0f;
+        cnt = 0;
         q2 = q3 = 0;
     }
 
-    /* fold the finished bucket's partial into the compensated total */
-    __device__ __forceinline__ void end_bucket()
-    {
-        const float y = __fsub_rn(b, c);
-        const float u = __fadd_rn(s, y);
-        c = __fsub_rn(__fsub_rn(u, s), y);
-        s = u;
-        b = 0.0f;
-    }
-
-    template <bool LIST>
-    __device__ __forceinline__ void visit(float4 q, uint32_t j, float px, float py, float pz, float scale, float h2,
-                                          uint32_t *lp, uint32_t cap)
+    /* add a candidate's (h^2 - l^2)^3, 0 beyond h; whether it is in range */
+    __device__ __forceinline__ bool term(float4 q, float px, float py, float pz, float scale, float h2)
     {
         const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
-        if (r2 <= h2) {
-            const float t = __fsub_rn(h2, r2);
-            b = __fadd_rn(b, __fmul_rn(__fmul_rn(t, t), t));
-            if (!LIST) dcnt++; /* with a list every visit is an entry: cnt counts them */
+        const float t = fmaxf(__fsub_rn(h2, r2), 0.0f); /* 0 for a NaN too */
+        const float t3 = __fmul_rn(__fmul_rn(t, t), t);
+        const float u = __fadd_rn(s, t3);
+        c = __fadd_rn(c, __fsub_rn(t3, __fsub_rn(u, s)));
+        s = u;
+        return r2 <= h2;
+    }
+
+    __device__ __forceinline__ float sum() const { return __fadd_rn(s, c); }
+
+    template <bool LIST, bool COUNT>
+    __device__ __forceinline__ void visit(float4 q, uint32_t j, float px, float py, float pz, float scale, float h2,
+                                          uint32_t *lp, uint32_t cap)
+    {
+        if (term(q, px, py, pz, scale, h2)) {
+            if (COUNT) cnt++;
             if (LIST) {
                 q2 = q3;
                 q3 = j;
-                cnt++;
                 if ((cnt & 1u) == 0u && cnt <= cap) fg_st_list2(lp + cnt - 2u, q2, q3);
             }
         }
@@ -307,30 +304,57 @@ __device__ __forceinline__ bool fg_contact_marked(const FgScene *S, uint32_t sce
     return __ldg(G.near + (h >> 5)) >> (h & 31u) & 1u;
 }
 
+/* The (2r+1)^3 buckets around a particle, and how position q of their walk
+ * order (z outer, x inner) splits by multiplication: exact for q < 17^3 and
+ * divisors up to 17, as (divisor * reciprocal - 2^20) q < 2^20. */
+struct ContactShape {
+    uint32_t nx, ny, total, inv_x, inv_y;
+    int rx, ry, rz;
+    __device__ __forceinline__ explicit ContactShape(const FgScene *S)
+        : rx(S->f2r_rel[0]), ry(S->f2r_rel[1]), rz(S->f2r_rel[2])
+    {
+        nx = 2u * rx + 1u;
+        ny = 2u * ry + 1u;
+        total = nx * ny * (2u * rz + 1u);
+        inv_x = (1u << 20) / nx + 1u;
+        inv_y = (1u << 20) / ny + 1u;
+    }
+};
+
 /* fg_fluid_rigid_contact of one particle by a whole warp (converged, p and v
- * the same in every lane): the lanes look four buckets each up at once, then
- * test a sphere each, and the contacts, a few, are added in the walk's order:
- * the same bits in two or three memory latencies instead of one per bucket
- * row and sphere (about 55 spheres at the default half-width of 2). */
-__device__ __forceinline__ float3 fg_contact_warp(const FgScene *S, float4 p, float4 v, const RigidGrid &G,
-                                                  bool dynamic)
+ * the same in every lane): the lanes hash the axes once, look four buckets
+ * each up at once, then test a sphere each, and the contacts, a few, are added
+ * in the walk's order: the same bits in two or three memory latencies instead
+ * of one per bucket row and sphere (about 55 spheres at the default half-width
+ * of 2). */
+__device__ __forceinline__ float3 fg_contact_warp(const FgScene *S, const ContactShape &C, float4 p, float4 v,
+                                                  const RigidGrid &G, bool dynamic)
 {
     const uint32_t full = 0xffffffffu, lane = threadIdx.x & 31u;
     float3 acc = make_float3(0.f, 0.f, 0.f);
     const float mind = S->fluid_radius + S->rb_radius + S->fluid_eps;
     const float3 P = make_float3(p.x, p.y, p.z), V = make_float3(v.x, v.y, v.z);
-    const int rx = S->f2r_rel[0], ry = S->f2r_rel[1], rz = S->f2r_rel[2];
-    const uint32_t nx = 2u * rx + 1u, ny = 2u * ry + 1u, total = nx * ny * (2u * rz + 1u);
-    for (uint32_t b0 = 0; b0 < total; b0 += 128u) {
+    /* lanes 10 a + k: offset k - r of axis a, for half-widths up to 4 */
+    const bool small = max(C.rx, max(C.ry, C.rz)) <= 4;
+    const uint32_t ax = lane / 10u, ak = lane - 10u * ax;
+    const uint32_t ah = ax == 0u   ? fg_axis_hash_rel(p.x, S->rb_cell[0], (int)ak - C.rx, FG_PX)
+                        : ax == 1u ? fg_axis_hash_rel(p.y, S->rb_cell[1], (int)ak - C.ry, FG_PY)
+                                   : fg_axis_hash_rel(p.z, S->rb_cell[2], (int)ak - C.rz, FG_PZ);
+    for (uint32_t b0 = 0; b0 < C.total; b0 += 128u) {
         uint32_t st[4], cnt[4], sum = 0u;
 #pragma unroll
         for (uint32_t u = 0; u < 4u; u++) {
-            const uint32_t q = b0 + 4u * lane + u, row = q / nx;
+            const uint32_t q = b0 + 4u * lane + u, row = (q * C.inv_x) >> 20, z = (row * C.inv_y) >> 20;
+            const uint32_t x = q - row * C.nx, y = row - z * C.ny;
+            uint32_t hx = __shfl_sync(full, ah, (int)x), hy = __shfl_sync(full, ah, (int)(10u + y)),
+                     hz = __shfl_sync(full, ah, (int)(20u + z));
             st[u] = cnt[u] = 0u;
-            if (q < total) {
-                const uint32_t hx = fg_axis_hash_rel(p.x, S->rb_cell[0], (int)(q - row * nx) - rx, FG_PX),
-                               hy = fg_axis_hash_rel(p.y, S->rb_cell[1], (int)(row % ny) - ry, FG_PY),
-                               hz = fg_axis_hash_rel(p.z, S->rb_cell[2], (int)(row / ny) - rz, FG_PZ);
+            if (q < C.total) {
+                if (!small) {
+                    hx = fg_axis_hash_rel(p.x, S->rb_cell[0], (int)x - C.rx, FG_PX);
+                    hy = fg_axis_hash_rel(p.y, S->rb_cell[1], (int)y - C.ry, FG_PY);
+                    hz = fg_axis_hash_rel(p.z, S->rb_cell[2], (int)z - C.rz, FG_PZ);
+                }
                 const uint32_t b = G.own_geometry ? fg_bucket(hx, hy, hz, G.nb, G.mask)
                                                   : S->rb_bucket_base + fg_bucket(hx, hy, hz, S->rb_nb, S->rb_nb_mask);
                 const uint32_t a = __ldg(G.start + b), e = __ldg(G.end + b);

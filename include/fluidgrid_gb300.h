@@ -178,19 +178,20 @@ int fg_world_set_graphs(fg_world *w, int on);
 /* Tunables (they change how work is scheduled, not which neighbours are
  * summed):
  *   FG_OPT_KERNEL         density/force kernels:
- *                         1 = one thread per particle with in-range
- *                             neighbour lists recorded by the density pass
+ *                         1 = in-range neighbour lists recorded by the
+ *                             density pass, which searches by warp, and read
+ *                             by the force pass, a thread per particle
  *                             (default);
- *                         0 = one thread per particle walking the 27 buckets
- *                             in both passes;
+ *                         0 = no lists: a thread per particle walks the 27
+ *                             buckets in the force pass;
  *                         2 = one warp per run, one target at a time
  *   FG_OPT_NEIGHBOR_LIST  1 = kernel 1, 0 = kernel 0
- *   FG_OPT_TARGET_ORDER   kernels 0/1: 1 = targets in Morton order of their
- *                         cells, 0 = hashed bucket order, 2 = Morton order in
- *                         the force pass only (default, server worlds too): the
- *                         density pass walks in bucket order, where a warp's
- *                         lanes share their buckets, and the force pass's
- *                         lanes, spatially close, share neighbour records
+ *   FG_OPT_TARGET_ORDER   kernels 0/1, the force pass: 1 or 2 = targets in
+ *                         Morton order of their cells (default 2, server
+ *                         worlds too): its lanes, spatially close, share
+ *                         neighbour records; 0 = hashed bucket order.  The
+ *                         density pass takes its targets in bucket order,
+ *                         where they stand cell by cell
  *   FG_OPT_ORDER_PERIOD   steps between refreshes of the Morton order (16)
  *   FG_OPT_DIGIT_BITS     radix digit width 1..8
  *   FG_OPT_AUTOTUNE_PERIOD  every this many steps the autotuner runs one
@@ -220,8 +221,8 @@ int fg_world_set_graphs(fg_world *w, int on);
  *                         1 = CTAs per SM, 2 = radix digit width, 4 = the
  *                         sort variant of FG_OPT_ONE_PASS_SORT, 8 = block
  *                         size, 16 = runs per CTA (default 31)
- *   FG_OPT_BLOCK_SIZE     kernels 0/1: threads per CTA of the density/force
- *                         grids, 64, 128 (default) or 256; work items stay
+ *   FG_OPT_BLOCK_SIZE     kernels 0/1: threads per CTA of the force grid, 64,
+ *                         128 (default) or 256; work items stay
  *                         128 particles (two passes of a 64-thread CTA, two
  *                         items per 256-thread CTA) and the threads per SM
  *                         stay those of FG_OPT_CTAS_PER_SM
