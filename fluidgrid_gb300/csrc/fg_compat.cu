@@ -13,6 +13,7 @@
 #include "fg_types.h"
 #include "fg_kernels.h"
 #include "fg_engine.h"
+#include "fg_device.cuh"
 #include "../../include/fluidgrid_gb300.h"
 #include "../../include/fluidgrid_reference.h"
 
@@ -114,6 +115,52 @@ void sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t bits, uint32_t n)
     fg::RadixScratch rs{g_sort.k, g_sort.v, g_sort.h};
     fg::radix_sort(keys, vals, keys, vals, n, bits, 8, rs, 0);
     finish();
+}
+
+/* Bit tables of the cells near the static and the dynamic spheres (as the
+ * world's, marked from the sorted grid the launcher is given), for the force
+ * launcher to search the particles near a sphere only.  Fixed in the module:
+ * the launchers use one stream, and g_mu keeps a call's clear, mark and force
+ * launches together. */
+constexpr uint32_t kNearBits = 1u << 20;
+__device__ uint32_t g_near[2][kNearBits / 32u];
+
+__global__ void __launch_bounds__(256) k_mark_near(const float4 *__restrict__ spos, const uint32_t *__restrict__ start,
+                                                   const uint32_t *__restrict__ end, uint32_t nb, float mind,
+                                                   uint32_t *near, uint32_t mask)
+{
+    const float inv = fg_near_inv(mind);
+    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < nb; b += gridDim.x * blockDim.x) {
+        const uint32_t st = __ldg(start + b), en = __ldg(end + b);
+        if (st == FG_EMPTY) continue;
+        for (uint32_t j = st; j < en; j++) {
+            const float4 q = __ldg(spos + j);
+            int cx, cy, cz;
+            fg_near_cell(q.x, q.y, q.z, inv, cx, cy, cz);
+            fg_near_mark(cx, cy, cz, 0u, near, mask);
+        }
+    }
+}
+
+/* grid.near marked from the grid's spheres */
+int mark_near(fg::RigidGrid &grid, uint32_t which, const FgScene &S)
+{
+    void *p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, g_near);
+    if (e != cudaSuccess) {
+        fg::set_error("cudaGetSymbolAddress", e);
+        return FG_E_CUDA;
+    }
+    uint32_t *const near = (uint32_t *)p + (size_t)which * (kNearBits / 32u);
+    uint32_t bits = 1u << 15; /* about 32 bits a bucket */
+    while (bits < kNearBits && bits / 32u < grid.nb) bits <<= 1;
+    cudaMemsetAsync(near, 0, bits / 8u, 0);
+    k_mark_near<<<fg::grid_for((grid.nb + 255u) / 256u, 8), 256>>>(grid.spos, grid.start, grid.end, grid.nb,
+                                                                   S.fluid_radius + S.rb_radius + S.fluid_eps, near,
+                                                                   bits - 1u);
+    grid.near = near;
+    grid.near_mask = bits - 1u;
+    return FG_OK;
 }
 
 } // namespace
@@ -282,6 +329,10 @@ void gSPHCalculateForcesWithSRB(float4 *oldPositions, float4 *oldVelocity, float
     fg::ForceOut o;
     o.vel = newVel;
     o.pos = nullptr;
+    std::lock_guard<std::mutex> lk(g_mu);
+    int r = useDynamicRB ? mark_near(dyn, 0u, S) : FG_OK;
+    if (r == FG_OK && useStaticRB) r = mark_near(sta, 1u, S);
+    if (r != FG_OK) { g_status = r; return; }
     fg::launch_forces(single_launch(&S, numParticles), oldPositions, oldVelocity, density_pressure, gridStart,
                       gridEnd, particleId, o, useDynamicRB ? &dyn : nullptr, useStaticRB ? &sta : nullptr, mass,
                       kViscosity, 1);

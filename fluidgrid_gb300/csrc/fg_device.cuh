@@ -283,6 +283,23 @@ __device__ __forceinline__ uint32_t fg_near_bit(int cx, int cy, int cz, uint32_t
     h ^= h >> 15;
     return h & mask;
 }
+/* The 27 marks of a sphere in cell (cx, cy, cz).  Neighbouring spheres mark
+ * the same cells: look, a plane of nine at once, before the atomics (a stale
+ * look costs one). */
+__device__ __forceinline__ void fg_near_mark(int cx, int cy, int cz, uint32_t scene, uint32_t *near, uint32_t mask)
+{
+    for (int z = -1; z <= 1; z++) {
+        uint32_t h[9], old[9];
+#pragma unroll
+        for (int o = 0; o < 9; o++) {
+            h[o] = fg_near_bit(cx + o % 3 - 1, cy + o / 3 - 1, cz + z, scene, mask);
+            old[o] = __ldcg(near + (h[o] >> 5));
+        }
+#pragma unroll
+        for (int o = 0; o < 9; o++)
+            if (!(old[o] >> (h[o] & 31u) & 1u)) atomicOr(near + (h[o] >> 5), 1u << (h[o] & 31u));
+    }
+}
 __device__ __forceinline__ float fg_near_inv(float mind) { return 1.0f / (1.25f * mind); }
 
 /* float atomics on the ordered-int encoding (for bounding boxes) */

@@ -115,19 +115,7 @@ __global__ void __launch_bounds__(FG_CHUNK) k_hash_offset(const FgWork *__restri
                 int cx, cy, cz;
                 const float mind = S->fluid_radius + S->rb_radius + S->fluid_eps;
                 fg_near_cell(a.x, a.y, a.z, fg_near_inv(mind), cx, cy, cz);
-                /* neighbouring spheres mark the same cells: look, a plane of
-                 * nine at once, before the atomics (a stale look costs one) */
-                for (int z = -1; z <= 1; z++) {
-                    uint32_t h[9], old[9];
-#pragma unroll
-                    for (int o = 0; o < 9; o++) {
-                        h[o] = fg_near_bit(cx + o % 3 - 1, cy + o / 3 - 1, cz + z, it.scene, near_mask);
-                        old[o] = __ldcg(near + (h[o] >> 5));
-                    }
-#pragma unroll
-                    for (int o = 0; o < 9; o++)
-                        if (!(old[o] >> (h[o] & 31u) & 1u)) atomicOr(near + (h[o] >> 5), 1u << (h[o] & 31u));
-                }
+                fg_near_mark(cx, cy, cz, it.scene, near, near_mask);
             }
         }
         if (aabb) {

@@ -259,18 +259,112 @@ struct RigidArgs {
     int use_dyn, use_sta;
 };
 
-template <bool LIST, int BLOCK>
+/* A world particle's contact with the bodies: stored by the contact pass, or
+ * walked here. */
+__device__ __forceinline__ float3 force_contact(const FgScene *S, uint32_t scene, float4 p, float4 v, uint32_t oi,
+                                                const RigidArgs &R)
+{
+    if (!R.use_dyn || !(S->flags & FG_SCENE_HAS_RB)) return make_float3(0.f, 0.f, 0.f);
+    if (!R.dyn.pre) return fg_fluid_rigid_contact(S, scene, p, v, R.dyn, true);
+    if (fg_contact_outside(S, scene, p, R.dyn) || !fg_contact_marked(S, scene, p, R.dyn))
+        return make_float3(0.f, 0.f, 0.f);
+    const float4 q = R.dyn.pre[oi];
+    return make_float3(q.x, q.y, q.z);
+}
+
+/* The contact of a warp's particles (whole warp, converged) with a grid whose
+ * near cells are marked, one particle after another by the whole warp. */
+__device__ __forceinline__ float3 force_contact_warp(const FgScene *S, bool active, float4 p, float4 v,
+                                                     const RigidGrid &G, bool dynamic)
+{
+    float3 c = make_float3(0.f, 0.f, 0.f);
+    const ContactShape C(S);
+    for (uint32_t m = __ballot_sync(FG_FULL, active && fg_contact_marked(S, 0u, p, G)); m; m &= m - 1u) {
+        const int b = __ffs((int)m) - 1;
+        const float4 pb = make_float4(__shfl_sync(FG_FULL, p.x, b), __shfl_sync(FG_FULL, p.y, b),
+                                      __shfl_sync(FG_FULL, p.z, b), 1.f);
+        const float4 vb = make_float4(__shfl_sync(FG_FULL, v.x, b), __shfl_sync(FG_FULL, v.y, b),
+                                      __shfl_sync(FG_FULL, v.z, b), 0.f);
+        const float3 r = fg_contact_warp(S, C, pb, vb, G, dynamic);
+        if ((int)(threadIdx.x & 31u) == b) c = r;
+    }
+    return c;
+}
+
+/* Pair terms of one target by a walk over its 27 buckets. */
+__device__ __forceinline__ void walk_terms(const FgScene *S, uint32_t i, float4 p, float4 v, float kv,
+                                           const float4 *__restrict__ spos, const float4 *__restrict__ svel,
+                                           const float2 *__restrict__ dp, const uint32_t *__restrict__ start,
+                                           const uint32_t *__restrict__ end, float &fx, float &fy, float &fz)
+{
+    const float scale = S->scale, h = S->h, h2 = S->h2, kspiky = S->kspiky;
+    const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
+    const float2 di = dp[i];
+    fg_walk27(p.x, p.y, p.z, S, start, end, [&](uint32_t j) {
+        if (j == i) return;
+        const float4 q = __ldg(spos + j);
+        const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
+        if (r2 <= h2) {
+            const float4 vj = __ldg(svel + j);
+            const float2 dj = __ldg(dp + j);
+            fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, di.x, di.y, v, dj.x, dj.y, vj);
+        }
+    });
+}
+
+/* From the summed pair terms to the particle's new velocity (and, fused, its
+ * position): F = internal * mass + gravity + rigid contact, walls, force clamp
+ * (K_FluidSim.cu:287-307, 389-411), newVel[id] = vel + F dt. */
+__device__ __forceinline__ void force_finish(const FgScene *S, float4 p, float4 v, float fx, float fy, float fz,
+                                             float mass, float3 sta, float3 dyn, uint32_t oi,
+                                             float4 *__restrict__ vel_out, float4 *__restrict__ pos_out)
+{
+    float3 F = make_float3(0.f, 0.f, 0.f);
+    if (p.w > 0.0f) {
+        F = make_float3(fx * mass + S->gravity[0], fy * mass + S->gravity[1], fz * mass + S->gravity[2]);
+        F.x += sta.x; F.y += sta.y; F.z += sta.z;
+        F.x += dyn.x; F.y += dyn.y; F.z += dyn.z;
+        const float3 wl = fg_walls(*S, make_float3(p.x, p.y, p.z), make_float3(v.x, v.y, v.z));
+        F.x += wl.x; F.y += wl.y; F.z += wl.z;
+        const float sp2 = F.x * F.x + F.y * F.y + F.z * F.z;
+        const float speed = sqrtf(sp2);
+        if (speed > S->vlimit) {
+            const float t = S->vlimit / speed;
+            F.x *= t; F.y *= t; F.z *= t;
+        }
+    }
+    const float dt = S->dt;
+    float4 nv;
+    nv.x = v.x + F.x * dt;
+    nv.y = v.y + F.y * dt;
+    nv.z = v.z + F.z * dt;
+    nv.w = v.w + 0.0f;
+    vel_out[oi] = nv;
+    if (pos_out && p.w > 0.0f) {
+        /* SPHIntegrateK fused: pos += vel * (dt / scale), unfused rounding */
+        const float c = S->dt_over_scale;
+        float4 np;
+        np.x = __fadd_rn(p.x, __fmul_rn(nv.x, c));
+        np.y = __fadd_rn(p.y, __fmul_rn(nv.y, c));
+        np.z = __fadd_rn(p.z, __fmul_rn(nv.z, c));
+        np.w = __fadd_rn(p.w, __fmul_rn(nv.w, c));
+        pos_out[oi] = np;
+    }
+}
+
+/* The list form of the force pass (kernel 1). */
+template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces(const FgWork *__restrict__ work, uint32_t nwork,
                                                     uint32_t n_single, const FgScene *__restrict__ table,
                                                     const __grid_constant__ FgScene single,
                                                     const float4 *__restrict__ spos, const float4 *__restrict__ svel,
-                                                    const float2 *__restrict__ dp,
                                                     const uint32_t *__restrict__ start,
                                                     const uint32_t *__restrict__ end,
                                                     const uint32_t *__restrict__ ids, float4 *__restrict__ vel_out,
                                                     float4 *__restrict__ pos_out,
-                                                    const __grid_constant__ RigidArgs R, float mass_o, float visc_o,
-                                                    int use_o, const __grid_constant__ NbrList list, TargetOrder ord)
+                                                    const __grid_constant__ RigidArgs R,
+                                                    const __grid_constant__ NbrList list, TargetOrder ord)
 {
     constexpr uint32_t IPC = FG_ITEMS_PER_CTA(BLOCK), PASSES = FG_PASSES(BLOCK);
     const uint32_t sub = IPC > 1u ? threadIdx.x / FG_CHUNK : 0u;
@@ -287,122 +381,270 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces(const FgWork *__r
         const uint32_t i = ord.tord ? __ldg(ord.inv + pid) : tpos;
         const float4 p = spos[i];
         const float4 v = svel[i];
-        float3 F = make_float3(0.f, 0.f, 0.f);
+        float fx = 0.f, fy = 0.f, fz = 0.f;
+        float3 dyn = make_float3(0.f, 0.f, 0.f);
+        const uint32_t oi = ord.tord ? pid : __ldg(ids + i);
         if (p.w > 0.0f) {
             const float scale = S->scale, h = S->h, h2 = S->h2;
-            const float mass = use_o ? mass_o : S->mass;
-            const float visc = use_o ? visc_o : S->visc;
-            const float kspiky = S->kspiky, kv = S->kvisc * visc;
+            const float kspiky = S->kspiky, kv = S->kvisc * S->visc;
             const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
-            float fx = 0.f, fy = 0.f, fz = 0.f;
-            if (LIST) {
-                const float4 r0 = list.rec[2 * i], r1 = list.rec[2 * i + 1];
-                const float rho_i = r0.w, P_i = r1.w;
-                const uint32_t c = list.cnt[i];
-                if (c <= __ldg(list.cap)) {
-                    /* in-range visits in walk order (the target's own
-                     * entries skipped) */
-                    const uint32_t *nl = list.idx + (size_t)i * list.stride;
-                    /* the list is padded with i to whole groups of four */
-                    const uint32_t c4 = (c + 3u) & ~3u;
-                    /* four 32-byte records in flight, one 256-bit load each,
-                     * their target's own entries skipped */
-                    auto group = [&](const uint4 q) {
-                        const uint32_t jj[4] = {q.x, q.y, q.z, q.w};
-                        float4 a[4], b[4];
+            const float4 r0 = list.rec[2 * i], r1 = list.rec[2 * i + 1];
+            const float rho_i = r0.w, P_i = r1.w;
+            const uint32_t c = list.cnt[i];
+            if (c <= __ldg(list.cap)) {
+                /* in-range visits in walk order (the target's own
+                 * entries skipped) */
+                const uint32_t *nl = list.idx + (size_t)i * list.stride;
+                /* the list is padded with i to whole groups of four */
+                const uint32_t c4 = (c + 3u) & ~3u;
+                /* four 32-byte records in flight, one 256-bit load each,
+                 * their target's own entries skipped */
+                auto group = [&](const uint4 q) {
+                    const uint32_t jj[4] = {q.x, q.y, q.z, q.w};
+                    float4 a[4], b[4];
 #pragma unroll
-                        for (int e = 0; e < 4; e++) fg_ld_rec(list.rec + 2 * jj[e], a[e], b[e]);
+                    for (int e = 0; e < 4; e++) fg_ld_rec(list.rec + 2 * jj[e], a[e], b[e]);
 #pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            if (jj[e] != i) {
-                                const float dx = fmaf(-a[e].x, scale, px), dy = fmaf(-a[e].y, scale, py),
-                                            dz = fmaf(-a[e].z, scale, pz);
-                                const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
-                                fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, rho_i, P_i, v, a[e].w, b[e].w,
-                                        b[e]);
-                            }
+                    for (int e = 0; e < 4; e++) {
+                        if (jj[e] != i) {
+                            const float dx = fmaf(-a[e].x, scale, px), dy = fmaf(-a[e].y, scale, py),
+                                        dz = fmaf(-a[e].z, scale, pz);
+                            const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
+                            fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, rho_i, P_i, v, a[e].w, b[e].w,
+                                    b[e]);
                         }
-                    };
-                    /* eight indices (one sector, 32-byte aligned: the stride
-                     * is a multiple of 8) per load, the next eight loading
-                     * while these records do */
-                    uint4 qa = make_uint4(0u, 0u, 0u, 0u), qb = qa;
-                    if (c4) fg_ld_idx8(nl, qa, qb);
-                    for (uint32_t k = 0; k < c4; k += 8) {
-                        const uint4 ca = qa, cb = qb;
-                        if (k + 8u < c4) fg_ld_idx8(nl + k + 8u, qa, qb);
-                        group(ca);
-                        if (k + 4u < c4) group(cb);
                     }
-                } else {
-                    /* more in-range visits than list slots: walk the buckets */
-                    fg_walk27(p.x, p.y, p.z, S, start, end, [&](uint32_t j) {
-                        if (j == i) return;
-                        const float4 q0 = __ldg(list.rec + 2 * j);
-                        const float dx = fmaf(-q0.x, scale, px), dy = fmaf(-q0.y, scale, py),
-                                    dz = fmaf(-q0.z, scale, pz);
-                        const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
-                        if (r2 <= h2) {
-                            const float4 q1 = __ldg(list.rec + 2 * j + 1);
-                            fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, rho_i, P_i, v, q0.w, q1.w, q1);
-                        }
-                    });
+                };
+                /* eight indices (one sector, 32-byte aligned: the stride
+                 * is a multiple of 8) per load, the next eight loading
+                 * while these records do */
+                uint4 qa = make_uint4(0u, 0u, 0u, 0u), qb = qa;
+                if (c4) fg_ld_idx8(nl, qa, qb);
+                for (uint32_t k = 0; k < c4; k += 8) {
+                    const uint4 ca = qa, cb = qb;
+                    if (k + 8u < c4) fg_ld_idx8(nl + k + 8u, qa, qb);
+                    group(ca);
+                    if (k + 4u < c4) group(cb);
                 }
             } else {
-                const float2 di = dp[i];
+                /* more in-range visits than list slots: walk the buckets */
                 fg_walk27(p.x, p.y, p.z, S, start, end, [&](uint32_t j) {
                     if (j == i) return;
-                    const float4 q = __ldg(spos + j);
-                    const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
+                    const float4 q0 = __ldg(list.rec + 2 * j);
+                    const float dx = fmaf(-q0.x, scale, px), dy = fmaf(-q0.y, scale, py),
+                                dz = fmaf(-q0.z, scale, pz);
                     const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
                     if (r2 <= h2) {
-                        const float4 vj = __ldg(svel + j);
-                        const float2 dj = __ldg(dp + j);
-                        fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, di.x, di.y, v, dj.x, dj.y, vj);
+                        const float4 q1 = __ldg(list.rec + 2 * j + 1);
+                        fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, rho_i, P_i, v, q0.w, q1.w, q1);
                     }
                 });
             }
-            F = make_float3(fx * mass + S->gravity[0], fy * mass + S->gravity[1], fz * mass + S->gravity[2]);
-            if (R.use_sta) {
-                float3 c = fg_fluid_rigid_contact(S, it.scene, p, v, R.sta, false);
-                F.x += c.x; F.y += c.y; F.z += c.z;
-            }
-            if (R.use_dyn && (S->flags & FG_SCENE_HAS_RB)) {
-                float3 c = make_float3(0.f, 0.f, 0.f);
-                if (!R.dyn.pre) {
-                    c = fg_fluid_rigid_contact(S, it.scene, p, v, R.dyn, true);
-                } else if (!fg_contact_outside(S, it.scene, p, R.dyn) && fg_contact_marked(S, it.scene, p, R.dyn)) {
-                    const float4 q = R.dyn.pre[ord.tord ? pid : __ldg(ids + i)];
-                    c = make_float3(q.x, q.y, q.z);
-                }
-                F.x += c.x; F.y += c.y; F.z += c.z;
-            }
-            const float3 wl = fg_walls(*S, make_float3(p.x, p.y, p.z), make_float3(v.x, v.y, v.z));
-            F.x += wl.x; F.y += wl.y; F.z += wl.z;
-            const float sp2 = F.x * F.x + F.y * F.y + F.z * F.z;
-            const float speed = sqrtf(sp2);
-            if (speed > S->vlimit) {
-                const float t = S->vlimit / speed;
-                F.x *= t; F.y *= t; F.z *= t;
-            }
+            dyn = force_contact(S, it.scene, p, v, oi, R);
         }
-        const float dt = S->dt;
-        float4 nv;
-        nv.x = v.x + F.x * dt;
-        nv.y = v.y + F.y * dt;
-        nv.z = v.z + F.z * dt;
-        nv.w = v.w + 0.0f;
+        force_finish(S, p, v, fx, fy, fz, S->mass, make_float3(0.f, 0.f, 0.f), dyn, oi, vel_out, pos_out);
+    }
+}
+
+/* The walking form (kernel 0), each thread over its target's 27 buckets: the
+ * same terms in the same order as the list form. */
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces_walk(
+    const FgWork *__restrict__ work, uint32_t nwork, uint32_t n_single, const FgScene *__restrict__ table,
+    const __grid_constant__ FgScene single, const float4 *__restrict__ spos, const float4 *__restrict__ svel,
+    const float2 *__restrict__ dp, const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+    const uint32_t *__restrict__ ids, float4 *__restrict__ vel_out, float4 *__restrict__ pos_out,
+    const __grid_constant__ RigidArgs R, TargetOrder ord)
+{
+    constexpr uint32_t IPC = FG_ITEMS_PER_CTA(BLOCK), PASSES = FG_PASSES(BLOCK);
+    const uint32_t sub = IPC > 1u ? threadIdx.x / FG_CHUNK : 0u;
+    const uint32_t lt = IPC > 1u ? threadIdx.x % FG_CHUNK : threadIdx.x;
+    for (uint32_t w = blockIdx.x * IPC + sub; w < nwork; w += gridDim.x * IPC)
+#pragma unroll 1
+    for (uint32_t ps = 0; ps < PASSES; ps++) {
+        const uint32_t tid = lt + ps * BLOCK;
+        const FgWork it = fg_work(work, w, n_single);
+        if (tid >= it.count) continue;
+        const FgScene *S = fg_scene(table, &single, it.scene);
+        const uint32_t tpos = it.first + tid; /* target slot */
+        const uint32_t pid = ord.tord ? __ldg(ord.tord + tpos) : 0u;
+        const uint32_t i = ord.tord ? __ldg(ord.inv + pid) : tpos;
         const uint32_t oi = ord.tord ? pid : __ldg(ids + i);
-        vel_out[oi] = nv;
-        if (pos_out && p.w > 0.0f) {
-            /* SPHIntegrateK fused: pos += vel * (dt / scale), unfused rounding */
-            const float c = S->dt_over_scale;
-            float4 np;
-            np.x = __fadd_rn(p.x, __fmul_rn(nv.x, c));
-            np.y = __fadd_rn(p.y, __fmul_rn(nv.y, c));
-            np.z = __fadd_rn(p.z, __fmul_rn(nv.z, c));
-            np.w = __fadd_rn(p.w, __fmul_rn(nv.w, c));
-            pos_out[oi] = np;
+        const float4 p = spos[i];
+        const float4 v = svel[i];
+        float fx = 0.f, fy = 0.f, fz = 0.f;
+        float3 dyn = make_float3(0.f, 0.f, 0.f);
+        if (p.w > 0.0f) {
+            walk_terms(S, i, p, v, S->kvisc * S->visc, spos, svel, dp, start, end, fx, fy, fz);
+            dyn = force_contact(S, it.scene, p, v, oi, R);
+        }
+        force_finish(S, p, v, fx, fy, fz, S->mass, make_float3(0.f, 0.f, 0.f), dyn, oi, vel_out, pos_out);
+    }
+}
+
+/* The form without lists (the reference-named launchers).  A warp takes its
+ * targets' cells one after another: it stages a cell's candidates as in the
+ * density pass, with velocity, density and pressure, then tests them for two
+ * targets at a time, a candidate a lane, and compacts the hits, so that the
+ * pair terms, four times a test's work for one candidate in four, run with all
+ * lanes busy; a shuffle tree adds them.  (A walk by thread takes the pair
+ * branch on nearly every candidate for a few of its lanes, and waits there for
+ * the neighbour's velocity and density: 83 us at 33,333 particles of 0.5 h
+ * spacing, 1381 us at 1,048,576 of 0.4 h; here 30 and 917.  Hits queued per
+ * thread and drained together, 1923: lanes of a cell lose the loads that they
+ * share while they walk in step.  Hits taken by a lane per target, 1268: their
+ * numbers differ by lane and round.)  192 staged candidates leave twelve CTAs
+ * an SM: 256, 991 us; 128, 1073.  The rigid contact follows by warp, for the
+ * particles in cells marked near a sphere; walked by every particle, it was
+ * three quarters of the 660 us at 262,144 particles (215 now). */
+#ifndef FG_FORCE_STAGE
+#define FG_FORCE_STAGE 192u
+#endif
+#ifndef FG_FORCE_CTAS
+#define FG_FORCE_CTAS 12
+#endif
+#define FG_FORCE_THREADS 64u
+struct ForceShared {
+    float4 a[FG_FORCE_STAGE];         /* x, y, z, rho */
+    float4 b[FG_FORCE_STAGE];         /* vx, vy, vz, P */
+    uint32_t j[FG_FORCE_STAGE];       /* sorted index */
+    uint16_t hit[2][FG_FORCE_STAGE];  /* two targets' slots in range */
+    uint32_t idx[FG_STAGE_WINDOW];
+};
+
+__global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_search(
+    uint32_t n_all, const __grid_constant__ FgScene scene, uint32_t range, const float4 *__restrict__ spos,
+    const float4 *__restrict__ svel, const float2 *__restrict__ dp, const uint32_t *__restrict__ start,
+    const uint32_t *__restrict__ end, const uint32_t *__restrict__ ids, float4 *__restrict__ vel_out,
+    float4 *__restrict__ pos_out, const __grid_constant__ RigidArgs R, float mass, float visc)
+{
+    __shared__ ForceShared shared[FG_FORCE_THREADS / 32];
+    ForceShared &sm = shared[threadIdx.x >> 5];
+    const FgScene *S = &scene;
+    const StageGrid G(S);
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lt = (1u << lane) - 1u;
+    const float scale = S->scale, h = S->h, h2 = S->h2;
+    const float kspiky = S->kspiky, kv = S->kvisc * visc;
+    for (uint32_t b0 = (blockIdx.x * (FG_FORCE_THREADS / 32u) + (threadIdx.x >> 5)) * range; b0 < n_all;
+         b0 += gridDim.x * (FG_FORCE_THREADS / 32u) * range) {
+        uint32_t next, stop;
+        fg_stage_range(b0, range, 0u, n_all, G, spos, next, stop);
+        while (next < stop) {
+            const uint32_t i0 = next, i = next + lane; /* sorted index */
+            uint32_t n = min(32u, stop - next);
+            const float4 p = lane < n ? spos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const StageSig sig = fg_stage_sig(p, G);
+            if (stop - next > 32u) n = fg_stage_trim(sig, __ldg(spos + next + 32u), G);
+            next += n;
+            const bool valid = lane < n;
+            const bool active = valid && p.w > 0.0f;
+            const float4 v = valid ? svel[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float2 di = active ? dp[i] : make_float2(1.f, 0.f);
+            const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
+            float fx = 0.f, fy = 0.f, fz = 0.f;
+            uint32_t lead, leads;
+            fg_stage_groups(sig, __ballot_sync(FG_FULL, active && !sig.odd), 32u, lead, leads);
+            for (; leads; leads &= leads - 1u) {
+                const uint32_t l = (uint32_t)__ffs((int)leads) - 1u;
+                const uint32_t group = __ballot_sync(FG_FULL, lead == l);
+                fg_stage_rounds<FG_FORCE_STAGE>(
+                    sig, lead, 1u << l, px, py, pz, G, spos, start, end, sm.idx,
+                    [&](uint32_t slot, uint32_t j, float4 c) {
+                        sm.a[slot] = c;
+                        sm.j[slot] = j;
+                    },
+                    [&](uint32_t, uint32_t, uint32_t used) {
+#pragma unroll 4
+                        for (uint32_t s = lane; s < used; s += 32u) {
+                            const uint32_t j = sm.j[s];
+                            const float4 w = __ldg(svel + j);
+                            const float2 d = __ldg(dp + j);
+                            sm.b[s] = make_float4(w.x, w.y, w.z, d.y);
+                            sm.a[s].w = d.x;
+                        }
+                        __syncwarp();
+                        for (uint32_t g = group; g;) {
+                            int t[2];
+                            float tx[2], ty[2], tz[2];
+                            uint32_t cnt[2] = {0u, 0u};
+                            t[0] = __ffs((int)g) - 1;
+                            g &= g - 1u;
+                            const bool two = g != 0u;
+                            t[1] = two ? __ffs((int)g) - 1 : t[0];
+                            if (two) g &= g - 1u;
+#pragma unroll
+                            for (int u = 0; u < 2; u++) {
+                                tx[u] = __shfl_sync(FG_FULL, px, t[u]);
+                                ty[u] = __shfl_sync(FG_FULL, py, t[u]);
+                                tz[u] = __shfl_sync(FG_FULL, pz, t[u]);
+                            }
+                            for (uint32_t s0 = 0u; s0 < used; s0 += 32u) {
+                                const uint32_t s = s0 + lane;
+                                const float4 q = sm.a[min(s, FG_FORCE_STAGE - 1u)];
+                                const uint32_t j = s < used ? sm.j[s] : 0xffffffffu;
+#pragma unroll
+                                for (int u = 0; u < 2; u++) {
+                                    const float dx = fmaf(-q.x, scale, tx[u]), dy = fmaf(-q.y, scale, ty[u]),
+                                                dz = fmaf(-q.z, scale, tz[u]);
+                                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
+                                    const bool in = r2 <= h2 && s < used && j != i0 + (uint32_t)t[u] && (u == 0 || two);
+                                    const uint32_t m = __ballot_sync(FG_FULL, in);
+                                    if (in) sm.hit[u][cnt[u] + (uint32_t)__popc(m & lt)] = (uint16_t)s;
+                                    cnt[u] += (uint32_t)__popc(m);
+                                }
+                            }
+                            __syncwarp();
+                            float f[2][3];
+#pragma unroll
+                            for (int u = 0; u < 2; u++) {
+                                f[u][0] = f[u][1] = f[u][2] = 0.f;
+                                const float rho_t = __shfl_sync(FG_FULL, di.x, t[u]),
+                                            P_t = __shfl_sync(FG_FULL, di.y, t[u]);
+                                const float4 vt = make_float4(__shfl_sync(FG_FULL, v.x, t[u]),
+                                                              __shfl_sync(FG_FULL, v.y, t[u]),
+                                                              __shfl_sync(FG_FULL, v.z, t[u]), 0.f);
+                                for (uint32_t k = lane; k < cnt[u]; k += 32u) {
+                                    const uint32_t s = sm.hit[u][k];
+                                    const float4 a = sm.a[s], b = sm.b[s];
+                                    const float dx = fmaf(-a.x, scale, tx[u]), dy = fmaf(-a.y, scale, ty[u]),
+                                                dz = fmaf(-a.z, scale, tz[u]);
+                                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
+                                    fg_pair(f[u][0], f[u][1], f[u][2], dx, dy, dz, r2, h, kspiky, kv, rho_t, P_t, vt,
+                                            a.w, b.w, b);
+                                }
+                            }
+                            __syncwarp();
+                            /* two targets' sums: one exchange leaves each half
+                             * of the warp one target, a tree adds it up */
+                            const bool hi = lane & 16u;
+                            float r[3];
+#pragma unroll
+                            for (int c = 0; c < 3; c++) {
+                                r[c] = __fadd_rn(hi ? f[1][c] : f[0][c],
+                                                 __shfl_xor_sync(FG_FULL, hi ? f[0][c] : f[1][c], 16));
+#pragma unroll
+                                for (int o = 8; o; o >>= 1) r[c] = __fadd_rn(r[c], __shfl_xor_sync(FG_FULL, r[c], o));
+                            }
+#pragma unroll
+                            for (int u = 0; u < 2; u++) {
+                                const float x = __shfl_sync(FG_FULL, r[0], 16 * u), y = __shfl_sync(FG_FULL, r[1], 16 * u),
+                                            z = __shfl_sync(FG_FULL, r[2], 16 * u);
+                                if ((int)lane == t[u] && (u == 0 || two)) {
+                                    fx = __fadd_rn(fx, x);
+                                    fy = __fadd_rn(fy, y);
+                                    fz = __fadd_rn(fz, z);
+                                }
+                            }
+                        }
+                    });
+            }
+            if (active && sig.odd) walk_terms(S, i, p, v, kv, spos, svel, dp, start, end, fx, fy, fz);
+            __syncwarp();
+            float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
+            if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false);
+            if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true);
+            if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, __ldg(ids + i), vel_out, pos_out);
         }
     }
 }
@@ -417,22 +659,30 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
     memset(&R, 0, sizeof(R));
     if (rigid) { R.dyn = *rigid; R.use_dyn = 1; }
     if (statics) { R.sta = *statics; R.use_sta = 1; }
-    NbrList none;
-    memset(&none, 0, sizeof(none));
-    const NbrList &nl = list ? *list : none;
+    if (!list && use_o) {
+        const uint32_t range = stage_range(L.nwork), warps = (L.n + range - 1u) / range;
+        const uint32_t per_cta = FG_FORCE_THREADS / 32u;
+        k_forces_search<<<grid_for((warps + per_cta - 1u) / per_cta, 128), FG_FORCE_THREADS, 0, L.stream>>>(
+            L.n, *L.single, range, spos, svel, dp, start, end, ids, out.vel, out.pos, R, mass_o, visc_o);
+        return;
+    }
     const uint32_t B = L.block ? L.block : FG_CHUNK;
     const uint32_t ipc = FG_ITEMS_PER_CTA(B);
     const int per_sm = (int)(((L.ctas_per_sm ? L.ctas_per_sm : 64u) * FG_CHUNK) / B);
     const uint32_t g = grid_for((L.nwork + ipc - 1u) / ipc, per_sm > 0 ? per_sm : 1);
-#define FG_FORCES(LI, BL)                                                                                        \
-    k_forces<LI, BL><<<g, BL, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, spos, svel, dp, start, end, \
-                                             ids, out.vel, out.pos, R, mass_o, visc_o, use_o, nl, ord)
+#define FG_FORCES(BL)                                                                                              \
+    if (list)                                                                                                      \
+        k_forces<BL><<<g, BL, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, spos, svel, start, end, ids, \
+                                             out.vel, out.pos, R, *list, ord);                                     \
+    else                                                                                                           \
+        k_forces_walk<BL><<<g, BL, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, spos, svel, dp, start, \
+                                                  end, ids, out.vel, out.pos, R, ord)
     if (B == 64u) {
-        if (list) FG_FORCES(true, 64); else FG_FORCES(false, 64);
+        FG_FORCES(64);
     } else if (B == 256u) {
-        if (list) FG_FORCES(true, 256); else FG_FORCES(false, 256);
+        FG_FORCES(256);
     } else {
-        if (list) FG_FORCES(true, 128); else FG_FORCES(false, 128);
+        FG_FORCES(128);
     }
 #undef FG_FORCES
 }
