@@ -636,7 +636,7 @@ void World::enqueue_rb_grid(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches
         radix_sort(rb_keys_u, nullptr, rb_keys, rb_ids, nspheres, rb_key_bits, 8, rs, st);
         cudaMemsetAsync(rb_start, 0xff, 4 * (size_t)total_rb_buckets, st);
         launch_cell_ranges(rb_keys, rb_ids, rb_world, nullptr, rb_start, rb_end, rb_spos, nullptr, nspheres, st);
-        launches += 3 + 3 * radix_passes(rb_key_bits, 8);
+        launches += 3 + radix_launches(nspheres, rb_key_bits, 8);
     }
     if (ev) cudaEventRecord(ev[9], st);
 }
@@ -722,7 +722,7 @@ uint32_t World::sort_launches() const
      * step hashes too */
     if (bucket_sort_on && bucket_sort_fits()) return n ? ((stages & FG_STAGE_HASH) ? 4u : 5u) : 2u;
     const uint32_t P = (uint32_t)radix_passes(key_bits, digit_bits);
-    return (one_pass_sort && n && P <= 6) ? 2 + P : 3 * P;
+    return (one_pass_sort && n && P <= 6) ? 2 + P : (P ? radix_launches(n, key_bits, digit_bits) : 0u);
 }
 
 /* The hash pass; when the counting sort follows, it counts the keys too. */
@@ -915,7 +915,7 @@ void World::enqueue_order_refresh()
     if (!n) return;
     launch_morton_keys(fluid_launch(), pos, keys, order_bits, order_scene_shift);
     radix_sort(keys, nullptr, keys_u, tord, n, order_key_bits, digit_bits, rs, stream);
-    kernels_enqueued += 1 + 3 * (uint64_t)radix_passes(order_key_bits, digit_bits);
+    kernels_enqueued += 1 + (uint64_t)radix_launches(n, order_key_bits, digit_bits);
     order_valid = true;
 }
 
@@ -1376,7 +1376,7 @@ uint32_t World::launches_per_step()
     if (stages & FG_STAGE_DENSITY) c += 1;
     if (nbodies) {
         if (stages & FG_STAGE_RB_GRID) /* aabb reset, hash, sort + ranges */
-            c += rb_small_scenes ? 3 : 3 + 3 * radix_passes(rb_key_bits, 8);
+            c += rb_small_scenes ? 3 : 3 + radix_launches(nspheres, rb_key_bits, 8);
         if (stages & FG_STAGE_RB_CONTACT) c += 1 + (any_rb_rb ? 1 : 0) + (fluid_contact_pass() ? 1 : 0);
         if (stages & FG_STAGE_BODIES) c += body_launches();
     }

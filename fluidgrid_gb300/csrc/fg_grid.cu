@@ -8,6 +8,7 @@
  * entries.  All kernels stream coalesced 16-byte loads; the sort is a
  * reduce-then-scan LSD radix sort whose CTAs never wait on one another. */
 #include <cuda_runtime.h>
+#include <cooperative_groups.h>
 #include <stdint.h>
 #include <algorithm>
 #include "fg_device.cuh"
@@ -153,7 +154,7 @@ void launch_hash_with_offset(const Launch &L, const float4 *local, const float4 
  * LSD radix sort, up to 8 bits per pass, tiles of RS_TILE keys:
  *   upsweep   per-tile digit counts          hist[d * T + t]
  *   scan      per digit, exclusive over tiles  (one CTA per digit) + totals
- *   downsweep stable in-tile ranking (warp match_any), shared-memory
+ *   downsweep stable in-tile ranking (a ballot a bit), shared-memory
  *             staging in digit order, coalesced scatter.
  * Ranks within a tile follow particle order (warp w holds keys
  * [w*512, w*512+512) of the tile, item k of lane l is key w*512 + 32k + l and
@@ -179,18 +180,44 @@ int radix_passes(uint32_t bits, uint32_t digit_bits)
     return (int)((bits + digit_bits - 1) / digit_bits);
 }
 
+/* The lanes of the warp whose digit (of `bits` bits) is the same: a ballot a
+ * bit.  match_any takes a round for each distinct value of the warp: with it
+ * the downsweep of 700,000 pairs took 11.4 us, with the ballots 9.2. */
+__device__ __forceinline__ uint32_t rs_peers(uint32_t d, uint32_t bits)
+{
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (uint32_t b = 0; b < 8u; b++)
+        if (b < bits) {
+            const bool one = d >> b & 1u;
+            const uint32_t m = __ballot_sync(0xffffffffu, one);
+            peers &= one ? m : ~m;
+        }
+    return peers;
+}
+
+/* keep_k, keep_v (optional): copies of the pass's input */
 __global__ void __launch_bounds__(RS_THREADS) k_rs_upsweep(const uint32_t *__restrict__ keys, uint32_t n,
                                                           uint32_t shift, uint32_t mask, uint32_t *__restrict__ hist,
-                                                          uint32_t T)
+                                                          uint32_t T, const uint32_t *__restrict__ vals,
+                                                          uint32_t *__restrict__ keep_k,
+                                                          uint32_t *__restrict__ keep_v)
 {
     __shared__ uint32_t cnt[RS_RADIX];
     cnt[threadIdx.x] = 0;
     __syncthreads();
     size_t base = (size_t)blockIdx.x * RS_TILE;
-#pragma unroll 4
+#pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
         size_t i = base + (size_t)k * RS_THREADS + threadIdx.x;
-        if (i < n) atomicAdd(&cnt[(__ldg(keys + i) >> shift) & mask], 1u);
+        if (i < n) {
+            const uint32_t key = __ldg(keys + i);
+            atomicAdd(&cnt[(key >> shift) & mask], 1u);
+            if (keep_k) {
+                keep_k[i] = key;
+                keep_v[i] = vals ? __ldg(vals + i) : (uint32_t)i;
+            }
+        }
     }
     __syncthreads();
     hist[(size_t)threadIdx.x * T + blockIdx.x] = cnt[threadIdx.x];
@@ -273,27 +300,26 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const uint32_t *__r
 
     uint32_t key[RS_ITEMS], val[RS_ITEMS], rank[RS_ITEMS];
     const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t bits = (uint32_t)__popc(mask);
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
-        size_t i = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane;
-        bool valid = i < n;
-        key[k] = valid ? __ldg(kin + i) : 0xffffffffu;
-        val[k] = valid ? (vin ? __ldg(vin + i) : (uint32_t)i) : 0u;
-        uint32_t active = __ballot_sync(0xffffffffu, valid);
-        uint32_t r = 0;
-        if (valid) {
-            uint32_t d = (key[k] >> shift) & mask;
-            uint32_t peers = __match_any_sync(active, d);
-            uint32_t leader = __ffs(peers) - 1;
-            uint32_t b = 0;
-            if (lane == leader) {
-                b = s_whist[wid][d];
-                s_whist[wid][d] = b + __popc(peers);
-            }
-            b = __shfl_sync(active, b, leader);
-            r = b + __popc(peers & lt);
+        const size_t i = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane;
+        key[k] = i < n ? __ldg(kin + i) : 0xffffffffu;
+        val[k] = i < n ? (vin ? __ldg(vin + i) : (uint32_t)i) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; k++) {
+        const bool valid = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane < n;
+        const uint32_t d = (key[k] >> shift) & mask;
+        const uint32_t peers = rs_peers(d, bits) & __ballot_sync(0xffffffffu, valid);
+        const uint32_t leader = valid ? (uint32_t)__ffs((int)peers) - 1u : lane;
+        uint32_t b = 0;
+        if (valid && lane == leader) {
+            b = s_whist[wid][d];
+            s_whist[wid][d] = b + __popc(peers);
         }
-        rank[k] = r;
+        b = __shfl_sync(0xffffffffu, b, (int)leader);
+        rank[k] = b + __popc(peers & lt);
         __syncwarp();
     }
     __syncthreads();
@@ -341,6 +367,188 @@ __global__ void k_iota_copy(const uint32_t *__restrict__ kin, const uint32_t *__
     }
 }
 
+/* ---- up to 65,536 pairs: the whole sort in one launch ----
+ * One cluster of up to eight CTAs keeps the pairs on chip: ITEMS a thread in
+ * registers, ranked in the CTA as k_rs_downsweep does; the CTAs read one
+ * another's digit totals, order their tile by digit in shared memory and write
+ * its runs into one another's, two cluster barriers a pass, 8 bits a pass.  A
+ * digit that all keys share is skipped (a 32-bit sort of small keys).  The
+ * three kernels a pass above are, at these sizes, launches and latency.
+ * Measured in a captured graph, three kernels a pass before (with a
+ * match_any a key) -> one launch, 17 bits: 39.9 -> 10.9 us at 4,096 pairs,
+ * 40.6 -> 15.9 at 16,384, 42.4 -> 23.8 at 32,768, 42.7 -> 32.4 at 65,536; 32
+ * bits, no digit shared: 52 -> 14.2, 21.1, 32.0, 56 -> 44.6.  The time is the
+ * ranking and the staging of eight pairs a thread on eight SMs by then.
+ * Scattering each pair straight into the other CTA's memory, a word at a time,
+ * took 43.3 us at 65,536 pairs of 17 bits: 32 destinations a warp. */
+#define CS_THREADS 1024
+#define CS_CTAS 8u
+
+template <int ITEMS>
+struct ClusterSort {
+    uint2 stage[CS_THREADS * ITEMS]; /* the tile's pairs by digit */
+    uint2 pair[CS_THREADS * ITEMS];  /* the cluster's, from any CTA */
+    uint16_t whist[CS_THREADS / 32][RS_RADIX];
+    uint32_t part[4][RS_RADIX];
+    uint32_t tot[2][RS_RADIX]; /* of alternate passes: the cluster may still read the one before */
+    uint32_t goff[RS_RADIX], loff[RS_RADIX]; /* a digit's first place in the cluster and in the stage */
+    uint32_t wsum[2 * RS_RADIX / 32];
+    uint32_t same[2];
+};
+
+template <int ITEMS>
+__global__ void __launch_bounds__(CS_THREADS, 1) k_sort_cluster(const uint32_t *kin, const uint32_t *vin,
+                                                               uint32_t *kout, uint32_t *vout, uint32_t n,
+                                                               uint32_t bits) /* kout may be kin, vout vin */
+{
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char smem[];
+    ClusterSort<ITEMS> &S = *reinterpret_cast<ClusterSort<ITEMS> *>(smem);
+    cg::cluster_group cl = cg::this_cluster();
+    constexpr uint32_t TILE = CS_THREADS * ITEMS;
+    const uint32_t me = cl.block_rank(), ctas = cl.num_blocks(), all = ctas * TILE;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, lt = (1u << lane) - 1u;
+    const uint32_t mine = wid * 32u * ITEMS + lane; /* item k: mine + 32 k of the tile */
+    uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        /* past the end: the largest key, after all equal ones */
+        const uint32_t i = me * TILE + mine + 32u * k;
+        key[k] = i < n ? kin[i] : 0xffffffffu;
+        val[k] = i < n ? (vin ? vin[i] : i) : 0u;
+    }
+    uint32_t turn = 0u;
+    for (uint32_t shift = 0u; shift < bits; shift += 8u, turn ^= 1u) {
+        const uint32_t db = min(8u, bits - shift), mask = (1u << db) - 1u;
+        for (uint32_t w = tid; w < sizeof(S.whist) / 4u; w += CS_THREADS) ((uint32_t *)S.whist)[w] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint32_t d = key[k] >> shift & mask, peers = rs_peers(d, db);
+            const uint32_t b = S.whist[wid][d];
+            __syncwarp();
+            if ((peers & lt) == 0u) S.whist[wid][d] = (uint16_t)(b + __popc(peers));
+            rank[k] = b + __popc(peers & lt);
+            __syncwarp();
+        }
+        __syncthreads();
+        /* per digit: exclusive over the warps, eight of them a thread */
+        const uint32_t d = tid & 255u, q = tid >> 8;
+        uint32_t run = 0u, c[8];
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            c[w] = S.whist[8u * q + w][d];
+            run += c[w];
+        }
+        S.part[q][d] = run;
+        __syncthreads();
+        uint32_t before = 0u;
+        for (uint32_t r = 0; r < q; r++) before += S.part[r][d];
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            S.whist[8u * q + w][d] = (uint16_t)before;
+            before += c[w];
+        }
+        if (q == 3u) S.tot[turn][d] = before;
+        cl.sync();
+        /* each digit's first place: of all its pairs and of the tile's among
+         * them (threads 0 to 255), and in the staged tile (the next 256) */
+        uint32_t ahead = 0u, total = 0u;
+        if (tid < RS_RADIX) {
+            for (uint32_t r = 0; r < ctas; r++) {
+                const uint32_t t = *cl.map_shared_rank(&S.tot[turn][d], (int)r);
+                total += t;
+                if (r < me) ahead += t;
+            }
+            if (tid == 0u) S.same[turn] = 0u;
+        } else if (tid < 2 * RS_RADIX) {
+            total = S.tot[turn][d];
+        }
+        uint32_t incl = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (tid < 2 * RS_RADIX && lane == 31u) S.wsum[wid] = incl;
+        __syncthreads();
+        if (tid < 2 * RS_RADIX) {
+            uint32_t base = incl - total;
+            for (uint32_t w = wid & ~(RS_RADIX / 32u - 1u); w < wid; w++) base += S.wsum[w];
+            (tid < RS_RADIX ? S.goff : S.loff)[d] = base + ahead;
+            /* all n keys in one digit: those past the end stay behind them */
+            if (tid < RS_RADIX && total - (d == mask ? all - n : 0u) == n) S.same[turn] = 1u;
+        }
+        __syncthreads();
+        if (S.same[turn]) continue; /* the same decision in every CTA */
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint32_t dk = key[k] >> shift & mask;
+            S.stage[S.loff[dk] + S.whist[wid][dk] + rank[k]] = make_uint2(key[k], val[k]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint32_t i = tid + (uint32_t)k * CS_THREADS;
+            const uint2 kv = S.stage[i];
+            const uint32_t dk = kv.x >> shift & mask, g = S.goff[dk] + (i - S.loff[dk]);
+            *cl.map_shared_rank(&S.pair[g % TILE], (int)(g / TILE)) = kv;
+        }
+        cl.sync();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint2 kv = S.pair[mine + 32u * k];
+            key[k] = kv.x;
+            val[k] = kv.y;
+        }
+    }
+    /* every CTA has its input in registers since the first barrier (in place) */
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint32_t i = me * TILE + mine + 32u * k;
+        if (i < n) {
+            kout[i] = key[k];
+            vout[i] = val[k];
+        }
+    }
+    cl.sync(); /* no CTA leaves while another may read its totals */
+}
+
+template <int ITEMS>
+static cudaError_t cluster_sort(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, uint32_t n,
+                                uint32_t bits, cudaStream_t st)
+{
+    const size_t smem = sizeof(ClusterSort<ITEMS>);
+    cudaError_t e = cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return e;
+    uint32_t ctas = 1u;
+    while (ctas * CS_THREADS * ITEMS < n) ctas <<= 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(CS_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_sort_cluster<ITEMS>, kin, vin, kout, vout, n, bits);
+}
+
+/* Pairs that one launch sorts.  The three kernels a pass, over the whole chip,
+ * take 34.6 us for one pair more (17 bits; 32 bits: 44.2), where the cluster
+ * takes 32.4 (44.6, and less with each digit it skips); below that theirs
+ * stay at that latency. */
+#define CS_MAX (CS_CTAS * CS_THREADS * 8u)
+
+uint32_t radix_launches(uint32_t n, uint32_t bits, uint32_t digit_bits)
+{
+    return n <= CS_MAX ? 1u : 3u * (uint32_t)radix_passes(bits, digit_bits);
+}
+
 cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
                        uint32_t n, uint32_t bits, uint32_t digit_bits, const RadixScratch &s, cudaStream_t st)
 {
@@ -353,33 +561,43 @@ cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_
             k_iota_copy<<<grid_for((n + 255) / 256, 8), 256, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n);
         return cudaSuccess;
     }
+    if (n <= CS_MAX) {
+        /* as many CTAs as give each thread one pair, up to eight CTAs */
+        const uint32_t per = CS_CTAS * CS_THREADS;
+        if (n <= per) return cluster_sort<1>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
+        if (n <= 2u * per) return cluster_sort<2>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
+        if (n <= 4u * per) return cluster_sort<4>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
+        return cluster_sort<8>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
+    }
     const uint32_t T = (n + RS_TILE - 1) / RS_TILE;
     uint32_t *totals = s.hist + (size_t)RS_RADIX * T;
-    const bool inplace = (keys_in == keys_out);
-    /* choose the first destination so the last pass lands in *_out */
+    /* the last pass lands in *_out: an odd number of passes starts towards it,
+     * from the input or, in place, from a copy that the first upsweep leaves
+     * in the scratch */
+    const bool copy = P % 2 == 1 && keys_in == keys_out;
     const uint32_t *kin = keys_in;
     const uint32_t *vin = vals_in;
-    bool to_out = (P % 2 == 1) && !inplace;
+    bool to_out = P % 2 == 1;
     for (int p = 0; p < P; p++) {
         uint32_t shift = (uint32_t)p * digit_bits;
         uint32_t b = std::min(digit_bits, bits - shift);
         uint32_t mask = (1u << b) - 1u;
         uint32_t *ko = to_out ? keys_out : s.keys_alt;
         uint32_t *vo = to_out ? vals_out : s.vals_alt;
-        k_rs_upsweep<<<T, RS_THREADS, 0, st>>>(kin, n, shift, mask, s.hist, T);
+        const bool keep = copy && p == 0;
+        k_rs_upsweep<<<T, RS_THREADS, 0, st>>>(kin, n, shift, mask, s.hist, T, vin, keep ? s.keys_alt : nullptr,
+                                               keep ? s.vals_alt : nullptr);
+        if (keep) {
+            kin = s.keys_alt;
+            vin = s.vals_alt;
+        }
         k_rs_scan<<<RS_RADIX, RS_THREADS, 0, st>>>(s.hist, T, totals);
         k_rs_downsweep<<<T, RS_THREADS, 0, st>>>(kin, vin, ko, vo, n, shift, mask, s.hist, totals, T);
         kin = ko;
         vin = vo;
         to_out = !to_out;
     }
-    cudaError_t e = cudaSuccess;
-    if (kin != keys_out) {
-        e = cudaMemcpyAsync(keys_out, kin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
-        const cudaError_t e2 = cudaMemcpyAsync(vals_out, vin, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = e2;
-    }
-    return e;
+    return cudaSuccess;
 }
 
 /* ------------------------------------------- counting sort by bucket
@@ -671,27 +889,26 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_pass(const uint32_t *__restri
 
     uint32_t key[RS_ITEMS], val[RS_ITEMS], rank[RS_ITEMS];
     const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t bits = (uint32_t)__popc(mask);
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
-        size_t i = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane;
-        bool valid = i < n;
-        key[k] = valid ? __ldg(kin + i) : 0xffffffffu;
-        val[k] = valid ? (vin ? __ldg(vin + i) : (uint32_t)i) : 0u;
-        uint32_t active = __ballot_sync(0xffffffffu, valid);
-        uint32_t r = 0;
-        if (valid) {
-            uint32_t d = (key[k] >> shift) & mask;
-            uint32_t peers = __match_any_sync(active, d);
-            uint32_t leader = __ffs(peers) - 1;
-            uint32_t b = 0;
-            if (lane == leader) {
-                b = s_whist[wid][d];
-                s_whist[wid][d] = b + __popc(peers);
-            }
-            b = __shfl_sync(active, b, leader);
-            r = b + __popc(peers & lt);
+        const size_t i = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane;
+        key[k] = i < n ? __ldg(kin + i) : 0xffffffffu;
+        val[k] = i < n ? (vin ? __ldg(vin + i) : (uint32_t)i) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < RS_ITEMS; k++) {
+        const bool valid = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane < n;
+        const uint32_t d = (key[k] >> shift) & mask;
+        const uint32_t peers = rs_peers(d, bits) & __ballot_sync(0xffffffffu, valid);
+        const uint32_t leader = valid ? (uint32_t)__ffs((int)peers) - 1u : lane;
+        uint32_t b = 0;
+        if (valid && lane == leader) {
+            b = s_whist[wid][d];
+            s_whist[wid][d] = b + __popc(peers);
         }
-        rank[k] = r;
+        b = __shfl_sync(0xffffffffu, b, (int)leader);
+        rank[k] = b + __popc(peers & lt);
         __syncwarp();
     }
     __syncthreads();

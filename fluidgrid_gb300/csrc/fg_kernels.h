@@ -45,6 +45,8 @@ struct RadixScratch {
 };
 size_t radix_hist_words(uint32_t n);
 int radix_passes(uint32_t bits, uint32_t digit_bits);
+/* kernel launches of a radix_sort */
+uint32_t radix_launches(uint32_t n, uint32_t bits, uint32_t digit_bits);
 /* One-kernel-per-pass variant (decoupled look-back) for the world's fluid
  * sort: same result as radix_sort with vals_in = 0..n-1.  os is
  * onesweep_words(n) words of scratch; err receives FG_DEV_SORT_TIMEOUT if a
@@ -56,9 +58,9 @@ bool onesweep_sort(const uint32_t *keys_in, uint32_t *keys_out, uint32_t *vals_o
                    uint32_t digit_bits, const RadixScratch &s, uint32_t *os, uint32_t *err, cudaStream_t st);
 /* Stable ascending sort of (key, value) by the low `bits` bits of the key.
  * vals_in == nullptr means values 0..n-1.  keys_out/vals_out may alias
- * keys_in/vals_in (in-place).  Returns the status of the device-to-device
- * copies an odd pass count in place ends with (kernel launch errors are
- * left for cudaGetLastError). */
+ * keys_in/vals_in (in-place).  Up to 65,536 pairs take one launch (8-bit
+ * digits), whose status it returns; other kernel launch errors are left for
+ * cudaGetLastError. */
 cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
                 uint32_t n, uint32_t bits, uint32_t digit_bits, const RadixScratch &s, cudaStream_t st);
 
