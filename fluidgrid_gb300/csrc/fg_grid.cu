@@ -384,12 +384,60 @@ __global__ void k_iota_copy(const uint32_t *__restrict__ kin, const uint32_t *__
 #define CS_THREADS 1024
 #define CS_CTAS 8u
 
+struct TileRank {
+    uint16_t whist[CS_THREADS / 32][RS_RADIX];
+    uint32_t part[4][RS_RADIX];
+};
+
+/* One digit of a CTA's tile (item k of lane l of warp w is pair
+ * (w * ITEMS + k) * 32 + l): rank[] is each pair's place among its warp's of
+ * the digit, R.whist[w][d] how many the warps before w hold; returns, in the
+ * last 256 threads, the tile's count of digit threadIdx.x & 255.  A warp with
+ * `idle` holds no pairs. */
+template <int ITEMS>
+__device__ __forceinline__ uint32_t rs_tile_rank(TileRank &R, const uint32_t (&key)[ITEMS], uint32_t (&rank)[ITEMS],
+                                                 uint32_t shift, uint32_t db, bool idle)
+{
+    const uint32_t tid = threadIdx.x, wid = tid >> 5, lt = (1u << (tid & 31u)) - 1u, mask = (1u << db) - 1u;
+    for (uint32_t w = tid; w < sizeof(R.whist) / 4u; w += CS_THREADS) ((uint32_t *)R.whist)[w] = 0u;
+    __syncthreads();
+    if (!idle) {
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint32_t d = key[k] >> shift & mask, peers = rs_peers(d, db);
+            const uint32_t b = R.whist[wid][d];
+            __syncwarp();
+            if ((peers & lt) == 0u) R.whist[wid][d] = (uint16_t)(b + __popc(peers));
+            rank[k] = b + __popc(peers & lt);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    /* per digit: exclusive over the warps, eight of them a thread */
+    const uint32_t d = tid & 255u, q = tid >> 8;
+    uint32_t run = 0u, c[8];
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        c[w] = R.whist[8u * q + w][d];
+        run += c[w];
+    }
+    R.part[q][d] = run;
+    __syncthreads();
+    uint32_t before = 0u;
+    for (uint32_t r = 0; r < q; r++) before += R.part[r][d];
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        R.whist[8u * q + w][d] = (uint16_t)before;
+        before += c[w];
+    }
+    return before;
+}
+
 template <int ITEMS>
 struct ClusterSort {
     uint2 stage[CS_THREADS * ITEMS]; /* the tile's pairs by digit */
     uint2 pair[CS_THREADS * ITEMS];  /* the cluster's, from any CTA */
-    uint16_t whist[CS_THREADS / 32][RS_RADIX];
-    uint32_t part[4][RS_RADIX];
+    TileRank tile;
     uint32_t tot[2][RS_RADIX]; /* of alternate passes: the cluster may still read the one before */
     uint32_t goff[RS_RADIX], loff[RS_RADIX]; /* a digit's first place in the cluster and in the stage */
     uint32_t wsum[2 * RS_RADIX / 32];
@@ -407,7 +455,7 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_sort_cluster(const uint32_t *
     cg::cluster_group cl = cg::this_cluster();
     constexpr uint32_t TILE = CS_THREADS * ITEMS;
     const uint32_t me = cl.block_rank(), ctas = cl.num_blocks(), all = ctas * TILE;
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, lt = (1u << lane) - 1u;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
     const uint32_t mine = wid * 32u * ITEMS + lane; /* item k: mine + 32 k of the tile */
     uint32_t key[ITEMS], val[ITEMS], rank[ITEMS];
 #pragma unroll
@@ -420,36 +468,9 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_sort_cluster(const uint32_t *
     uint32_t turn = 0u;
     for (uint32_t shift = 0u; shift < bits; shift += 8u, turn ^= 1u) {
         const uint32_t db = min(8u, bits - shift), mask = (1u << db) - 1u;
-        for (uint32_t w = tid; w < sizeof(S.whist) / 4u; w += CS_THREADS) ((uint32_t *)S.whist)[w] = 0u;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < ITEMS; k++) {
-            const uint32_t d = key[k] >> shift & mask, peers = rs_peers(d, db);
-            const uint32_t b = S.whist[wid][d];
-            __syncwarp();
-            if ((peers & lt) == 0u) S.whist[wid][d] = (uint16_t)(b + __popc(peers));
-            rank[k] = b + __popc(peers & lt);
-            __syncwarp();
-        }
-        __syncthreads();
-        /* per digit: exclusive over the warps, eight of them a thread */
-        const uint32_t d = tid & 255u, q = tid >> 8;
-        uint32_t run = 0u, c[8];
-#pragma unroll
-        for (int w = 0; w < 8; w++) {
-            c[w] = S.whist[8u * q + w][d];
-            run += c[w];
-        }
-        S.part[q][d] = run;
-        __syncthreads();
-        uint32_t before = 0u;
-        for (uint32_t r = 0; r < q; r++) before += S.part[r][d];
-#pragma unroll
-        for (int w = 0; w < 8; w++) {
-            S.whist[8u * q + w][d] = (uint16_t)before;
-            before += c[w];
-        }
-        if (q == 3u) S.tot[turn][d] = before;
+        const uint32_t count = rs_tile_rank<ITEMS>(S.tile, key, rank, shift, db, false);
+        const uint32_t d = tid & 255u;
+        if (tid >= CS_THREADS - RS_RADIX) S.tot[turn][d] = count;
         cl.sync();
         /* each digit's first place: of all its pairs and of the tile's among
          * them (threads 0 to 255), and in the staged tile (the next 256) */
@@ -484,7 +505,7 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_sort_cluster(const uint32_t *
 #pragma unroll
         for (int k = 0; k < ITEMS; k++) {
             const uint32_t dk = key[k] >> shift & mask;
-            S.stage[S.loff[dk] + S.whist[wid][dk] + rank[k]] = make_uint2(key[k], val[k]);
+            S.stage[S.loff[dk] + S.tile.whist[wid][dk] + rank[k]] = make_uint2(key[k], val[k]);
         }
         __syncthreads();
 #pragma unroll
@@ -544,9 +565,11 @@ static cudaError_t cluster_sort(const uint32_t *kin, const uint32_t *vin, uint32
  * stay at that latency. */
 #define CS_MAX (CS_CTAS * CS_THREADS * 8u)
 
+bool radix_one_launch(uint32_t n) { return n <= CS_MAX; }
+
 uint32_t radix_launches(uint32_t n, uint32_t bits, uint32_t digit_bits)
 {
-    return n <= CS_MAX ? 1u : 3u * (uint32_t)radix_passes(bits, digit_bits);
+    return radix_one_launch(n) ? 1u : 3u * (uint32_t)radix_passes(bits, digit_bits);
 }
 
 cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
@@ -561,7 +584,7 @@ cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_
             k_iota_copy<<<grid_for((n + 255) / 256, 8), 256, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n);
         return cudaSuccess;
     }
-    if (n <= CS_MAX) {
+    if (radix_one_launch(n)) {
         /* as many CTAs as give each thread one pair, up to eight CTAs */
         const uint32_t per = CS_CTAS * CS_THREADS;
         if (n <= per) return cluster_sort<1>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
@@ -1152,57 +1175,92 @@ void launch_morton_keys(const Launch &L, const float4 *pos, uint32_t *keys, uint
 /* ------------------------------------------ rigid-sphere grid per scene
  * The sort + start/end of FindCellOffsetOrderingPosK (K_HashGrid.cu:140-197)
  * for the rigid-sphere grid, in one CTA per scene when every scene has at
- * most FG_RB_SCENE_MAX spheres.  The scene's (key, index) pairs are sorted
- * as 64-bit words by a bitonic network in shared memory -- the index in the
- * low word makes the order the stable one, so keys, ids and ranges equal the
- * radix path's bit for bit.  A scene's spheres and rigid buckets are its own
- * ranges of the global arrays, and the global stable order is the scenes'
- * orders one after another (keys carry the scene's rigid bucket base). */
-__global__ void __launch_bounds__(1024) k_rb_sort_ranges(const FgScene *__restrict__ table,
-                                                        const __grid_constant__ FgScene single,
-                                                        const uint32_t *__restrict__ keys_u,
-                                                        const float4 *__restrict__ world,
-                                                        uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
-                                                        float4 *__restrict__ spos, uint32_t *__restrict__ rstart,
-                                                        uint32_t *__restrict__ rend)
+ * most FG_RB_SCENE_MAX spheres: a stable radix sort of the scene's (key,
+ * index) pairs in shared memory, four a thread, 8 bits a pass, so keys, ids
+ * and ranges equal the general path's bit for bit.  A scene's spheres and rigid
+ * buckets are its own ranges of the global arrays, and the global stable order
+ * is the scenes' orders one after another (keys carry the scene's rigid bucket
+ * base, which the sort leaves out: two or three passes).  Bound by the
+ * latency of one CTA's barriers; a bitonic network of 64-bit words in its
+ * place took 78 rounds of them for 4,096 spheres, 55 us, longer than the fluid
+ * sort it runs beside (1M particles with one such body: 541 -> 519 us a step). */
+#define RB_ITEMS 4
+static_assert(FG_RB_SCENE_MAX <= CS_THREADS * RB_ITEMS, "a scene's spheres are one CTA's tile");
+
+__global__ void __launch_bounds__(CS_THREADS) k_rb_sort_ranges(const FgScene *__restrict__ table,
+                                                              const __grid_constant__ FgScene single,
+                                                              const uint32_t *__restrict__ keys_u,
+                                                              const float4 *__restrict__ world,
+                                                              uint32_t *__restrict__ keys, uint32_t *__restrict__ ids,
+                                                              float4 *__restrict__ spos, uint32_t *__restrict__ rstart,
+                                                              uint32_t *__restrict__ rend)
 {
-    __shared__ unsigned long long s[FG_RB_SCENE_MAX];
+    __shared__ TileRank R;
+    __shared__ uint32_t s_key[CS_THREADS * RB_ITEMS];
+    __shared__ uint16_t s_val[CS_THREADS * RB_ITEMS];
+    __shared__ uint32_t s_off[RS_RADIX], s_wsum[RS_RADIX / 32];
     const FgScene *S = table ? table + blockIdx.x : &single;
-    const uint32_t n = S->nsph, base = S->sph_base;
+    const uint32_t n = S->nsph, base = S->sph_base, bucket0 = S->rb_bucket_base, nb = S->rb_nb;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5;
     if (!(S->flags & FG_SCENE_HAS_RB)) return; /* the scene has no rigid buckets */
-    for (uint32_t b = threadIdx.x; b < S->rb_nb; b += blockDim.x) rstart[S->rb_bucket_base + b] = FG_EMPTY;
+    const uint32_t mine = wid * 32u * RB_ITEMS + lane;
+    uint32_t key[RB_ITEMS], val[RB_ITEMS], rank[RB_ITEMS];
+#pragma unroll
+    for (int k = 0; k < RB_ITEMS; k++) {
+        val[k] = mine + 32u * k;
+        key[k] = val[k] < n ? __ldg(keys_u + base + val[k]) - bucket0 : 0xffffffffu; /* the largest, and last */
+    }
+    for (uint32_t b = tid; b < nb; b += CS_THREADS) rstart[bucket0 + b] = FG_EMPTY;
     if (!n) return;
-    uint32_t P = 1;
-    while (P < n) P <<= 1;
-    for (uint32_t i = threadIdx.x; i < P; i += blockDim.x)
-        s[i] = i < n ? (((unsigned long long)__ldg(keys_u + base + i) << 32) | i) : ~0ull;
-    __syncthreads();
-    for (uint32_t k = 2; k <= P; k <<= 1)
-        for (uint32_t j = k >> 1; j; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
-                const uint32_t l = i ^ j;
-                if (l > i) {
-                    const unsigned long long a = s[i], c = s[l];
-                    if ((a > c) == ((i & k) == 0)) {
-                        s[i] = c;
-                        s[l] = a;
-                    }
-                }
+    const bool idle = wid * 32u * RB_ITEMS >= n;
+    const uint32_t bits = nb > 1u ? 32u - (uint32_t)__clz((int)(nb - 1u)) : 1u;
+    for (uint32_t shift = 0u; shift < bits; shift += 8u) {
+        const uint32_t db = min(8u, bits - shift), mask = (1u << db) - 1u;
+        const uint32_t count = rs_tile_rank<RB_ITEMS>(R, key, rank, shift, db, idle);
+        uint32_t incl = count;
+        if (tid >= CS_THREADS - RS_RADIX) {
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
             }
-            __syncthreads();
+            if (lane == 31u) s_wsum[wid & 7u] = incl;
         }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned long long v = s[i];
-        const uint32_t key = (uint32_t)(v >> 32), id = base + (uint32_t)(v & 0xffffffffu);
-        keys[base + i] = key;
+        __syncthreads();
+        if (tid >= CS_THREADS - RS_RADIX) {
+            uint32_t first = incl - count;
+            for (uint32_t w = 0; w < (wid & 7u); w++) first += s_wsum[w];
+            s_off[tid & 255u] = first;
+        }
+        __syncthreads();
+        if (!idle) {
+#pragma unroll
+            for (int k = 0; k < RB_ITEMS; k++) {
+                const uint32_t d = key[k] >> shift & mask, to = s_off[d] + R.whist[wid][d] + rank[k];
+                s_key[to] = key[k];
+                s_val[to] = (uint16_t)val[k];
+            }
+        }
+        __syncthreads();
+        if (!idle) {
+#pragma unroll
+            for (int k = 0; k < RB_ITEMS; k++) {
+                key[k] = s_key[mine + 32u * k];
+                val[k] = s_val[mine + 32u * k];
+            }
+        }
+    }
+    for (uint32_t i = tid; i < n; i += CS_THREADS) {
+        const uint32_t k = bucket0 + s_key[i], id = base + s_val[i];
+        keys[base + i] = k;
         ids[base + i] = id;
         spos[base + i] = __ldg(world + id);
-        const uint32_t prev = i ? (uint32_t)(s[i - 1] >> 32) : key;
-        if (i == 0 || key != prev) {
-            rstart[key] = base + i;
+        const uint32_t prev = i ? bucket0 + s_key[i - 1] : k;
+        if (i == 0 || k != prev) {
+            rstart[k] = base + i;
             if (i) rend[prev] = base + i;
         }
-        if (i == n - 1) rend[key] = base + n;
+        if (i == n - 1) rend[k] = base + n;
     }
 }
 
@@ -1211,7 +1269,7 @@ void launch_rb_sort_ranges(const FgScene *table, const FgScene *single, uint32_t
                            uint32_t *rend, cudaStream_t s)
 {
     if (!nscenes) return;
-    k_rb_sort_ranges<<<nscenes, 1024, 0, s>>>(table, *single, keys_u, world, keys, ids, spos, rstart, rend);
+    k_rb_sort_ranges<<<nscenes, CS_THREADS, 0, s>>>(table, *single, keys_u, world, keys, ids, spos, rstart, rend);
 }
 
 __global__ void k_fill(uint32_t *buf, size_t words, uint32_t v)

@@ -47,6 +47,8 @@ size_t radix_hist_words(uint32_t n);
 int radix_passes(uint32_t bits, uint32_t digit_bits);
 /* kernel launches of a radix_sort */
 uint32_t radix_launches(uint32_t n, uint32_t bits, uint32_t digit_bits);
+/* whether a radix_sort of n pairs is one launch, which leaves the scratch alone */
+bool radix_one_launch(uint32_t n);
 /* One-kernel-per-pass variant (decoupled look-back) for the world's fluid
  * sort: same result as radix_sort with vals_in = 0..n-1.  os is
  * onesweep_words(n) words of scratch; err receives FG_DEV_SORT_TIMEOUT if a
