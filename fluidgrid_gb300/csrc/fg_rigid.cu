@@ -200,32 +200,55 @@ void launch_rb_from_rb(const Launch &L, const float4 *rb_spos, const uint32_t *r
 
 /* ---------------------------------------------------------- FP64 bodies */
 
-__device__ __forceinline__ FgD4 fg_d4(double x, double y, double z, double w)
-{
-    FgD4 r;
-    r.x = x; r.y = y; r.z = z; r.w = w;
-    return r;
-}
-
-struct d4 {
-    double x, y, z, w;
-};
-__device__ __forceinline__ d4 qprod_d(d4 a, d4 b)
-{
-    d4 r;
-    double dotv = a.x * b.x + a.y * b.y + a.z * b.z;
-    r.w = a.w * b.w - dotv;
-    r.x = (a.w * b.x) + (b.w * a.x) + (a.y * b.z - a.z * b.y);
-    r.y = (a.w * b.y) + (b.w * a.y) + (a.z * b.x - a.x * b.z);
-    r.z = (a.w * b.z) + (b.w * a.z) + (a.x * b.y - a.y * b.x);
-    return r;
-}
-
 #define BODY_THREADS 256
 
+/* Sums of the eight components over the warp: lane l gets component l >> 2.
+ * Halves the components a lane carries at each exchange: the sums of a
+ * butterfly over all eight, bit for bit, for nine FP64 additions instead of
+ * forty (the FP64 pipe takes a warp's addition in many cycles): 10 -> 4.3 us
+ * for 32 bodies of 512 spheres. */
+__device__ __forceinline__ double body_sum8(double (&a)[8])
+{
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int o = 16, n = 4; o >= 4; o >>= 1, n >>= 1) {
+        const bool upper = lane & (uint32_t)o;
+#pragma unroll
+        for (int q = 0; q < n; q++) {
+            const double keep = upper ? a[n + q] : a[q], give = upper ? a[q] : a[n + q];
+            a[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 2);
+    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+    return a[0];
+}
+
+/* One CTA's sums of force and torque (component threadIdx.x of eight, in the
+ * first eight threads) over spheres first + [lo, hi): threads stride them, then
+ * a warp tree and the warps in order (deterministic). */
+__device__ __forceinline__ double body_sum_cta(uint32_t first, uint32_t lo, uint32_t hi,
+                                               const float4 *__restrict__ force, const float4 *__restrict__ torque,
+                                               double (*s_red)[8])
+{
+    double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (uint32_t k = lo + threadIdx.x; k < hi; k += BODY_THREADS) {
+        const float4 f = __ldg(force + first + k), t = __ldg(torque + first + k);
+        a[0] += f.x; a[1] += f.y; a[2] += f.z; a[3] += f.w;
+        a[4] += t.x; a[5] += t.y; a[6] += t.z; a[7] += t.w;
+    }
+    const double sum = body_sum8(a);
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+    if ((lane & 3u) == 0u) s_red[wid][lane >> 2] = sum;
+    __syncthreads();
+    double v = 0.0;
+    if (threadIdx.x < 8)
+        for (int wv = 0; wv < BODY_THREADS / 32; wv++) v += s_red[wv][threadIdx.x];
+    return v;
+}
+
 /* FP64 partial force/torque sums of one body's spheres: chunk blockIdx.x of
- * FG_BODY_CHUNKS, body blockIdx.y; threads stride the chunk, then a warp
- * shuffle tree and the warps in order (deterministic). */
+ * FG_BODY_CHUNKS, body blockIdx.y. */
 __global__ void __launch_bounds__(BODY_THREADS) k_body_partial(const uint32_t *__restrict__ body_first,
                                                               const uint32_t *__restrict__ body_count,
                                                               const float4 *__restrict__ force,
@@ -234,31 +257,101 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_partial(const uint32_t *_
 {
     __shared__ double s_red[BODY_THREADS / 32][8];
     const uint32_t b = blockIdx.y, c = blockIdx.x;
-    const uint32_t first = body_first[b], cnt = body_count[b];
+    const uint32_t cnt = body_count[b];
     const uint32_t per = (cnt + FG_BODY_CHUNKS - 1) / FG_BODY_CHUNKS;
-    const uint32_t lo = min(cnt, c * per), hi = min(cnt, lo + per);
-    double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t k = lo + threadIdx.x; k < hi; k += BODY_THREADS) {
-        const float4 f = __ldg(force + first + k), t = __ldg(torque + first + k);
-        a[0] += f.x; a[1] += f.y; a[2] += f.z; a[3] += f.w;
-        a[4] += t.x; a[5] += t.y; a[6] += t.z; a[7] += t.w;
-    }
-#pragma unroll
-    for (int q = 0; q < 8; q++)
-#pragma unroll
-        for (int o = 16; o; o >>= 1) a[q] += __shfl_xor_sync(0xffffffffu, a[q], o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < 8; q++) s_red[wid][q] = a[q];
-    __syncthreads();
-    if (threadIdx.x < 8) {
-        double v = 0.0;
-        for (int wv = 0; wv < BODY_THREADS / 32; wv++) v += s_red[wv][threadIdx.x];
-        partial[((size_t)b * FG_BODY_CHUNKS + c) * 8 + threadIdx.x] = v;
-    }
+    const double v = body_sum_cta(body_first[b], min(cnt, c * per), min(cnt, (c + 1) * per), force, torque, s_red);
+    if (threadIdx.x < 8) partial[((size_t)b * FG_BODY_CHUNKS + c) * 8 + threadIdx.x] = v;
 }
 
+/* What the lanes of a body's warp read of one another, by component x, y, z, w
+ * or matrix element (row-major). */
+struct BodyWarp {
+    double F[4], L[4], q[4], om[4], R[9], Tm[9], G[9];
+};
+
+/* Component c of the quaternion product a * b, c = 3 the scalar part. */
+__device__ __forceinline__ double body_qprod(const double *a, const double *b, uint32_t c)
+{
+    if (c == 3u) {
+        const double dotv = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+        return a[3] * b[3] - dotv;
+    }
+    const uint32_t d = c == 2u ? 0u : c + 1u, e = c == 0u ? 2u : c - 1u;
+    return (a[3] * b[c]) + (b[3] * a[c]) + (a[d] * b[e] - a[e] * b[d]);
+}
+
+/* IntegrateRBK in double for one body by one warp: lane c < 4 has component c
+ * of the sums F and T and of the vectors, lane e < 9 element e of the
+ * matrices.  A body is a chain of some 60 FP64 operations, two square roots
+ * and two divides that way, 11 us; one thread went through some 500, 22 us. */
+__device__ __forceinline__ void body_integrate(const FgScene *S, uint32_t b, double F, double T, const BodyState &st,
+                                               BodyWarp &W)
+{
+    const uint32_t lane = threadIdx.x & 31u, c = lane & 3u, e = min(lane, 8u), r = e / 3u, k = e % 3u;
+    const double vl = S->rb_vlimit, dt = S->rb_dt;
+    if (lane < 4u) {
+        W.F[c] = F;
+        W.q[c] = ((const double *)(st.q + b))[c];
+    }
+    __syncwarp();
+    const double spd = sqrt(W.F[0] * W.F[0] + W.F[1] * W.F[1] + W.F[2] * W.F[2] + W.F[3] * W.F[3]);
+    if (spd > vl) F *= vl / spd;
+    const double acc = ((F + (double)S->rb_gravity[c]) / st.mass[b]) * dt;
+    double v = ((const double *)(st.v + b))[c], x = ((const double *)(st.x + b))[c];
+    v += acc * dt;
+    if (c < 3u) x += v * dt;
+    double L = ((const double *)(st.L + b))[c];
+    L = (L + T * dt) * (double)0.9f;
+    /* AngularVelocityD: R * Iinv * R^T * L.  R's diagonal: (1 - 2 a a) - 2 b b
+     * of the other two components; else (2 q_r q_k) +- 2 w q_o of the third */
+    {
+        const bool diag = r == k, plus = !diag && (k == r + 1u || (r == 2u && k == 0u));
+        const double a1 = W.q[diag ? (r == 0u ? 1u : 0u) : r], a2 = W.q[diag ? (r == 0u ? 1u : 0u) : k];
+        const double b1 = diag ? W.q[r == 2u ? 1u : 2u] : W.q[3], b2 = W.q[diag ? (r == 2u ? 1u : 2u) : 3u - r - k];
+        const double u = diag ? 1.0 - 2.0 * a1 * a2 : 2.0 * a1 * a2;
+        if (lane < 9u) W.R[e] = plus ? u + 2.0 * b1 * b2 : u - 2.0 * b1 * b2;
+        if (lane < 4u) W.L[c] = L;
+    }
+    __syncwarp();
+    const double *I = st.inv_inertia + 9 * b;
+    if (lane < 9u) W.Tm[e] = W.R[3u * r] * I[k] + W.R[3u * r + 1u] * I[3u + k] + W.R[3u * r + 2u] * I[6u + k];
+    __syncwarp();
+    if (lane < 9u)
+        W.G[e] = W.Tm[3u * r] * W.R[3u * k] + W.Tm[3u * r + 1u] * W.R[3u * k + 1u] + W.Tm[3u * r + 2u] * W.R[3u * k + 2u];
+    __syncwarp();
+    if (lane < 4u)
+        W.om[c] = c < 3u ? W.G[3u * c] * W.L[0] + W.G[3u * c + 1u] * W.L[1] + W.G[3u * c + 2u] * W.L[2] : 0.0;
+    __syncwarp();
+    const double om = body_qprod(W.om, W.q, c) * (double)0.5f;
+    __syncwarp();
+    if (lane < 4u) W.om[c] = om * dt * (double)0.1f;
+    __syncwarp();
+    double q = W.q[c] + body_qprod(W.om, W.q, c);
+    __syncwarp();
+    if (lane < 4u) W.q[c] = q;
+    __syncwarp();
+    q /= sqrt(W.q[3] * W.q[3] + W.q[0] * W.q[0] + W.q[1] * W.q[1] + W.q[2] * W.q[2]);
+    const double rest = (double)-0.7f;
+    if (c == 1u) {
+        if (x < (double)S->rb_vmin[1]) { x = S->rb_vmin[1]; v *= rest; }
+    } else if (c != 3u) {
+        if (x <= (double)S->rb_vmin[c]) { x = S->rb_vmin[c]; v *= rest; }
+        else if (x >= (double)S->rb_vmax[c]) { x = S->rb_vmax[c]; v *= rest; }
+    }
+    if (lane < 4u) {
+        ((double *)(st.x + b))[c] = x;
+        ((double *)(st.v + b))[c] = v;
+        ((double *)(st.L + b))[c] = L;
+        ((double *)(st.q + b))[c] = q;
+        ((float *)(st.x_f + b))[c] = (float)x;
+        ((float *)(st.v_f + b))[c] = (float)v;
+        ((float *)(st.q_f + b))[c] = (float)q;
+    }
+    __syncwarp();
+}
+
+/* A CTA per body: its sum, or its partial sums in order, then the first warp
+ * integrates it. */
 __global__ void __launch_bounds__(BODY_THREADS) k_body_update(const FgScene *__restrict__ table,
                                                              const __grid_constant__ FgScene single,
                                                              const uint32_t *__restrict__ body_scene,
@@ -269,109 +362,26 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_update(const FgScene *__r
                                                              int integrate)
 {
     __shared__ double s_red[BODY_THREADS / 32][8];
+    __shared__ BodyWarp W;
     for (uint32_t b = blockIdx.x; b < nbodies; b += gridDim.x) {
-        const uint32_t first = body_first[b], cnt = st.partial ? 0u : body_count[b];
-        double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (uint32_t k = threadIdx.x; k < cnt; k += BODY_THREADS) {
-            float4 f = __ldg(force + first + k), t = __ldg(torque + first + k);
-            a[0] += f.x; a[1] += f.y; a[2] += f.z; a[3] += f.w;
-            a[4] += t.x; a[5] += t.y; a[6] += t.z; a[7] += t.w;
-        }
+        double v = 0.0;
+        if (st.partial) {
+            if (threadIdx.x < 8) {
+                const double *pp = st.partial + (size_t)b * FG_BODY_CHUNKS * 8 + threadIdx.x;
 #pragma unroll
-        for (int c = 0; c < 8; c++)
-#pragma unroll
-            for (int o = 16; o; o >>= 1) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
-        const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-        if (lane == 0)
-#pragma unroll
-            for (int c = 0; c < 8; c++) s_red[wid][c] = a[c];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double F[4] = {0, 0, 0, 0}, T[4] = {0, 0, 0, 0};
-            if (st.partial) {
-                const double *pp = st.partial + (size_t)b * FG_BODY_CHUNKS * 8;
-                for (int ch = 0; ch < FG_BODY_CHUNKS; ch++)
-                    for (int c = 0; c < 4; c++) {
-                        F[c] += pp[ch * 8 + c];
-                        T[c] += pp[ch * 8 + 4 + c];
-                    }
-            } else {
-                for (int wv = 0; wv < BODY_THREADS / 32; wv++)
-                    for (int c = 0; c < 4; c++) {
-                        F[c] += s_red[wv][c];
-                        T[c] += s_red[wv][4 + c];
-                    }
+                for (int ch = 0; ch < FG_BODY_CHUNKS; ch++) v += pp[ch * 8];
             }
-            st.force_sum[b] = fg_d4(F[0], F[1], F[2], F[3]);
-            st.torque_sum[b] = fg_d4(T[0], T[1], T[2], T[3]);
+        } else {
+            v = body_sum_cta(body_first[b], 0u, body_count[b], force, torque, s_red);
+        }
+        if (threadIdx.x < 32) {
+            if (threadIdx.x < 8) ((double *)((threadIdx.x < 4 ? st.force_sum : st.torque_sum) + b))[threadIdx.x & 3] = v;
+            const double T = __shfl_sync(0xffffffffu, v, (threadIdx.x & 3) + 4);
+            const double F = __shfl_sync(0xffffffffu, v, threadIdx.x & 3);
             /* mass 0: a static body (the reference's "static" rigid-body
              * file type), never integrated */
-            if (integrate && st.mass[b] != 0.0) {
-                const FgScene *S = table ? table + body_scene[b] : &single;
-                /* IntegrateRBK in double */
-                const double vl = S->rb_vlimit;
-                double spd = sqrt(F[0] * F[0] + F[1] * F[1] + F[2] * F[2] + F[3] * F[3]);
-                if (spd > vl) {
-                    double t = vl / spd;
-                    for (int c = 0; c < 4; c++) F[c] *= t;
-                }
-                const double dt = S->rb_dt, m = st.mass[b];
-                FgD4 x = st.x[b], v = st.v[b], L = st.L[b], q4 = st.q[b];
-                double acc[4];
-                for (int c = 0; c < 4; c++) acc[c] = ((F[c] + (double)S->rb_gravity[c]) / m) * dt;
-                v.x += acc[0] * dt; v.y += acc[1] * dt; v.z += acc[2] * dt; v.w += acc[3] * dt;
-                x.x += v.x * dt; x.y += v.y * dt; x.z += v.z * dt;
-                const double damp = (double)0.9f;
-                L.x = (L.x + T[0] * dt) * damp;
-                L.y = (L.y + T[1] * dt) * damp;
-                L.z = (L.z + T[2] * dt) * damp;
-                L.w = (L.w + T[3] * dt) * damp;
-                /* AngularVelocityD: R * Iinv * R^T * L */
-                const double *I = st.inv_inertia + 9 * b;
-                d4 q = {q4.x, q4.y, q4.z, q4.w};
-                double R[3][3];
-                R[0][0] = 1.0 - (2.0 * q.y * q.y) - (2.0 * q.z * q.z);
-                R[0][1] = (2.0 * q.x * q.y) + (2.0 * q.w * q.z);
-                R[0][2] = (2.0 * q.x * q.z) - (2.0 * q.w * q.y);
-                R[1][0] = (2.0 * q.x * q.y) - (2.0 * q.w * q.z);
-                R[1][1] = 1.0 - (2.0 * q.x * q.x) - (2.0 * q.z * q.z);
-                R[1][2] = (2.0 * q.y * q.z) + (2.0 * q.w * q.x);
-                R[2][0] = (2.0 * q.x * q.z) + (2.0 * q.w * q.y);
-                R[2][1] = (2.0 * q.y * q.z) - (2.0 * q.w * q.x);
-                R[2][2] = 1.0 - (2.0 * q.x * q.x) - (2.0 * q.y * q.y);
-                double Tm[3][3], G[3][3];
-                for (int r = 0; r < 3; r++)
-                    for (int c = 0; c < 3; c++)
-                        Tm[r][c] = R[r][0] * I[0 * 3 + c] + R[r][1] * I[1 * 3 + c] + R[r][2] * I[2 * 3 + c];
-                for (int r = 0; r < 3; r++)
-                    for (int c = 0; c < 3; c++) G[r][c] = Tm[r][0] * R[c][0] + Tm[r][1] * R[c][1] + Tm[r][2] * R[c][2];
-                d4 om;
-                om.x = G[0][0] * L.x + G[0][1] * L.y + G[0][2] * L.z;
-                om.y = G[1][0] * L.x + G[1][1] * L.y + G[1][2] * L.z;
-                om.z = G[2][0] * L.x + G[2][1] * L.y + G[2][2] * L.z;
-                om.w = 0.0;
-                om = qprod_d(om, q);
-                const double half = (double)0.5f, tenth = (double)0.1f;
-                om.x *= half; om.y *= half; om.z *= half; om.w *= half;
-                d4 ws = {om.x * dt * tenth, om.y * dt * tenth, om.z * dt * tenth, om.w * dt * tenth};
-                d4 dq = qprod_d(ws, q);
-                q.x += dq.x; q.y += dq.y; q.z += dq.z; q.w += dq.w;
-                double nrm = sqrt(q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z);
-                q.x /= nrm; q.y /= nrm; q.z /= nrm; q.w /= nrm;
-                const double rest = (double)-0.7f;
-                if (x.y < (double)S->rb_vmin[1]) { x.y = S->rb_vmin[1]; v.y *= rest; }
-                if (x.x <= (double)S->rb_vmin[0]) { x.x = S->rb_vmin[0]; v.x *= rest; }
-                else if (x.x >= (double)S->rb_vmax[0]) { x.x = S->rb_vmax[0]; v.x *= rest; }
-                if (x.z <= (double)S->rb_vmin[2]) { x.z = S->rb_vmin[2]; v.z *= rest; }
-                else if (x.z >= (double)S->rb_vmax[2]) { x.z = S->rb_vmax[2]; v.z *= rest; }
-                st.x[b] = x;
-                st.v[b] = v;
-                st.L[b] = L;
-                st.q[b] = fg_d4(q.x, q.y, q.z, q.w);
-                st.x_f[b] = make_float4((float)x.x, (float)x.y, (float)x.z, (float)x.w);
-                st.v_f[b] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
-                st.q_f[b] = make_float4((float)q.x, (float)q.y, (float)q.z, (float)q.w);
-            }
+            if (integrate && st.mass[b] != 0.0)
+                body_integrate(table ? table + body_scene[b] : &single, b, F, T, st, W);
         }
         __syncthreads();
     }
@@ -387,7 +397,7 @@ void launch_body_update(const FgScene *table, const FgScene *single, const uint3
                                                                             st.partial);
     else
         st.partial = nullptr;
-    k_body_update<<<grid_for(nbodies, 4), BODY_THREADS, 0, s>>>(table, *single, body_scene, body_first, body_count,
+    k_body_update<<<grid_for(nbodies, st.partial ? 16 : 4), st.partial ? 32 : BODY_THREADS, 0, s>>>(table, *single, body_scene, body_first, body_count,
                                                                 nbodies, force, torque, st, integrate);
 }
 
