@@ -36,6 +36,26 @@ uint32_t grid_for(uint32_t nwork, int ctas_per_sm)
 
 /* ------------------------------------------------------------- hashing */
 
+/* cnt[key] += 1 for every valid lane of the (converged) warp; the count that
+ * the lane finds there, its own place in the bucket: one L2 atomic per run of
+ * equal keys in neighbouring lanes (a match_any finds the same runs in as many
+ * rounds as there are keys; 1M particles of a lattice: 15 -> 10.5 us). */
+__device__ __forceinline__ uint32_t bs_count_in(uint32_t key, bool valid, uint32_t *__restrict__ cnt)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const uint32_t act = __ballot_sync(0xffffffffu, valid); /* a prefix of the lanes */
+    const uint32_t heads = __ballot_sync(0xffffffffu, valid && (lane == 0u || key != prev));
+    const uint32_t upto = heads & (0xffffffffu >> (31u - lane)), later = heads & ~(0xffffffffu >> (31u - lane));
+    const uint32_t head = upto ? 31u - (uint32_t)__clz((int)upto) : lane;
+    uint32_t o = 0u;
+    if (valid && head == lane) {
+        const uint32_t next = later ? (uint32_t)__ffs((int)later) - 1u : (uint32_t)__popc(act);
+        o = atomicAdd(cnt + key, next - lane);
+    }
+    return __shfl_sync(0xffffffffu, o, (int)head) + lane - head;
+}
+
 /* CalcHashKeyK (K_HashGrid.cu:26-38): key = bucket_base + HashKeyD(pos),
  * id = particle index.  With cnt, also the counting sort's first pass (as
  * k_bs_count): cnt[key] += 1 by L2 atomics, one per run of equal keys in a
@@ -47,7 +67,6 @@ __global__ void __launch_bounds__(FG_CHUNK) k_hash(const FgWork *__restrict__ wo
                                                   uint32_t *__restrict__ ids, uint32_t *__restrict__ cnt,
                                                   uint32_t *__restrict__ off)
 {
-    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t w = blockIdx.x; w < nwork; w += gridDim.x) {
         FgWork it = fg_work(work, w, n_single);
         const FgScene *S = fg_scene(table, &single, it.scene);
@@ -61,14 +80,8 @@ __global__ void __launch_bounds__(FG_CHUNK) k_hash(const FgWork *__restrict__ wo
             if (ids) ids[i] = i;
         }
         if (cnt) { /* uniform: every lane of the warp gets here */
-            const uint32_t act = __ballot_sync(0xffffffffu, valid);
-            if (valid) {
-                const uint32_t peers = __match_any_sync(act, k);
-                const uint32_t leader = (uint32_t)(__ffs(peers) - 1);
-                uint32_t o = 0;
-                if (lane == leader) o = atomicAdd(cnt + k, (uint32_t)__popc(peers));
-                off[i] = __shfl_sync(peers, o, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-            }
+            const uint32_t o = bs_count_in(k, valid, cnt);
+            if (valid) off[i] = o;
         }
     }
 }
@@ -647,6 +660,7 @@ cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_
 #define BS_ITEMS 8
 #define BS_TILE (BS_THREADS * BS_ITEMS)
 static_assert(BS_THREADS == RS_THREADS, "the tile scans use rs_block_excl");
+#define BS_RANKS 2u /* particles that a thread of k_bs_rank_reorder has in flight */
 
 __global__ void __launch_bounds__(256) k_bs_count(const uint32_t *__restrict__ keys, uint32_t n,
                                                  uint32_t *__restrict__ cnt, uint32_t *__restrict__ off)
@@ -657,15 +671,8 @@ __global__ void __launch_bounds__(256) k_bs_count(const uint32_t *__restrict__ k
     for (uint32_t b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b0 < n; b0 += stride) {
         const uint32_t i = b0 + lane;
         const bool valid = i < n;
-        const uint32_t act = __ballot_sync(0xffffffffu, valid);
-        if (valid) {
-            const uint32_t k = __ldg(keys + i);
-            const uint32_t peers = __match_any_sync(act, k);
-            const uint32_t leader = (uint32_t)(__ffs(peers) - 1);
-            uint32_t o = 0;
-            if (lane == leader) o = atomicAdd(cnt + k, (uint32_t)__popc(peers));
-            off[i] = __shfl_sync(peers, o, leader) + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-        }
+        const uint32_t o = bs_count_in(valid ? __ldg(keys + i) : 0u, valid, cnt);
+        if (valid) off[i] = o;
     }
 }
 
@@ -765,7 +772,9 @@ __global__ void __launch_bounds__(256) k_bs_rank(const uint32_t *__restrict__ ke
 /* k_bs_rank and the ranges pass's reorder in one: the particle's sorted
  * index p = start + rank gets its id, position and velocity, inv[id] = p,
  * and a rank-0 particle appends its bucket's first index to runs (in no
- * particular order, as the ranges pass does). */
+ * particular order, as the ranges pass does).  Bound by the gathers' sectors
+ * and by a chain of four loads a particle: two particles a thread at a time
+ * take 123 us where one took 133 (4M; four: 118 there, no better at 1M). */
 __global__ void __launch_bounds__(256) k_bs_rank_reorder(const uint32_t *__restrict__ keys_out,
                                                         const uint32_t *__restrict__ tmp, uint32_t n,
                                                         const uint32_t *__restrict__ start,
@@ -774,29 +783,53 @@ __global__ void __launch_bounds__(256) k_bs_rank_reorder(const uint32_t *__restr
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b0 < n; b0 += stride) {
-        const uint32_t s = b0 + lane;
-        const bool valid = s < n;
-        uint32_t st = 0, r = 0;
-        if (valid) {
-            const uint32_t k = __ldg(keys_out + s);
-            st = __ldg(start + k);
-            const uint32_t en = __ldg(end + k);
-            const uint32_t e = __ldg(tmp + s);
-            for (uint32_t f = st; f < en; f++) r += __ldg(tmp + f) < e ? 1u : 0u;
-            const uint32_t p = st + r;
-            vals_out[p] = e;
-            R.spos[p] = __ldg(R.pos + e);
-            if (R.vel) R.svel[p] = __ldg(R.vel + e);
-            if (R.inv) R.inv[e] = p;
+    for (uint32_t b0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); b0 < n; b0 += BS_RANKS * stride) {
+        uint32_t st[BS_RANKS], en[BS_RANKS], e[BS_RANKS], r[BS_RANKS];
+#pragma unroll
+        for (uint32_t u = 0; u < BS_RANKS; u++) {
+            const uint32_t s = b0 + u * stride + lane;
+            st[u] = s < n ? __ldg(keys_out + s) : 0u;
+            e[u] = s < n ? __ldg(tmp + s) : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < BS_RANKS; u++) {
+            const uint32_t k = st[u];
+            st[u] = en[u] = r[u] = 0u;
+            if (b0 + u * stride + lane < n) {
+                st[u] = __ldg(start + k);
+                en[u] = __ldg(end + k);
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < BS_RANKS; u++)
+            for (uint32_t f = st[u]; f < en[u]; f++) r[u] += __ldg(tmp + f) < e[u] ? 1u : 0u;
+        float4 x[BS_RANKS], v[BS_RANKS];
+#pragma unroll
+        for (uint32_t u = 0; u < BS_RANKS; u++)
+            if (b0 + u * stride + lane < n) {
+                x[u] = __ldg(R.pos + e[u]);
+                if (R.vel) v[u] = __ldg(R.vel + e[u]);
+            }
+#pragma unroll
+        for (uint32_t u = 0; u < BS_RANKS; u++) {
+            if (b0 + u * stride + lane < n) {
+                const uint32_t p = st[u] + r[u];
+                vals_out[p] = e[u];
+                R.spos[p] = x[u];
+                if (R.vel) R.svel[p] = v[u];
+                if (R.inv) R.inv[e[u]] = p;
+            }
         }
         if (R.runs) {
-            const bool head = valid && r == 0u;
-            const uint32_t m = __ballot_sync(0xffffffffu, head);
-            uint32_t base = 0;
-            if (lane == 0 && m) base = atomicAdd(R.nruns, (uint32_t)__popc(m));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if (head) R.runs[base + __popc(m & ((1u << lane) - 1u))] = st;
+#pragma unroll
+            for (uint32_t u = 0; u < BS_RANKS; u++) {
+                const bool head = b0 + u * stride + lane < n && r[u] == 0u;
+                const uint32_t m = __ballot_sync(0xffffffffu, head);
+                uint32_t base = 0;
+                if (lane == 0 && m) base = atomicAdd(R.nruns, (uint32_t)__popc(m));
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (head) R.runs[base + __popc(m & ((1u << lane) - 1u))] = st[u];
+            }
         }
     }
 }
