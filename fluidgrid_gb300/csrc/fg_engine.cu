@@ -783,8 +783,11 @@ uint32_t World::enqueue_step(cudaEvent_t *ev)
         CK0(cudaStreamWaitEvent(stream2, ev_fork, 0));
         enqueue_rb_grid(stream2, nullptr, launches);
     }
-    /* end-to-end step: the velocities upload on a third stream while the
-     * positions upload and the hash and sort run; the reorder waits for them */
+    /* end-to-end step: the positions upload first, then the velocities on a
+     * third stream while the hash and sort run; the reorder waits for them
+     * (one direction of the link carries one copy at a time: with the
+     * velocities first, the hash waited for both, 372 against 352 us a step
+     * at 262,144 particles) */
     const size_t iob = 16 * (size_t)n;
     if (cur_io && iob) {
         CK0(cudaEventRecord(ev_io_fork, stream));
@@ -792,19 +795,17 @@ uint32_t World::enqueue_step(cudaEvent_t *ev)
         /* the previous step's velocities go down while this step's
          * positions come up (the link carries both directions at once) */
         if (cur_io->prev_vel) CK0(cudaMemcpyAsync(cur_io->ov, vel, iob, cudaMemcpyDeviceToHost, stream3));
+        CK0(cudaMemcpyAsync(pos, cur_io->hp, iob, cudaMemcpyHostToDevice, stream));
+        CK0(cudaEventRecord(ev_pos_in, stream));
+        CK0(cudaStreamWaitEvent(stream3, ev_pos_in, 0));
         CK0(cudaMemcpyAsync(vel, cur_io->hv, iob, cudaMemcpyHostToDevice, stream3));
         CK0(cudaEventRecord(ev_vel_in, stream3));
-        CK0(cudaMemcpyAsync(pos, cur_io->hp, iob, cudaMemcpyHostToDevice, stream));
     }
     if (fork) {
         /* the fluid side of the contact follows the sphere grid on the second
          * stream, beside the hash and sort; an end-to-end step's pass waits
          * for the state's upload */
-        if (cur_io && iob && fluid_contact_pass()) {
-            CK0(cudaEventRecord(ev_pos_in, stream));
-            CK0(cudaStreamWaitEvent(stream2, ev_pos_in, 0));
-            CK0(cudaStreamWaitEvent(stream2, ev_vel_in, 0));
-        }
+        if (cur_io && iob && fluid_contact_pass()) CK0(cudaStreamWaitEvent(stream2, ev_vel_in, 0));
         enqueue_fluid_contact(stream2, launches);
     }
     counted_in_hash = false;
