@@ -127,7 +127,7 @@ C_ABI_SYMBOLS = [
     "fg_sort_pairs_noalloc", "fg_selftest_bounded_wait", "fg_world_set_option", "fg_world_get_option", "fg_world_tuning_stats",
     "fg_world_counters", "fg_world_list_overflows", "fg_world_timed_blocks", "fg_world_diagnostics", "fg_server_config_defaults", "fg_server_create",
     "fg_server_destroy", "fg_server_submit", "fg_server_step", "fg_server_request", "fg_server_result",
-    "fg_server_stats", "fg_server_active",
+    "fg_server_stats", "fg_server_active", "fg_server_take", "fg_host_state_free",
     "fg_memcpy_d2h", "fg_memcpy_h2d",
     "fg_device_synchronize", "fg_last_error", "fg_version"]
 REFERENCE_SYMBOLS = [
@@ -206,6 +206,9 @@ def load():
     L.fg_server_step.argtypes = [VP, P(fg_server_step_info)]
     L.fg_server_request.argtypes = [VP, ctypes.c_uint64, P(fg_request_info)]
     L.fg_server_result.argtypes = [VP, ctypes.c_uint64, VP, VP, ctypes.c_int]
+    L.fg_server_take.argtypes = [VP, ctypes.c_uint64, P(VP), P(VP), P(VP)]
+    L.fg_host_state_free.argtypes = [VP]
+    L.fg_host_state_free.restype = None
     L.fg_server_stats.argtypes = [VP, P(fg_server_stats_info)]
     L.fg_server_active.argtypes = [VP, P(ctypes.c_uint64), c_u32, P(c_u32)]
     L.fg_memcpy_d2h.argtypes = [VP, VP, ctypes.c_size_t]

@@ -361,7 +361,7 @@ int World::reserve(const Capacity &c)
 /* Scene table, work tables and the static per-body and per-sphere data of
  * the scenes d[0..ns) (which must fit the capacity).  Dynamic state --
  * particle positions, velocities, densities and the bodies' motion -- is not
- * touched: upload_scene or a migration fills it. */
+ * touched: upload_particles and upload_bodies or a migration fill it. */
 int World::set_layout(const fg_scene_desc *d, uint32_t ns)
 {
     const Capacity need = needs(d, ns);
@@ -462,53 +462,67 @@ int World::set_layout(const fg_scene_desc *d, uint32_t ns)
                 hm[gb] = bd.mass;
                 for (int c = 0; c < 9; c++) hinv[9 * gb + c] = bd.inv_inertia[c];
             }
-        if (S) CK(cudaMemcpy(rb_local, local.data(), 16 * S, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bmass, hm.data(), 8 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(binv, hinv.data(), 72 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(body_scene, hbs.data(), 4 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(body_first, hbf.data(), 4 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(body_count, hbc.data(), 4 * B, cudaMemcpyHostToDevice));
+        auto up = [&](void *dst, const void *src, size_t bytes) {
+            return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream) : cudaSuccess;
+        };
+        cudaError_t e = up(rb_local, local.data(), 16 * S);
+        if (e == cudaSuccess) e = up(bmass, hm.data(), 8 * B);
+        if (e == cudaSuccess) e = up(binv, hinv.data(), 72 * B);
+        if (e == cudaSuccess) e = up(body_scene, hbs.data(), 4 * B);
+        if (e == cudaSuccess) e = up(body_first, hbf.data(), 4 * B);
+        if (e == cudaSuccess) e = up(body_count, hbc.data(), 4 * B);
+        const cudaError_t es = cudaStreamSynchronize(stream); /* the host arrays end here */
+        CK(e);
+        CK(es);
     }
     stale_graphs();
     return FG_OK;
 }
 
-/* Initial dynamic state of scene s from its description: positions,
- * velocities (zero if none) and the bodies at rest at their poses. */
-int World::upload_scene(uint32_t s, const fg_scene_desc &d)
+/* Initial positions and velocities (zero if none) of scene s, ahead on the
+ * stream: the arrays of the description must outlive the copies. */
+int World::upload_particles(uint32_t s, const fg_scene_desc &d)
 {
     const FgScene &S = scenes_h[s];
-    if (S.n) {
-        CK(cudaMemcpyAsync(pos + S.pbase, d.positions, 16 * (size_t)S.n, cudaMemcpyHostToDevice, stream));
-        if (d.velocities)
-            CK(cudaMemcpyAsync(vel + S.pbase, d.velocities, 16 * (size_t)S.n, cudaMemcpyHostToDevice, stream));
-        else
-            CK(cudaMemsetAsync(vel + S.pbase, 0, 16 * (size_t)S.n, stream));
-        CK(cudaMemsetAsync(dp + S.pbase, 0, 8 * (size_t)S.n, stream));
-    }
-    if (S.nbodies) {
-        const size_t B = S.nbodies;
-        std::vector<double> hx(4 * B), hv(4 * B, 0.0), hq(4 * B), hL(4 * B, 0.0);
-        std::vector<float> hxf(4 * B), hvf(4 * B, 0.0f), hqf(4 * B);
-        for (uint32_t b = 0; b < S.nbodies; b++) {
-            const fg_body_desc &bd = d.bodies[b];
-            for (int c = 0; c < 3; c++) hx[4 * b + c] = bd.position[c];
-            hx[4 * b + 3] = 0.0;
-            for (int c = 0; c < 4; c++) hq[4 * b + c] = bd.orientation[c];
-            for (int c = 0; c < 4; c++) {
-                hxf[4 * b + c] = (float)hx[4 * b + c];
-                hqf[4 * b + c] = (float)hq[4 * b + c];
-            }
+    if (!S.n) return FG_OK;
+    CK(cudaMemcpyAsync(pos + S.pbase, d.positions, 16 * (size_t)S.n, cudaMemcpyHostToDevice, stream));
+    if (d.velocities)
+        CK(cudaMemcpyAsync(vel + S.pbase, d.velocities, 16 * (size_t)S.n, cudaMemcpyHostToDevice, stream));
+    else
+        CK(cudaMemsetAsync(vel + S.pbase, 0, 16 * (size_t)S.n, stream));
+    CK(cudaMemsetAsync(dp + S.pbase, 0, 8 * (size_t)S.n, stream));
+    return FG_OK;
+}
+
+/* The bodies of a description at rest at their poses, as bodies o, o + 1, ... */
+void BodyMotion::rest(const fg_scene_desc &d, size_t o)
+{
+    for (uint32_t b = 0; b < d.n_bodies; b++, o++) {
+        const fg_body_desc &bd = d.bodies[b];
+        for (int c = 0; c < 4; c++) {
+            x[4 * o + c] = c < 3 ? bd.position[c] : 0.0;
+            q[4 * o + c] = bd.orientation[c];
+            v[4 * o + c] = L[4 * o + c] = 0.0;
+            xf[4 * o + c] = (float)x[4 * o + c];
+            qf[4 * o + c] = (float)q[4 * o + c];
+            vf[4 * o + c] = 0.0f;
         }
-        const size_t o = S.body_base;
-        CK(cudaMemcpy(bx + o, hx.data(), 32 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bv + o, hv.data(), 32 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bq + o, hq.data(), 32 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bL + o, hL.data(), 32 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bxf + o, hxf.data(), 16 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bvf + o, hvf.data(), 16 * B, cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(bqf + o, hqf.data(), 16 * B, cudaMemcpyHostToDevice));
     }
+}
+
+/* Every body's motion, ahead on the stream (m must outlive the copies): the
+ * arrays hold the scenes' bodies one after another, so a copy an array. */
+int World::upload_bodies(const BodyMotion &m)
+{
+    if (!nbodies) return FG_OK;
+    const size_t B = nbodies;
+    CK(cudaMemcpyAsync(bx, m.x.data(), 32 * B, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(bv, m.v.data(), 32 * B, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(bq, m.q.data(), 32 * B, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(bL, m.L.data(), 32 * B, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(bxf, m.xf.data(), 16 * B, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(bvf, m.vf.data(), 16 * B, cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(bqf, m.qf.data(), 16 * B, cudaMemcpyHostToDevice, stream));
     return FG_OK;
 }
 
@@ -575,9 +589,14 @@ int World::create(const fg_scene_desc *d, uint32_t ns, cudaStream_t st)
     }
     if ((r = reserve(c)) != FG_OK) return r;
     if ((r = set_layout(d, ns)) != FG_OK) return r;
-    for (uint32_t s = 0; s < ns; s++)
-        if ((r = upload_scene(s, d[s])) != FG_OK) return r;
+    BodyMotion m(nbodies);
+    for (uint32_t s = 0; s < ns; s++) {
+        if ((r = upload_particles(s, d[s])) != FG_OK) return r;
+        m.rest(d[s], scenes_h[s].body_base);
+    }
+    r = upload_bodies(m);
     CK(cudaStreamSynchronize(stream));
+    if (r != FG_OK) return r;
     return FG_OK;
 }
 

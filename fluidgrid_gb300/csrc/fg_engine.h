@@ -37,6 +37,29 @@ struct Capacity {
  * (sort variant 2) by default */
 #define FG_BUCKET_SORT_RATIO 64
 
+/* The bodies' motion on the host, in the layout of the device arrays: FP64
+ * position, velocity, orientation, angular momentum; their FP32 mirrors. */
+struct BodyMotion {
+    std::vector<double> x, v, q, L;
+    std::vector<float> xf, vf, qf;
+    explicit BodyMotion(size_t n) : x(4 * n), v(4 * n), q(4 * n), L(4 * n), xf(4 * n), vf(4 * n), qf(4 * n) {}
+    void rest(const fg_scene_desc &d, size_t o);
+    /* n bodies of another layout, from its body i, as bodies o, o + 1, ... */
+    void copy(const BodyMotion &m, size_t i, size_t o, size_t n)
+    {
+        auto part = [&](auto &to, const auto &from) {
+            std::copy(from.begin() + 4 * i, from.begin() + 4 * (i + n), to.begin() + 4 * o);
+        };
+        part(x, m.x);
+        part(v, m.v);
+        part(q, m.q);
+        part(L, m.L);
+        part(xf, m.xf);
+        part(vf, m.vf);
+        part(qf, m.qf);
+    }
+};
+
 struct World {
     /* layout */
     uint32_t nscenes = 0, n = 0, total_buckets = 0, nspheres = 0, nbodies = 0, total_rb_buckets = 0;
@@ -218,7 +241,8 @@ struct World {
     int init_stream(cudaStream_t st);
     int reserve(const Capacity &c);
     int set_layout(const fg_scene_desc *d, uint32_t ns);
-    int upload_scene(uint32_t s, const fg_scene_desc &d);
+    int upload_particles(uint32_t s, const fg_scene_desc &d);
+    int upload_bodies(const BodyMotion &m);
     void drop_graphs();  /* destroys every captured graph */
     void stale_graphs(); /* keeps them for in-place updates */
     /* FP64 conservation diagnostics */

@@ -26,11 +26,14 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string.h>
+#include <stdlib.h>
 #include <algorithm>
 #include <chrono>
 #include <deque>
 #include <map>
 #include <memory>
+#include <mutex>
+#include <new>
 #include <unordered_map>
 #include <vector>
 #include "../../include/fluidgrid_gb300.h"
@@ -47,17 +50,99 @@ namespace fg {
         }                                                                                          \
     } while (0)
 
+/* Host memory of particle states, kept for the next requests: fresh pages cost
+ * more to touch than to copy into (16 MB: 1.0 ms against 0.6).  Shared by a
+ * server and the results handed out, so any thread may give an array back; at
+ * most FG_SERVER_SPARE_BYTES are kept, and they go with the last owner. */
+#define FG_SERVER_SPARE_BYTES ((size_t)256 << 20)
+struct HostPool {
+    std::mutex mu;
+    std::vector<std::pair<size_t, float *>> spare; /* floats, array */
+    size_t bytes = 0;
+
+    ~HostPool()
+    {
+        for (auto &s : spare) free(s.second);
+    }
+    /* an array of at least n floats, not initialised (nullptr: no memory) */
+    float *take(size_t n, size_t &cap)
+    {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            size_t best = spare.size();
+            for (size_t k = 0; k < spare.size(); k++)
+                if (spare[k].first >= n && spare[k].first / 2 <= n &&
+                    (best == spare.size() || spare[k].first < spare[best].first))
+                    best = k;
+            if (best < spare.size()) {
+                float *p = spare[best].second;
+                cap = spare[best].first;
+                bytes -= sizeof(float) * cap;
+                spare[best] = spare.back();
+                spare.pop_back();
+                return p;
+            }
+        }
+        cap = n;
+        return (float *)malloc(sizeof(float) * n);
+    }
+    void give(float *p, size_t cap)
+    {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (bytes + sizeof(float) * cap <= FG_SERVER_SPARE_BYTES && spare.size() < spare.capacity()) {
+                bytes += sizeof(float) * cap;
+                spare.push_back({cap, p});
+                return;
+            }
+        }
+        free(p);
+    }
+    HostPool() { spare.reserve(1024); } /* give() allocates nothing */
+};
+
+struct HostArray {
+    std::shared_ptr<HostPool> pool;
+    float *p = nullptr;
+    size_t cap = 0;
+
+    HostArray() = default;
+    HostArray(const HostArray &) = delete;
+    HostArray &operator=(const HostArray &) = delete;
+    ~HostArray()
+    {
+        if (p) pool->give(p, cap);
+    }
+    bool alloc(const std::shared_ptr<HostPool> &from, size_t n)
+    {
+        if (!n) return true;
+        pool = from;
+        p = pool->take(n, cap);
+        return p != nullptr;
+    }
+    void swap(HostArray &o)
+    {
+        std::swap(pool, o.pool);
+        std::swap(p, o.p);
+        std::swap(cap, o.cap);
+    }
+};
+
+/* a finished request's arrays, handed to the caller */
+struct HostState {
+    HostArray pos, vel;
+};
+
 struct Request {
     uint64_t id = 0;
     fg_scene_desc desc;
-    std::vector<float> pos, vel;             /* initial state (host copies) */
+    HostArray pos, vel;                      /* initial state (host copies), then the final one */
     std::vector<fg_body_desc> bodies;
     std::vector<std::vector<float>> spheres; /* local sphere positions per body */
     uint32_t steps_total = 0, steps_done = 0;
     int state = FG_REQ_QUEUED;
     double t_submit = 0, t_admit = 0, t_done = 0;
     size_t bytes = 0;                        /* budget charge while resident */
-    std::vector<float> out_pos, out_vel;     /* final state */
 };
 
 #define FG_SERVER_RING 16 /* pipeline_depth is clamped below this */
@@ -76,6 +161,8 @@ struct Server {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     std::unique_ptr<World> w;
+    std::shared_ptr<HostPool> pool = std::make_shared<HostPool>();
+    BodyMotion moved{0}; /* the old layout's bodies, in a re-layout */
     std::deque<Request *> queue;
     std::vector<Request *> active;  /* wanted resident set, in layout order */
     std::vector<uint64_t> laid_out; /* request id of world scene s */
@@ -172,19 +259,17 @@ int Server::relayout()
     if (drain(0) != FG_OK) return FG_E_CUDA;
     if (w) CK(cudaStreamSynchronize(stream));
     /* body motion of continuing scenes goes through the host (small) */
-    std::vector<double> hx, hv, hq, hL;
-    std::vector<float> hxf, hvf, hqf;
     if (w && w->nbodies) {
         const size_t B = w->nbodies;
-        hx.resize(4 * B); hv.resize(4 * B); hq.resize(4 * B); hL.resize(4 * B);
-        hxf.resize(4 * B); hvf.resize(4 * B); hqf.resize(4 * B);
-        CK(cudaMemcpy(hx.data(), w->bx, 32 * B, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(hv.data(), w->bv, 32 * B, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(hq.data(), w->bq, 32 * B, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(hL.data(), w->bL, 32 * B, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(hxf.data(), w->bxf, 16 * B, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(hvf.data(), w->bvf, 16 * B, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(hqf.data(), w->bqf, 16 * B, cudaMemcpyDeviceToHost));
+        moved = BodyMotion(B);
+        CK(cudaMemcpyAsync(moved.x.data(), w->bx, 32 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync(moved.v.data(), w->bv, 32 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync(moved.q.data(), w->bq, 32 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync(moved.L.data(), w->bL, 32 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync(moved.xf.data(), w->bxf, 16 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync(moved.vf.data(), w->bvf, 16 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaMemcpyAsync(moved.qf.data(), w->bqf, 16 * B, cudaMemcpyDeviceToHost, stream));
+        CK(cudaStreamSynchronize(stream));
     }
     const float4 *src_pos = nullptr, *src_vel = nullptr;
     const float2 *src_dp = nullptr;
@@ -267,11 +352,13 @@ int Server::relayout()
     }
     int r = dst->set_layout(descs.data(), (uint32_t)descs.size());
     if (r != FG_OK) return r;
+    BodyMotion bodies(dst->nbodies);
     for (size_t s = 0; s < active.size(); s++) {
         const FgScene &S = dst->scenes_h[s];
         auto it = where.find(active[s]->id);
         if (it == where.end()) {
-            if ((r = dst->upload_scene((uint32_t)s, descs[s])) != FG_OK) return r;
+            if ((r = dst->upload_particles((uint32_t)s, descs[s])) != FG_OK) return r;
+            bodies.rest(descs[s], S.body_base);
             continue;
         }
         const FgScene &O = old_scenes[it->second];
@@ -283,19 +370,12 @@ int Server::relayout()
             CK(cudaMemcpyAsync(dst->dp + S.pbase, src_dp + O.pbase, 8 * (size_t)S.n, cudaMemcpyDefault,
                                stream));
         }
-        if (S.nbodies) {
-            const size_t B = S.nbodies, ob = O.body_base, nb = S.body_base;
-            CK(cudaMemcpyAsync(dst->bx + nb, hx.data() + 4 * ob, 32 * B, cudaMemcpyHostToDevice, stream));
-            CK(cudaMemcpyAsync(dst->bv + nb, hv.data() + 4 * ob, 32 * B, cudaMemcpyHostToDevice, stream));
-            CK(cudaMemcpyAsync(dst->bq + nb, hq.data() + 4 * ob, 32 * B, cudaMemcpyHostToDevice, stream));
-            CK(cudaMemcpyAsync(dst->bL + nb, hL.data() + 4 * ob, 32 * B, cudaMemcpyHostToDevice, stream));
-            CK(cudaMemcpyAsync(dst->bxf + nb, hxf.data() + 4 * ob, 16 * B, cudaMemcpyHostToDevice, stream));
-            CK(cudaMemcpyAsync(dst->bvf + nb, hvf.data() + 4 * ob, 16 * B, cudaMemcpyHostToDevice, stream));
-            CK(cudaMemcpyAsync(dst->bqf + nb, hqf.data() + 4 * ob, 16 * B, cudaMemcpyHostToDevice, stream));
-        }
+        bodies.copy(moved, O.body_base, S.body_base, S.nbodies);
     }
+    r = dst->upload_bodies(bodies);
     /* the host staging arrays and the old world must outlive the copies */
     CK(cudaStreamSynchronize(stream));
+    if (r != FG_OK) return r;
     if (grow) w = std::move(nw);
     laid_out.resize(active.size());
     for (size_t s = 0; s < active.size(); s++) laid_out[s] = active[s]->id;
@@ -321,11 +401,9 @@ int Server::retire_finished()
             continue;
         }
         const FgScene &S = w->scenes_h[s];
-        q->out_pos.resize(4 * (size_t)S.n);
-        q->out_vel.resize(4 * (size_t)S.n);
-        if (S.n) {
-            CK(cudaMemcpy(q->out_pos.data(), w->pos + S.pbase, 16 * (size_t)S.n, cudaMemcpyDeviceToHost));
-            CK(cudaMemcpy(q->out_vel.data(), w->vel + S.pbase, 16 * (size_t)S.n, cudaMemcpyDeviceToHost));
+        if (S.n) { /* over the initial state */
+            CK(cudaMemcpy(q->pos.p, w->pos + S.pbase, 16 * (size_t)S.n, cudaMemcpyDeviceToHost));
+            CK(cudaMemcpy(q->vel.p, w->vel + S.pbase, 16 * (size_t)S.n, cudaMemcpyDeviceToHost));
         }
         q->state = FG_REQ_DONE;
         q->t_done = now();
@@ -478,10 +556,14 @@ int fg_server_submit(fg_server *srv, const fg_scene_desc *d, uint32_t steps, uin
     std::unique_ptr<Request> q(new Request());
     q->desc = *d;
     const size_t n = d->n_particles;
-    q->pos.assign(d->positions, d->positions + 4 * n);
-    if (d->velocities) q->vel.assign(d->velocities, d->velocities + 4 * n);
-    q->desc.positions = n ? q->pos.data() : nullptr;
-    q->desc.velocities = d->velocities ? q->vel.data() : nullptr;
+    if (!q->pos.alloc(S->pool, 4 * n) || !q->vel.alloc(S->pool, 4 * n)) {
+        set_error_msg("no host memory for the request's state");
+        return FG_E_OOM;
+    }
+    if (n) memcpy(q->pos.p, d->positions, 16 * n);
+    if (n && d->velocities) memcpy(q->vel.p, d->velocities, 16 * n);
+    q->desc.positions = q->pos.p;
+    q->desc.velocities = d->velocities ? q->vel.p : nullptr;
     q->bodies.assign(d->bodies, d->bodies + d->n_bodies);
     q->spheres.resize(d->n_bodies);
     for (uint32_t b = 0; b < d->n_bodies; b++) {
@@ -547,11 +629,33 @@ int fg_server_result(fg_server *srv, uint64_t id, float *pos4, float *vel4, int 
     if (it == S->all.end()) return FG_E_INVALID;
     Request &q = *it->second;
     if (q.state != FG_REQ_DONE) return FG_E_STATE;
-    if (pos4 && !q.out_pos.empty()) memcpy(pos4, q.out_pos.data(), sizeof(float) * q.out_pos.size());
-    if (vel4 && !q.out_vel.empty()) memcpy(vel4, q.out_vel.data(), sizeof(float) * q.out_vel.size());
+    const size_t n = q.desc.n_particles;
+    if (pos4 && n) memcpy(pos4, q.pos.p, 16 * n);
+    if (vel4 && n) memcpy(vel4, q.vel.p, 16 * n);
     if (release) S->all.erase(it);
     return FG_OK;
 }
+
+int fg_server_take(fg_server *srv, uint64_t id, fg_host_state **state, float **pos4, float **vel4)
+{
+    if (!srv || !state || !pos4 || !vel4) return FG_E_INVALID;
+    Server *S = (Server *)srv;
+    auto it = S->all.find(id);
+    if (it == S->all.end()) return FG_E_INVALID;
+    Request &q = *it->second;
+    if (q.state != FG_REQ_DONE) return FG_E_STATE;
+    HostState *h = new (std::nothrow) HostState();
+    if (!h) return FG_E_OOM;
+    h->pos.swap(q.pos);
+    h->vel.swap(q.vel);
+    *state = (fg_host_state *)h;
+    *pos4 = h->pos.p;
+    *vel4 = h->vel.p;
+    S->all.erase(it);
+    return FG_OK;
+}
+
+void fg_host_state_free(fg_host_state *state) { delete (HostState *)state; }
 
 int fg_server_stats(const fg_server *srv, fg_server_stats_info *st)
 {

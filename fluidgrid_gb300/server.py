@@ -9,6 +9,26 @@ from . import _ffi
 from ._ffi import check
 
 
+class _HostState:
+    """A finished request's arrays, given back when the last numpy view of them goes."""
+
+    def __init__(self, L, server, rid):
+        self.L, self.h = L, ctypes.c_void_p()
+        self.pos, self.vel = ctypes.c_void_p(), ctypes.c_void_p()
+        check(L.fg_server_take(server, int(rid), ctypes.byref(self.h), ctypes.byref(self.pos), ctypes.byref(self.vel)),
+              "fg_server_take")
+
+    def __del__(self):
+        if self.h:
+            self.L.fg_host_state_free(self.h)
+
+
+class _HostView:
+    def __init__(self, state, addr, n):
+        self.state = state
+        self.__array_interface__ = {"shape": (n, 4), "typestr": "<f4", "data": (addr, False), "version": 3}
+
+
 class Server:
     def __init__(self, budget_bytes=120 << 30, max_particles=None, max_admit_per_step=0, use_graphs=True,
                  grow_via_host=False, stream=None, pipeline_depth=0, target_step_ms=None, head_wait_s=None):
@@ -76,6 +96,11 @@ class Server:
     def result(self, rid, release=True):
         """Final (positions, velocities) of a finished request."""
         n = self.n_of[rid]
+        if release and n:
+            # the request's own arrays: no copy, and no fresh pages
+            s = _HostState(self.L, self.h, rid)
+            del self.n_of[rid]
+            return np.asarray(_HostView(s, s.pos.value, n)), np.asarray(_HostView(s, s.vel.value, n))
         pos = np.empty((n, 4), np.float32)
         vel = np.empty((n, 4), np.float32)
         check(self.L.fg_server_result(self.h, int(rid), ctypes.c_void_p(pos.ctypes.data),

@@ -408,6 +408,13 @@ int fg_server_request(const fg_server *s, uint64_t request_id, fg_request_info *
  * finished request; release = 1 forgets the request.  FG_E_STATE if it has
  * not finished. */
 int fg_server_result(fg_server *s, uint64_t request_id, float *pos4, float *vel4, int release);
+/* The same without the copy: the finished request's arrays become the
+ * caller's (NULL for a scene of no particles) until fg_host_state_free, and
+ * the request is forgotten.  They may outlive the server and be freed by any
+ * thread. */
+typedef struct fg_host_state fg_host_state;
+int fg_server_take(fg_server *s, uint64_t request_id, fg_host_state **state, float **pos4, float **vel4);
+void fg_host_state_free(fg_host_state *state);
 int fg_server_stats(const fg_server *s, fg_server_stats_info *stats);
 /* Request ids of the resident scenes (the ones the next step advances), at
  * most `cap` of them; *count receives how many are resident. */
