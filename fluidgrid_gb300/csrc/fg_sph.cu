@@ -34,17 +34,19 @@
 namespace fg {
 
 /* The density pass, by warp: fg_stage.cuh's staging, then a lane per target
- * over its staged candidates.  Bound by instruction issue (about 180 warp
- * instructions a target at 0.5 h spacing, of which 100 are staging, and 620 at
- * 0.32 h; the walk by thread took 237 and 700).  524,288 particles with lists,
- * ncu, walk by thread -> here: 180 -> 139 us at 0.5 h, 249 -> 253 at 0.45 h
- * (cells of 8 to 27 targets fill a warp badly), 366 -> 311 at 0.36 h, 506 ->
- * 447 at 0.32 h; 4,194,304 particles 1790 -> 1182 us; 16,384 particles, where
- * a thread's chain of 216 candidate loads was the pass, 37 -> 14 us.
+ * over its staged candidates, two candidates an instruction where the sums'
+ * order allows.  Bound by instruction issue (about 165 warp instructions a
+ * target at 0.5 h spacing, of which 100 are staging, and 540 at 0.32 h; the
+ * walk by thread took 237 and 700).  With lists, walk by thread -> staged, one
+ * candidate at a time -> here: 1M particles at 0.5 h 351 -> 243 -> 229 us, 1M
+ * compressed 922 -> 782 -> 725, 4M 1788 -> 1182 -> 1094, 262,144 at 0.45 h
+ * (cells of 8 to 27 targets fill a warp badly) 138 -> 136 -> 126; 16,384, where
+ * a thread's chain of 216 candidate loads was the pass, 37 -> 14.
  *
  * Staged candidates of a warp: its targets lie in four or five groups of some
- * 90 (60-100 candidates kept of a cell's 216).  384 leave ten CTAs an SM;
- * 512 (nine CTAs): 1509 against 1192 us at 4M, 275 against 246 at 1M. */
+ * 90 (60-100 candidates kept of a cell's 216).  384 and ten CTAs an SM leave
+ * the L1 60 KB: nine CTAs with 448, whose shared memory is no more, take 1395
+ * us at 4M, ten with 320, more rounds, 1265, eleven 1480. */
 #ifndef FG_DENSITY_STAGE
 #define FG_DENSITY_STAGE 384u
 #endif
@@ -54,11 +56,11 @@ namespace fg {
 #define FG_STAGE_GROUPS 9u /* a warp whose targets lie in more groups walks by thread */
 #define FG_DENSITY_THREADS 64u
 
-template <bool LIST>
 struct DensityShared {
-    float4 cand[FG_DENSITY_STAGE]; /* x, y, z, sorted index as bits */
+    /* candidates, by component: four candidates a load, in pairs */
+    float4 x[FG_DENSITY_STAGE / 4], y[FG_DENSITY_STAGE / 4], z[FG_DENSITY_STAGE / 4];
+    uint4 j[FG_DENSITY_STAGE / 4]; /* sorted index */
     uint32_t idx[FG_STAGE_WINDOW];
-    uint32_t ring[LIST ? 16 : 1][32]; /* each lane's newest list entries */
 };
 
 /* One lane's list entries on their way to its list: collected in a ring of
@@ -67,39 +69,50 @@ struct DensityShared {
  * or not, kept by the count, an entry costs no divergent branch (0.32 h, 1M:
  * 855 us with two entries a store in a branch, 767 us so). */
 struct ListRing {
-    uint32_t cnt, done; /* entries; entries stored, a multiple of 8 */
+    /* 16 entries of a word a thread; at = 256 times the count, plus the
+     * thread's byte in an entry, so that one AND gives a push its address */
+    uint32_t *ring;
+    uint32_t at, done; /* done: entries stored, a multiple of 8 */
 
-    /* j if it is in range */
-    __device__ __forceinline__ void push(uint32_t (*ring)[32], uint32_t lane, uint32_t j, bool in)
+    __device__ __forceinline__ explicit ListRing(uint32_t *shared) : ring(shared), at(4u * threadIdx.x), done(0u) {}
+    __device__ __forceinline__ uint32_t count() const { return at >> 8; }
+    __device__ __forceinline__ uint32_t &slot(uint32_t a) const
     {
-        ring[cnt & 15u][lane] = j;
-        cnt += in ? 1u : 0u;
+        return *(uint32_t *)((char *)ring + (a & (16u * 256u - 4u)));
     }
-    __device__ __forceinline__ uint4 four(const uint32_t (*ring)[32], uint32_t lane, uint32_t k) const
+    /* j if it is in range */
+    __device__ __forceinline__ void push(uint32_t j, bool in)
     {
-        const uint32_t b = k & 15u; /* a multiple of 4 */
-        return make_uint4(ring[b][lane], ring[b + 1u][lane], ring[b + 2u][lane], ring[b + 3u][lane]);
+        slot(at) = j;
+        at += in ? 256u : 0u;
+    }
+    __device__ __forceinline__ uint4 four(uint32_t k) const
+    {
+        const uint32_t a = 256u * k + 4u * threadIdx.x; /* k: a multiple of 4 */
+        return make_uint4(slot(a), slot(a + 256u), slot(a + 512u), slot(a + 768u));
     }
     /* after at most eight pushes since the last call */
-    __device__ __forceinline__ void spill(const uint32_t (*ring)[32], uint32_t lane, uint32_t *lp, uint32_t cap)
+    __device__ __forceinline__ void spill(uint32_t *lp, uint32_t cap)
     {
-        if (cnt - done >= 8u) {
+        if (count() - done >= 8u) {
             if (done + 8u <= cap)
-                fg_st_list8(lp + done, four(ring, lane, done), four(ring, lane, done + 4u));
+                fg_st_list8(lp + done, four(done), four(done + 4u));
             else if (done + 4u <= cap)
-                fg_st_list4(lp + done, four(ring, lane, done));
+                fg_st_list4(lp + done, four(done));
             done += 8u;
         }
     }
     /* the rest, padded to a whole group of four with the target itself, which
      * the force pass skips, so it reads only whole groups */
-    __device__ __forceinline__ void finish(uint32_t (*ring)[32], uint32_t lane, uint32_t *lp, uint32_t cap, uint32_t self)
+    __device__ __forceinline__ void finish(uint32_t *lp, uint32_t cap, uint32_t self)
     {
+        const uint32_t cnt = count();
         if (cnt > cap) return;
-        for (uint32_t k = cnt; k & 3u; k++) ring[k & 15u][lane] = self;
-        for (; done < cnt; done += 4u) fg_st_list4(lp + done, four(ring, lane, done));
+        for (uint32_t a = at; a & 768u; a += 256u) slot(a) = self;
+        for (; done < cnt; done += 4u) fg_st_list4(lp + done, four(done));
     }
 };
+static_assert(FG_DENSITY_THREADS == 64u, "a ring entry is a word of each of 64 threads");
 
 template <bool LIST, bool COUNT>
 __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density(
@@ -109,8 +122,9 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
     float2 *__restrict__ dp, float gas_o, float rest_o, float mass_o, int use_o, const __grid_constant__ NbrList list,
     unsigned long long *__restrict__ pairs)
 {
-    __shared__ DensityShared<LIST> shared[FG_DENSITY_THREADS / 32];
-    DensityShared<LIST> &sm = shared[threadIdx.x >> 5];
+    __shared__ DensityShared shared[FG_DENSITY_THREADS / 32];
+    __shared__ uint32_t s_ring[LIST ? 16 * FG_DENSITY_THREADS : 1];
+    DensityShared &sm = shared[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t cap = LIST ? __ldg(list.cap) : 0u;
     unsigned long long pc = 0; /* in-range density visits of this thread */
@@ -140,7 +154,8 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
         const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
         DensityAcc acc;
         acc.init();
-        ListRing ring = {0u, 0u};
+        ListRing ring(s_ring);
+        uint32_t count = 0u; /* without a list */
         /* lists by sorted index: the force pass may visit the targets in another order */
         uint32_t *lp = LIST ? list.idx + (size_t)i * list.stride : nullptr;
         uint32_t lead, leads;
@@ -150,22 +165,39 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
             fg_stage_rounds<FG_DENSITY_STAGE>(
                 sig, lead, leads, px, py, pz, G, spos, start, end, sm.idx,
                 [&](uint32_t slot, uint32_t j, float4 c) {
-                    sm.cand[slot] = make_float4(c.x, c.y, c.z, __uint_as_float(j));
+                    ((float *)sm.x)[slot] = c.x;
+                    ((float *)sm.y)[slot] = c.y;
+                    ((float *)sm.z)[slot] = c.z;
+                    ((uint32_t *)sm.j)[slot] = j;
                 },
                 [&](uint32_t first, uint32_t stop, uint32_t) {
-                    for (uint32_t k = first; k < stop; k += 8u) {
+                    const F2 px2 = fg_pack(px, px), py2 = fg_pack(py, py), pz2 = fg_pack(pz, pz);
+                    const F2 ns2 = fg_pack(-scale, -scale), hh2 = fg_pack(h2, h2);
+                    for (uint32_t k = first >> 2; k < stop >> 2; k += 2u) {
 #pragma unroll
-                        for (uint32_t e = 0; e < 8u; e++) {
-                            const float4 q = sm.cand[k + e];
-                            const bool in = acc.term(q, px, py, pz, scale, h2);
-                            if (LIST) ring.push(sm.ring, lane, __float_as_uint(q.w), in);
-                            else if (COUNT) ring.cnt += in ? 1u : 0u;
+                        for (uint32_t e = 0; e < 2u; e++) {
+                            const float4 x = sm.x[k + e], y = sm.y[k + e], z = sm.z[k + e];
+                            const uint4 j = LIST ? sm.j[k + e] : make_uint4(0u, 0u, 0u, 0u);
+                            bool in[4];
+                            acc.term2(fg_pack(x.x, x.y), fg_pack(y.x, y.y), fg_pack(z.x, z.y), px2, py2, pz2, ns2, hh2,
+                                      h2, in[0], in[1]);
+                            acc.term2(fg_pack(x.z, x.w), fg_pack(y.z, y.w), fg_pack(z.z, z.w), px2, py2, pz2, ns2, hh2,
+                                      h2, in[2], in[3]);
+                            if (LIST) {
+                                ring.push(j.x, in[0]);
+                                ring.push(j.y, in[1]);
+                                ring.push(j.z, in[2]);
+                                ring.push(j.w, in[3]);
+                            } else if (COUNT) {
+#pragma unroll
+                                for (int u = 0; u < 4; u++) count += in[u] ? 1u : 0u;
+                            }
                         }
-                        if (LIST) ring.spill(sm.ring, lane, lp, cap);
+                        if (LIST) ring.spill(lp, cap);
                     }
                 });
-            if (LIST && active) ring.finish(sm.ring, lane, lp, cap, i);
-            acc.cnt = ring.cnt;
+            if (LIST && active) ring.finish(lp, cap, i);
+            acc.cnt = LIST ? ring.count() : count;
         } else if (active) {
             fg_walk27(
                 p.x, p.y, p.z, S, start, end,

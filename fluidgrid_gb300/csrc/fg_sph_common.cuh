@@ -54,6 +54,33 @@ __device__ __forceinline__ void fg_walk27(float px, float py, float pz, const Fg
     fg_walk27(px, py, pz, S, start, end, fn, [] {});
 }
 
+/* Two floats in a register pair, an instruction for both. */
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 fg_pack(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 fg_unpack(F2 v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ F2 fg_fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ F2 fg_mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 /* One target's state in a density pass: the sum of (h^2 - l^2)^3 over the
  * candidates with l <= h (an exact 0 at l = h, so the sum equals the
  * reference's l < h sum) and the force pass's neighbour list (every visit
@@ -74,17 +101,37 @@ struct DensityAcc {
         q2 = q3 = 0;
     }
 
+    __device__ __forceinline__ void add(float t3)
+    {
+        const float u = __fadd_rn(s, t3);
+        c = __fadd_rn(c, __fsub_rn(t3, __fsub_rn(u, s)));
+        s = u;
+    }
+
     /* add a candidate's (h^2 - l^2)^3, 0 beyond h; whether it is in range */
     __device__ __forceinline__ bool term(float4 q, float px, float py, float pz, float scale, float h2)
     {
         const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
         const float t = fmaxf(__fsub_rn(h2, r2), 0.0f); /* 0 for a NaN too */
-        const float t3 = __fmul_rn(__fmul_rn(t, t), t);
-        const float u = __fadd_rn(s, t3);
-        c = __fadd_rn(c, __fsub_rn(t3, __fsub_rn(u, s)));
-        s = u;
+        add(__fmul_rn(__fmul_rn(t, t), t));
         return r2 <= h2;
+    }
+
+    /* term() for two candidates, first and second of the pairs: the same
+     * operations, all but the sums two to an instruction */
+    __device__ __forceinline__ void term2(F2 x, F2 y, F2 z, F2 px, F2 py, F2 pz, F2 nscale, F2 h2, float h2s, bool &in0,
+                                          bool &in1)
+    {
+        const F2 dx = fg_fma2(x, nscale, px), dy = fg_fma2(y, nscale, py), dz = fg_fma2(z, nscale, pz);
+        const F2 r2 = fg_fma2(dx, dx, fg_fma2(dy, dy, fg_mul2(dz, dz)));
+        const float2 r = fg_unpack(r2), d = fg_unpack(fg_fma2(r2, fg_pack(-1.0f, -1.0f), h2));
+        const F2 t = fg_pack(fmaxf(d.x, 0.0f), fmaxf(d.y, 0.0f));
+        const float2 t3 = fg_unpack(fg_mul2(fg_mul2(t, t), t));
+        add(t3.x);
+        add(t3.y);
+        in0 = r.x <= h2s;
+        in1 = r.y <= h2s;
     }
 
     __device__ __forceinline__ float sum() const { return __fadd_rn(s, c); }
