@@ -186,6 +186,7 @@ struct World {
         cudaGraph_t graph;
         cudaGraphExec_t exec;
         StepIO io;
+        uint64_t launches = 0;
     };
     std::vector<CachedGraph> graphs;
     /* graphs whose parameters a layout change or a list reallocation made
@@ -195,6 +196,8 @@ struct World {
     uint64_t graph_signature() const;
     int graph_for_current(cudaGraphExec_t *out, uint32_t nsteps = 1);
     uint32_t graph_steps = 1; /* steps per captured graph launch */
+    bool graph_steps_chosen = false; /* explicitly: small worlds otherwise join steps (graph_span) */
+    uint32_t graph_span(uint32_t left) const;
     bool host_boundary(uint64_t s) const;
     /* online autotuner: every tune_period steps, each candidate value of one
      * tunable (kernel, block warps, digit width; the tunable rotates) runs

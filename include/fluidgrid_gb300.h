@@ -212,7 +212,9 @@ int fg_world_set_graphs(fg_world *w, int on);
  *   FG_OPT_LIST_AUTOGROW  kernel 1: 1 = every 25 steps grow the capacity to
  *                         1.125x the largest in-range count seen (default)
  *   FG_OPT_GRAPH_STEPS    steps captured in one CUDA graph launch (1..64,
- *                         default 1); such a launch never spans an
+ *                         default 1; until it is set, small worlds join up
+ *                         to four steps of one call once their step has been
+ *                         replayed a while); such a launch never spans an
  *                         autotuning round or a list capacity check
  *   FG_OPT_CTAS_PER_SM    kernels 0/1: CTAs per SM of the persistent
  *                         128-thread density/force grids (0 = 64; the
