@@ -41,7 +41,10 @@ namespace fg {
  * candidate at a time -> here: 1M particles at 0.5 h 351 -> 243 -> 229 us, 1M
  * compressed 922 -> 782 -> 725, 4M 1788 -> 1182 -> 1094, 262,144 at 0.45 h
  * (cells of 8 to 27 targets fill a warp badly) 138 -> 136 -> 126; 16,384, where
- * a thread's chain of 216 candidate loads was the pass, 37 -> 14.
+ * a thread's chain of 216 candidate loads was the pass, 37 -> 14.  64 worlds of
+ * 1.23M particles that have splashed apart, whose warps lie in more and smaller
+ * groups: 379 -> 378 after 20 steps, 504 -> 521 after 400 (a warp of more than
+ * nine groups walking by thread instead: 415 and 547).
  *
  * Staged candidates of a warp: its targets lie in four or five groups of some
  * 90 (60-100 candidates kept of a cell's 216).  384 and ten CTAs an SM leave
@@ -53,7 +56,7 @@ namespace fg {
 #ifndef FG_DENSITY_CTAS
 #define FG_DENSITY_CTAS 10
 #endif
-#define FG_STAGE_GROUPS 9u /* a warp whose targets lie in more groups walks by thread */
+#define FG_STAGE_GROUPS 9u /* staged together; a warp of more takes them nine by nine */
 #define FG_DENSITY_THREADS 64u
 
 struct DensityShared {
@@ -159,43 +162,49 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
         /* lists by sorted index: the force pass may visit the targets in another order */
         uint32_t *lp = LIST ? list.idx + (size_t)i * list.stride : nullptr;
         uint32_t lead, leads;
-        const bool staged = fg_stage_groups(sig, __ballot_sync(FG_FULL, active), FG_STAGE_GROUPS, lead, leads) &&
-                            !__any_sync(FG_FULL, active && sig.odd);
-        if (staged) {
-            fg_stage_rounds<FG_DENSITY_STAGE>(
-                sig, lead, leads, px, py, pz, G, spos, start, end, sm.idx,
-                [&](uint32_t slot, uint32_t j, float4 c) {
-                    ((float *)sm.x)[slot] = c.x;
-                    ((float *)sm.y)[slot] = c.y;
-                    ((float *)sm.z)[slot] = c.z;
-                    ((uint32_t *)sm.j)[slot] = j;
-                },
-                [&](uint32_t first, uint32_t stop, uint32_t) {
-                    const F2 px2 = fg_pack(px, px), py2 = fg_pack(py, py), pz2 = fg_pack(pz, pz);
-                    const F2 ns2 = fg_pack(-scale, -scale), hh2 = fg_pack(h2, h2);
-                    for (uint32_t k = first >> 2; k < stop >> 2; k += 2u) {
+        if (!__any_sync(FG_FULL, active && sig.odd)) {
+            fg_stage_groups(sig, __ballot_sync(FG_FULL, active), lead, leads);
+            while (leads) {
+                /* the first FG_STAGE_GROUPS of the groups left */
+                uint32_t later = leads;
+                for (uint32_t k = 0u; k < FG_STAGE_GROUPS; k++) later &= later - 1u;
+                const uint32_t batch = leads ^ later;
+                leads = later;
+                fg_stage_rounds<FG_DENSITY_STAGE>(
+                    sig, lead, batch, px, py, pz, G, spos, start, end, sm.idx,
+                    [&](uint32_t slot, uint32_t j, float4 c) {
+                        ((float *)sm.x)[slot] = c.x;
+                        ((float *)sm.y)[slot] = c.y;
+                        ((float *)sm.z)[slot] = c.z;
+                        ((uint32_t *)sm.j)[slot] = j;
+                    },
+                    [&](uint32_t first, uint32_t stop, uint32_t) {
+                        const F2 px2 = fg_pack(px, px), py2 = fg_pack(py, py), pz2 = fg_pack(pz, pz);
+                        const F2 ns2 = fg_pack(-scale, -scale), hh2 = fg_pack(h2, h2);
+                        for (uint32_t k = first >> 2; k < stop >> 2; k += 2u) {
 #pragma unroll
-                        for (uint32_t e = 0; e < 2u; e++) {
-                            const float4 x = sm.x[k + e], y = sm.y[k + e], z = sm.z[k + e];
-                            const uint4 j = LIST ? sm.j[k + e] : make_uint4(0u, 0u, 0u, 0u);
-                            bool in[4];
-                            acc.term2(fg_pack(x.x, x.y), fg_pack(y.x, y.y), fg_pack(z.x, z.y), px2, py2, pz2, ns2, hh2,
-                                      h2, in[0], in[1]);
-                            acc.term2(fg_pack(x.z, x.w), fg_pack(y.z, y.w), fg_pack(z.z, z.w), px2, py2, pz2, ns2, hh2,
-                                      h2, in[2], in[3]);
-                            if (LIST) {
-                                ring.push(j.x, in[0]);
-                                ring.push(j.y, in[1]);
-                                ring.push(j.z, in[2]);
-                                ring.push(j.w, in[3]);
-                            } else if (COUNT) {
+                            for (uint32_t e = 0; e < 2u; e++) {
+                                const float4 x = sm.x[k + e], y = sm.y[k + e], z = sm.z[k + e];
+                                const uint4 j = LIST ? sm.j[k + e] : make_uint4(0u, 0u, 0u, 0u);
+                                bool in[4];
+                                acc.term2(fg_pack(x.x, x.y), fg_pack(y.x, y.y), fg_pack(z.x, z.y), px2, py2, pz2, ns2,
+                                          hh2, h2, in[0], in[1]);
+                                acc.term2(fg_pack(x.z, x.w), fg_pack(y.z, y.w), fg_pack(z.z, z.w), px2, py2, pz2, ns2,
+                                          hh2, h2, in[2], in[3]);
+                                if (LIST) {
+                                    ring.push(j.x, in[0]);
+                                    ring.push(j.y, in[1]);
+                                    ring.push(j.z, in[2]);
+                                    ring.push(j.w, in[3]);
+                                } else if (COUNT) {
 #pragma unroll
-                                for (int u = 0; u < 4; u++) count += in[u] ? 1u : 0u;
+                                    for (int u = 0; u < 4; u++) count += in[u] ? 1u : 0u;
+                                }
                             }
+                            if (LIST) ring.spill(lp, cap);
                         }
-                        if (LIST) ring.spill(lp, cap);
-                    }
-                });
+                    });
+            }
             if (LIST && active) ring.finish(lp, cap, i);
             acc.cnt = LIST ? ring.count() : count;
         } else if (active) {
@@ -576,7 +585,7 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
             const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
             float fx = 0.f, fy = 0.f, fz = 0.f;
             uint32_t lead, leads;
-            fg_stage_groups(sig, __ballot_sync(FG_FULL, active && !sig.odd), 32u, lead, leads);
+            fg_stage_groups(sig, __ballot_sync(FG_FULL, active && !sig.odd), lead, leads);
             for (; leads; leads &= leads - 1u) {
                 const uint32_t l = (uint32_t)__ffs((int)leads) - 1u;
                 const uint32_t group = __ballot_sync(FG_FULL, lead == l);
@@ -776,9 +785,10 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out)
 {
     if (!L.nwork) return;
-    /* a CTA per item: most have nothing to search and leave their SM to the
-     * kernels beside this one */
-    k_fluid_contact<<<L.nwork, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos, vel,
+    /* an SM's worth of CTAs: a CTA per item queues ahead of the grid kernels
+     * beside this one (64 worlds after 400 steps 896 us a step, here 883; 4M
+     * particles 2163, here 2135) */
+    k_fluid_contact<<<grid_for(L.nwork, 8), FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos, vel,
                                                                   G, out);
 }
 

@@ -69,9 +69,8 @@ __device__ __forceinline__ StageSig fg_stage_sig(float4 p, const StageGrid &G)
 }
 
 /* The lane of the first target with the same signature, for each lane of
- * `todo` (whole warp, converged); gives up (returns false) beyond max groups. */
-__device__ __forceinline__ bool fg_stage_groups(const StageSig &s, uint32_t todo, uint32_t max, uint32_t &lead,
-                                                uint32_t &leads)
+ * `todo` (whole warp, converged). */
+__device__ __forceinline__ void fg_stage_groups(const StageSig &s, uint32_t todo, uint32_t &lead, uint32_t &leads)
 {
     const uint32_t lane = threadIdx.x & 31u;
     leads = 0u;
@@ -85,9 +84,7 @@ __device__ __forceinline__ bool fg_stage_groups(const StageSig &s, uint32_t todo
         if (same) lead = (uint32_t)l;
         todo &= ~__ballot_sync(FG_FULL, same);
         leads |= 1u << l;
-        if (max-- == 0u) return false;
     }
-    return true;
 }
 
 /* minimum / maximum over the warp, NaN ignored */
