@@ -12,7 +12,7 @@
  * (z-y-x order, same hashed buckets, a bucket reached twice is summed twice);
  * bucket indices are bit-exact.  Pair arithmetic is reorganised for the
  * GPU: squared-distance tests, rsqrt/rcp instead of divides, compensated
- * density sums (plain within a bucket, Kahan across buckets); the results
+ * density sums (each term's rounding error added up beside); the results
  * agree with the reference arithmetic to the tolerances the parity tests
  * state.
  *
@@ -35,8 +35,8 @@ namespace fg {
 
 /* The density pass, by warp: fg_stage.cuh's staging, then a lane per target
  * over its staged candidates, two candidates an instruction where the sums'
- * order allows.  Bound by instruction issue (about 165 warp instructions a
- * target at 0.5 h spacing, of which 100 are staging, and 540 at 0.32 h; the
+ * order allows.  Bound by instruction issue (about 167 warp instructions a
+ * target at 0.5 h spacing, of which 100 are staging, and 583 at 0.32 h; the
  * walk by thread took 237 and 700).  With lists, walk by thread -> staged, one
  * candidate at a time -> here: 1M particles at 0.5 h 351 -> 243 -> 229 us, 1M
  * compressed 922 -> 782 -> 725, 4M 1788 -> 1182 -> 1094, 262,144 at 0.45 h
