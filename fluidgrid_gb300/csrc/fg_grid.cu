@@ -381,7 +381,7 @@ __global__ void k_iota_copy(const uint32_t *__restrict__ kin, const uint32_t *__
 }
 
 /* ---- up to 65,536 pairs: the whole sort in one launch ----
- * One cluster of up to eight CTAs keeps the pairs on chip: ITEMS a thread in
+ * One cluster of up to sixteen CTAs keeps the pairs on chip: ITEMS a thread in
  * registers, ranked in the CTA as k_rs_downsweep does; the CTAs read one
  * another's digit totals, order their tile by digit in shared memory and write
  * its runs into one another's, two cluster barriers a pass, 8 bits a pass.  A
@@ -389,13 +389,14 @@ __global__ void k_iota_copy(const uint32_t *__restrict__ kin, const uint32_t *__
  * three kernels a pass above are, at these sizes, launches and latency.
  * Measured in a captured graph, three kernels a pass before (with a
  * match_any a key) -> one launch, 17 bits: 39.9 -> 10.9 us at 4,096 pairs,
- * 40.6 -> 15.9 at 16,384, 42.4 -> 23.8 at 32,768, 42.7 -> 32.4 at 65,536; 32
- * bits, no digit shared: 52 -> 14.2, 21.1, 32.0, 56 -> 44.6.  The time is the
- * ranking and the staging of eight pairs a thread on eight SMs by then.
- * Scattering each pair straight into the other CTA's memory, a word at a time,
- * took 43.3 us at 65,536 pairs of 17 bits: 32 destinations a warp. */
+ * 40.6 -> 13.5 at 16,384, 42.4 -> 18.0 at 32,768, 42.7 -> 25.8 at 65,536; 32
+ * bits, no digit shared: 52 -> 14.1, 17.8, 24.3, 56 -> 35.2.  The time is the
+ * ranking and the staging of four pairs a thread on sixteen SMs by then (of
+ * eight on eight, the portable cluster: 32.4 and 44.6).  Scattering each pair
+ * straight into the other CTA's memory, a word at a time, took 43.3 us at
+ * 65,536 pairs of 17 bits on eight: 32 destinations a warp. */
 #define CS_THREADS 1024
-#define CS_CTAS 8u
+#define CS_CTAS 16u
 
 struct TileRank {
     uint16_t whist[CS_THREADS / 32][RS_RADIX];
@@ -549,34 +550,59 @@ __global__ void __launch_bounds__(CS_THREADS, 1) k_sort_cluster(const uint32_t *
 }
 
 template <int ITEMS>
+static cudaError_t cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, uint32_t ctas, cudaStream_t st)
+{
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(CS_THREADS);
+    cfg.dynamicSmemBytes = sizeof(ClusterSort<ITEMS>);
+    cfg.stream = st;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)cfg.dynamicSmemBytes);
+    if (e != cudaSuccess || ctas <= 8u) return e;
+    return cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+
+/* CTAs of the largest cluster that the GPU places: sixteen, or the portable
+ * eight where no part of it has sixteen SMs together (a partition). */
+static uint32_t cluster_ctas()
+{
+    static uint32_t ctas = 0u;
+    if (!ctas) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        int active = 0;
+        if (cluster_config<4>(cfg, at[0], CS_CTAS, 0) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&active, k_sort_cluster<4>, &cfg) != cudaSuccess)
+            active = 0;
+        if (!active) cudaGetLastError();
+        ctas = active > 0 ? CS_CTAS : 8u;
+    }
+    return ctas;
+}
+
+template <int ITEMS>
 static cudaError_t cluster_sort(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, uint32_t n,
                                 uint32_t bits, cudaStream_t st)
 {
-    const size_t smem = sizeof(ClusterSort<ITEMS>);
-    cudaError_t e = cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
     uint32_t ctas = 1u;
     while (ctas * CS_THREADS * ITEMS < n) ctas <<= 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(CS_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = ctas;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    const cudaError_t e = cluster_config<ITEMS>(cfg, at[0], ctas, st);
+    if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, k_sort_cluster<ITEMS>, kin, vin, kout, vout, n, bits);
 }
 
 /* Pairs that one launch sorts.  The three kernels a pass, over the whole chip,
  * take 34.6 us for one pair more (17 bits; 32 bits: 44.2), where the cluster
- * takes 32.4 (44.6, and less with each digit it skips); below that theirs
- * stay at that latency. */
-#define CS_MAX (CS_CTAS * CS_THREADS * 8u)
+ * takes 25.8 (35.2, and less with each digit it skips); with eight pairs a
+ * thread it meets them at 98,304 pairs (34.6 and 34.6; 24 bits: 37.0 and 35.2). */
+#define CS_MAX (CS_CTAS * CS_THREADS * 4u)
 
 bool radix_one_launch(uint32_t n) { return n <= CS_MAX; }
 
@@ -598,8 +624,8 @@ cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_
         return cudaSuccess;
     }
     if (radix_one_launch(n)) {
-        /* as many CTAs as give each thread one pair, up to eight CTAs */
-        const uint32_t per = CS_CTAS * CS_THREADS;
+        /* as many CTAs as give each thread one pair, up to the largest cluster */
+        const uint32_t per = cluster_ctas() * CS_THREADS;
         if (n <= per) return cluster_sort<1>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
         if (n <= 2u * per) return cluster_sort<2>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
         if (n <= 4u * per) return cluster_sort<4>(keys_in, vals_in, keys_out, vals_out, n, bits, st);

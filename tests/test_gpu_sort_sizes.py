@@ -1,5 +1,5 @@
 """The pair sort across its forms: one launch up to 65,536 pairs (a thread one
-to eight pairs, one to eight CTAs), three kernels a pass beyond, odd and even
+to eight pairs, one to sixteen CTAs), three kernels a pass beyond, odd and even
 pass counts in place, digits that all keys share, many ties; against a stable
 key sort."""
 import ctypes
