@@ -78,6 +78,28 @@ fg::Launch single_launch(const FgScene *S, uint32_t n)
     return L;
 }
 
+/* single_launch of a pass that runs two kernels beside each other: the second
+ * stream is the device's, made by the first such call.  Several threads may
+ * share it, as they share the legacy stream it is forked from and joined to. */
+fg::Launch staged_launch(const FgScene *S, uint32_t n)
+{
+    constexpr int kDevices = 32;
+    static fg::SideStream sides[kDevices];
+    fg::Launch L = single_launch(S, n);
+    int dev = kDevices;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= kDevices) return L;
+    std::lock_guard<std::mutex> lk(g_mu);
+    fg::SideStream &s = sides[dev];
+    if (!s.stream && (cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) != cudaSuccess ||
+                      cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) != cudaSuccess ||
+                      cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess)) {
+        cudaGetLastError(); /* without it: one kernel, which takes every range */
+        s.stream = nullptr;
+    }
+    L.side = s;
+    return L;
+}
+
 void finish()
 {
     cudaError_t e = cudaPeekAtLastError();
@@ -246,7 +268,7 @@ void gCalcMassDensity(float4 *orderedPositions, float2 *mass_pressure, unsigned 
     if (!g_have_params || !g_have_kc) { g_status = FG_E_STATE; return; }
     if (numParticles <= 0) { g_status = FG_OK; return; }
     FgScene S = fluid_scene();
-    fg::launch_density(single_launch(&S, (uint32_t)numParticles), orderedPositions, gridStart, gridEnd,
+    fg::launch_density(staged_launch(&S, (uint32_t)numParticles), orderedPositions, gridStart, gridEnd,
                        mass_pressure, gasConstant, restDensity, mass, 1);
     finish();
 }

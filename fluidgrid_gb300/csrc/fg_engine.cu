@@ -93,6 +93,8 @@ World::~World()
     if (ev_io_fork) cudaEventDestroy(ev_io_fork);
     if (ev_vel_in) cudaEventDestroy(ev_vel_in);
     if (ev_pos_in) cudaEventDestroy(ev_pos_in);
+    if (ev_walk) cudaEventDestroy(ev_walk);
+    if (ev_walk_done) cudaEventDestroy(ev_walk_done);
     if (stream2) cudaStreamDestroy(stream2);
     if (stream3) cudaStreamDestroy(stream3);
     if (own_stream && stream) cudaStreamDestroy(stream);
@@ -310,6 +312,7 @@ int World::reserve(const Capacity &c)
     k_set_u32<<<1, 1, 0, stream>>>(list_cap_d, list_cap);
     nbr.max_count = max_count;
     nbr.overflow = overflow_counter;
+    nbr.dispersed = max_count + 2;
     CK(cudaMemsetAsync(dp, 0, 8 * N, stream));
     CK(cudaMemsetAsync(vel, 0, 16 * N, stream));
     CK(cudaMemsetAsync(end, 0, 4 * NB, stream));
@@ -568,6 +571,8 @@ int World::init_stream(cudaStream_t st)
     CK(cudaEventCreateWithFlags(&ev_io_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_vel_in, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_pos_in, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ev_walk, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ev_walk_done, cudaEventDisableTiming));
     return FG_OK;
 }
 
@@ -611,6 +616,7 @@ Launch World::fluid_launch() const
     L.stream = stream;
     L.ctas_per_sm = ctas_per_sm;
     L.block = block;
+    if (dispersed || !use_list) L.side = SideStream{stream3, ev_walk, ev_walk_done};
     return L;
 }
 
@@ -884,7 +890,7 @@ uint32_t World::enqueue_step(cudaEvent_t *ev)
             launch_density(L, spos, start, end, dp, 0.f, 0.f, 0.f, 0, svel, use_list ? &nbr : nullptr,
                            pair_counter);
         mark(3, 1);
-        launches++;
+        launches += use_cc ? 1u : density_launches(L);
     }
     if (rb && !fork) {
         enqueue_rb_grid(stream, ev, launches);
@@ -952,6 +958,7 @@ uint64_t World::graph_signature() const
            ((ordered && order_forces_only) ? 1ull << 19 : 0ull) | ((uint64_t)(ctas_per_sm & 0x7fu) << 20) |
            (one_pass_sort ? 1ull << 27 : 0ull) | (bucket_sort_on ? 1ull << 28 : 0ull) |
            ((uint64_t)((block >> 6) & 0x7u) << 29) | ((uint64_t)(cc_warps & 0x7u) << 32) |
+           (dispersed ? 1ull << 35 : 0ull) |
            ((uint64_t)nbr.stride << 40);
 }
 
@@ -1131,17 +1138,33 @@ int World::tune_finish()
 
 /* Every FG_LIST_CHECK_PERIOD steps (kernel 1): grow the neighbour-list
  * capacity to 1.125x the largest in-range count seen since the last check,
- * so the force pass walks lists instead of buckets as a scene compresses. */
+ * so the force pass walks lists instead of buckets as a scene compresses; and
+ * give the density pass's dispersed ranges a kernel of their own while they
+ * are an eighth of all or more. */
 int World::check_list_cap()
 {
-    uint32_t mx = 0;
-    CK(cudaMemcpyAsync(&mx, max_count, 4, cudaMemcpyDeviceToHost, stream));
+    const bool grow = step_count % FG_LIST_CHECK_PERIOD == 0;
+    uint32_t seen[3]; /* largest count, the capacity, dispersed ranges */
+    CK(cudaMemcpyAsync(seen, max_count, sizeof(seen), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
+    CK(cudaMemsetAsync(nbr.dispersed, 0, 4, stream));
+    /* an eighth of the ranges is counted, four to a work item */
+    dispersed = seen[2] && 16ull * seen[2] >= (step_count - checked_at) * nwork;
+    checked_at = step_count;
+    if (!grow) return FG_OK;
     CK(cudaMemsetAsync(max_count, 0, 4, stream));
+    const uint32_t mx = seen[0];
     if (mx <= list_cap) return FG_OK;
     const uint32_t want = std::min<uint32_t>(((mx + mx / 8u) + 31u) & ~31u, FG_LIST_CAP_MAX);
     if (want <= list_cap) return FG_OK;
     return set_list_cap(want);
+}
+
+/* Whether step s starts by that check, the one for dispersed ranges also after
+ * the first step. */
+bool World::list_check_due(uint64_t s) const
+{
+    return use_list && list_autogrow && s && (s % FG_LIST_CHECK_PERIOD == 0 || (s == 1 && density_ranges_wide(nwork)));
 }
 
 /* Whether step s starts by refreshing the Morton target order. */
@@ -1156,7 +1179,7 @@ bool World::order_refresh_due(uint64_t s) const
 bool World::host_boundary(uint64_t s) const
 {
     if (tune_period && s % tune_period == 0) return true;
-    if (use_list && list_autogrow && s % FG_LIST_CHECK_PERIOD == 0) return true;
+    if (list_check_due(s) || (use_list && list_autogrow && !s)) return true;
     if (order_refresh_due(s)) return true;
     return false;
 }
@@ -1216,7 +1239,7 @@ int World::step_loop(uint32_t nsteps)
             k += span - 1;
             continue;
         }
-        if (use_list && list_autogrow && step_count && (step_count % FG_LIST_CHECK_PERIOD == 0)) {
+        if (list_check_due(step_count)) {
             int r = check_list_cap();
             if (r != FG_OK) return r;
         }
@@ -1284,7 +1307,7 @@ int World::run_stage(int stage, int flags)
             tune_apply(tr.dim, tr.prev);
             tr.active = false;
         }
-        if (use_list && list_autogrow && step_count && (step_count % FG_LIST_CHECK_PERIOD == 0)) {
+        if (list_check_due(step_count)) {
             int r = check_list_cap();
             if (r != FG_OK) return r;
         }
@@ -1420,7 +1443,7 @@ uint32_t World::launches_per_step()
     if (stages & FG_STAGE_SORT) c += sort_launches();
     /* + one memset node; none with the counting sort's fused reorder */
     if ((stages & FG_STAGE_RANGES) && !(bucket_sort_on && bucket_sort_fits() && (stages & FG_STAGE_SORT))) c += 1;
-    if (stages & FG_STAGE_DENSITY) c += 1;
+    if (stages & FG_STAGE_DENSITY) c += use_cc ? 1u : density_launches(fluid_launch());
     if (nbodies) {
         if (stages & FG_STAGE_RB_GRID) /* aabb reset, hash, sort + ranges */
             c += rb_small_scenes ? 3 : 3 + radix_launches(nspheres, rb_key_bits, 8);

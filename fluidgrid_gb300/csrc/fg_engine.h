@@ -149,7 +149,10 @@ struct World {
     bool own_stream = false;
     cudaStream_t stream2 = nullptr; /* rigid-body branch of a full step */
     cudaEvent_t ev_fork = nullptr, ev_fluid_ready = nullptr, ev_rb_done = nullptr, ev_bodies_done = nullptr;
-    cudaStream_t stream3 = nullptr; /* velocity upload of an end-to-end step */
+    cudaStream_t stream3 = nullptr; /* velocity upload of an end-to-end step; the density pass's dispersed ranges */
+    cudaEvent_t ev_walk = nullptr, ev_walk_done = nullptr;
+    bool dispersed = false; /* those ranges are many: a kernel of their own (check_list_cap) */
+    uint64_t checked_at = 0; /* step of the last check */
     cudaEvent_t ev_io_fork = nullptr, ev_vel_in = nullptr, ev_pos_in = nullptr;
     void enqueue_rb_grid(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches);
     void enqueue_rb_contact(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches, bool with_fluid);
@@ -212,6 +215,7 @@ struct World {
     unsigned long long *overflow_counter = nullptr; /* list overflows since the last reset */
     uint32_t *max_count = nullptr; /* largest list count since the last capacity check */
     bool list_autogrow = true;     /* grow the list capacity to the largest count seen */
+    bool list_check_due(uint64_t s) const;
     int check_list_cap();
     int current_kernel() const { return use_cc ? 2 : (use_list ? 1 : 0); }
     void set_kernel(int k)

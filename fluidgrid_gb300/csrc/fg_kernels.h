@@ -9,6 +9,12 @@
 
 namespace fg {
 
+/* A second stream for a pass of two kernels that run beside each other. */
+struct SideStream {
+    cudaStream_t stream;
+    cudaEvent_t fork, join;
+};
+
 /* Launch geometry: work items of FG_CHUNK particles; grids are sized in
  * multiples of the SM count (persistent grid-stride loops). */
 struct Launch {
@@ -20,6 +26,7 @@ struct Launch {
     cudaStream_t stream;
     uint32_t ctas_per_sm;  /* density/force grids: CTAs of FG_CHUNK threads per SM (0 = 64) */
     uint32_t block;        /* density/force grids: threads per CTA, 64, 128 or 256 (0 = FG_CHUNK) */
+    SideStream side;       /* the staged passes' dispersed ranges go to kernels of their own beside them, or {} */
 };
 
 int sm_count();
@@ -135,8 +142,14 @@ struct NbrList {
     const uint32_t *cap;          /* device word: entries a target may store (<= stride) */
     uint32_t *max_count;          /* optional: atomicMax of cnt */
     unsigned long long *overflow; /* optional: targets with cnt > cap */
+    uint32_t *dispersed;          /* += an eighth of the dispersed ranges of 32 */
 };
 
+/* whether a density pass over nwork items takes ranges of 32 targets, whose
+ * dispersed ones can go to a kernel of their own */
+bool density_ranges_wide(uint32_t nwork);
+/* kernel launches of a launch_density */
+uint32_t density_launches(const Launch &L);
 void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, const uint32_t *end, float2 *dp,
                     float gas_override, float rest_override, float mass_override, int use_override,
                     const float4 *svel = nullptr, const NbrList *list = nullptr,

@@ -117,22 +117,113 @@ struct ListRing {
 };
 static_assert(FG_DENSITY_THREADS == 64u, "a ring entry is a word of each of 64 threads");
 
+/* Replacements for the scene's constants (the launchers'). */
+struct DensityConst {
+    float gas, rest, mass;
+    int use;
+};
+
+/* A thread's counts over its targets. */
+struct DensityTally {
+    unsigned long long pairs = 0; /* in-range visits, the target itself included */
+    uint32_t most = 0;            /* largest list count */
+    uint32_t overflow = 0;        /* targets with more entries than slots */
+
+    template <bool LIST>
+    __device__ __forceinline__ void add(uint32_t cnt, uint32_t cap)
+    {
+        pairs += cnt;
+        most = max(most, cnt);
+        overflow += (LIST && cnt > cap) ? 1u : 0u;
+    }
+    /* once per warp: in-range pair visits for reporting, and the largest list
+     * count for the capacity check */
+    template <bool LIST, bool COUNT>
+    __device__ __forceinline__ void flush(const NbrList &list, unsigned long long *out)
+    {
+        const uint32_t lane = threadIdx.x & 31u;
+        if (COUNT && out) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) pairs += __shfl_xor_sync(FG_FULL, pairs, o);
+            if (lane == 0 && pairs) atomicAdd(out, pairs);
+        }
+        if (LIST && list.max_count) {
+            most = __reduce_max_sync(FG_FULL, most);
+            if (lane == 0 && most) atomicMax(list.max_count, most);
+        }
+        if (LIST && list.overflow) {
+            overflow = __reduce_add_sync(FG_FULL, overflow);
+            if (lane == 0 && overflow) atomicAdd(list.overflow, (unsigned long long)overflow);
+        }
+    }
+};
+
+/* Density, pressure, record and list count of sorted target i at p. */
+template <bool LIST>
+__device__ __forceinline__ void density_store(const DensityAcc &acc, const FgScene *S, uint32_t i, float4 p,
+                                              bool active, const float4 *__restrict__ svel, float2 *__restrict__ dp,
+                                              const DensityConst &C, const NbrList &list)
+{
+    float2 d = make_float2(0.f, 0.f);
+    if (active) {
+        d = fg_density_out(C.use ? C.mass : S->mass, S->kpoly6, C.use ? C.gas : S->gas, C.use ? C.rest : S->rest,
+                           acc.sum());
+        dp[i] = d;
+    } else if (LIST) {
+        d = dp[i]; /* inactive particles stay neighbours with their stale density */
+    }
+    if (LIST) {
+        const float4 v = __ldg(svel + i);
+        list.rec[2 * i] = make_float4(p.x, p.y, p.z, d.x);
+        list.rec[2 * i + 1] = make_float4(v.x, v.y, v.z, d.y);
+        list.cnt[i] = acc.cnt;
+    }
+}
+
+/* The density sum and list of sorted target i by a walk, and its visits. */
+template <bool LIST, bool COUNT>
+__device__ __forceinline__ void density_walk(DensityAcc &acc, const FgScene *S, uint32_t i, float4 p,
+                                             const float4 *__restrict__ spos, const uint32_t *__restrict__ start,
+                                             const uint32_t *__restrict__ end, uint32_t *lp, uint32_t cap)
+{
+    const float scale = S->scale, h2 = S->h2;
+    const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
+    fg_walk27_rows(p.x, p.y, p.z, S, start, end, [&](uint32_t j) {
+        acc.visit<LIST, COUNT>(__ldg(spos + j), j, px, py, pz, scale, h2, lp, cap);
+    });
+    if (LIST) acc.flush(lp, cap, i);
+}
+
+/* The same out of line, for the staging kernel: inlined, it cost the staging 4%. */
+template <bool LIST, bool COUNT>
+__device__ __noinline__ uint2 density_walk_aside(const FgScene *S, uint32_t i, const float4 *spos,
+                                                 const uint32_t *start, const uint32_t *end, uint32_t *lp,
+                                                 uint32_t cap)
+{
+    DensityAcc acc;
+    acc.init();
+    density_walk<LIST, COUNT>(acc, S, i, __ldg(spos + i), spos, start, end, lp, cap);
+    return make_uint2(__float_as_uint(acc.sum()), acc.cnt);
+}
+
+/* What a pass does with its dispersed ranges: those of more than `most`
+ * buckets, whose targets share too little for a lookup and a cull a cell. */
+enum { DISPERSED_STAGED, DISPERSED_WALKED, DISPERSED_ASIDE /* another kernel has them */ };
+
 template <bool LIST, bool COUNT>
 __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density(
     const FgWork *__restrict__ work, uint32_t nwork, uint32_t n_single, const FgScene *__restrict__ table,
-    const __grid_constant__ FgScene single, uint32_t range, const float4 *__restrict__ spos,
-    const float4 *__restrict__ svel, const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
-    float2 *__restrict__ dp, float gas_o, float rest_o, float mass_o, int use_o, const __grid_constant__ NbrList list,
-    unsigned long long *__restrict__ pairs)
+    const __grid_constant__ FgScene single, uint32_t range, uint32_t most, int dispersed,
+    const float4 *__restrict__ spos, const float4 *__restrict__ svel, const uint32_t *__restrict__ start,
+    const uint32_t *__restrict__ end, float2 *__restrict__ dp, const __grid_constant__ DensityConst C,
+    const __grid_constant__ NbrList list, unsigned long long *__restrict__ pairs)
 {
     __shared__ DensityShared shared[FG_DENSITY_THREADS / 32];
     __shared__ uint32_t s_ring[LIST ? 16 * FG_DENSITY_THREADS : 1];
     DensityShared &sm = shared[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t cap = LIST ? __ldg(list.cap) : 0u;
-    unsigned long long pc = 0; /* in-range density visits of this thread */
-    uint32_t mx = 0;           /* largest list count of this thread */
-    uint32_t ovf = 0;          /* targets of this thread with more entries than slots */
+    DensityTally tally;
     const uint32_t per = FG_CHUNK / range; /* warps per work item */
     for (uint32_t warp = blockIdx.x * (FG_DENSITY_THREADS / 32u) + (threadIdx.x >> 5); warp < nwork * per;
          warp += gridDim.x * (FG_DENSITY_THREADS / 32u)) {
@@ -142,116 +233,137 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
         const FgScene *S = fg_scene(table, &single, it.scene);
         const uint32_t lo = table ? S->pbase : 0u, hi = table ? S->pbase + S->n : n_single;
         const float scale = S->scale, h2 = S->h2;
-        uint32_t next, stop;
         const StageGrid G(S);
-        fg_stage_range(it.first + q0, range, lo, hi, G, spos, next, stop);
+        uint32_t next, stop;
+        bool walk = fg_stage_range(it.first + q0, range, lo, hi, most, dispersed == DISPERSED_ASIDE, G, spos, next,
+                                   stop);
+        if (walk) {
+            /* an eighth of them, for the host */
+            if (LIST && list.dispersed && lane == 0u && (warp & 7u) == 0u) atomicAdd(list.dispersed, 1u);
+            if (dispersed == DISPERSED_ASIDE) continue;
+            walk = dispersed == DISPERSED_WALKED;
+        }
         while (next < stop) {
-        const uint32_t i = next + lane; /* sorted index */
-        uint32_t n = min(32u, stop - next);
-        float4 p = lane < n ? spos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const StageSig sig = fg_stage_sig(p, G);
-        if (stop - next > 32u) n = fg_stage_trim(sig, __ldg(spos + next + 32u), G);
-        next += n;
-        const bool valid = lane < n;
-        const bool active = valid && p.w > 0.0f; /* inactive: density not written */
-        const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
-        DensityAcc acc;
-        acc.init();
-        ListRing ring(s_ring);
-        uint32_t count = 0u; /* without a list */
-        /* lists by sorted index: the force pass may visit the targets in another order */
-        uint32_t *lp = LIST ? list.idx + (size_t)i * list.stride : nullptr;
-        uint32_t lead, leads;
-        if (!__any_sync(FG_FULL, active && sig.odd)) {
-            fg_stage_groups(sig, __ballot_sync(FG_FULL, active), lead, leads);
-            while (leads) {
-                /* the first FG_STAGE_GROUPS of the groups left */
-                uint32_t later = leads;
-                for (uint32_t k = 0u; k < FG_STAGE_GROUPS; k++) later &= later - 1u;
-                const uint32_t batch = leads ^ later;
-                leads = later;
-                fg_stage_rounds<FG_DENSITY_STAGE>(
-                    sig, lead, batch, px, py, pz, G, spos, start, end, sm.idx,
-                    [&](uint32_t slot, uint32_t j, float4 c) {
-                        ((float *)sm.x)[slot] = c.x;
-                        ((float *)sm.y)[slot] = c.y;
-                        ((float *)sm.z)[slot] = c.z;
-                        ((uint32_t *)sm.j)[slot] = j;
-                    },
-                    [&](uint32_t first, uint32_t stop, uint32_t) {
-                        const F2 px2 = fg_pack(px, px), py2 = fg_pack(py, py), pz2 = fg_pack(pz, pz);
-                        const F2 ns2 = fg_pack(-scale, -scale), hh2 = fg_pack(h2, h2);
-                        for (uint32_t k = first >> 2; k < stop >> 2; k += 2u) {
+            const uint32_t i = next + lane; /* sorted index */
+            uint32_t n = min(32u, stop - next);
+            float4 p = lane < n ? spos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const StageSig sig = fg_stage_sig(p, G);
+            if (stop - next > 32u) n = fg_stage_trim(sig, __ldg(spos + next + 32u), G);
+            next += n;
+            const bool valid = lane < n;
+            const bool active = valid && p.w > 0.0f; /* inactive: density not written */
+            const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
+            DensityAcc acc;
+            acc.init();
+            ListRing ring(s_ring);
+            uint32_t count = 0u; /* without a list */
+            /* lists by sorted index: the force pass may visit the targets in another order */
+            uint32_t *lp = LIST ? list.idx + (size_t)i * list.stride : nullptr;
+            uint32_t lead, leads;
+            if (!walk && !__any_sync(FG_FULL, active && sig.odd)) {
+                fg_stage_groups(sig, __ballot_sync(FG_FULL, active), lead, leads);
+                while (leads) {
+                    /* the first FG_STAGE_GROUPS of the groups left */
+                    uint32_t later = leads;
+                    for (uint32_t k = 0u; k < FG_STAGE_GROUPS; k++) later &= later - 1u;
+                    const uint32_t batch = leads ^ later;
+                    leads = later;
+                    fg_stage_rounds<FG_DENSITY_STAGE>(
+                        sig, lead, batch, px, py, pz, G, spos, start, end, sm.idx,
+                        [&](uint32_t slot, uint32_t j, float4 c) {
+                            ((float *)sm.x)[slot] = c.x;
+                            ((float *)sm.y)[slot] = c.y;
+                            ((float *)sm.z)[slot] = c.z;
+                            ((uint32_t *)sm.j)[slot] = j;
+                        },
+                        [&](uint32_t first, uint32_t stop, uint32_t) {
+                            const F2 px2 = fg_pack(px, px), py2 = fg_pack(py, py), pz2 = fg_pack(pz, pz);
+                            const F2 ns2 = fg_pack(-scale, -scale), hh2 = fg_pack(h2, h2);
+                            for (uint32_t k = first >> 2; k < stop >> 2; k += 2u) {
 #pragma unroll
-                            for (uint32_t e = 0; e < 2u; e++) {
-                                const float4 x = sm.x[k + e], y = sm.y[k + e], z = sm.z[k + e];
-                                const uint4 j = LIST ? sm.j[k + e] : make_uint4(0u, 0u, 0u, 0u);
-                                bool in[4];
-                                acc.term2(fg_pack(x.x, x.y), fg_pack(y.x, y.y), fg_pack(z.x, z.y), px2, py2, pz2, ns2,
-                                          hh2, h2, in[0], in[1]);
-                                acc.term2(fg_pack(x.z, x.w), fg_pack(y.z, y.w), fg_pack(z.z, z.w), px2, py2, pz2, ns2,
-                                          hh2, h2, in[2], in[3]);
-                                if (LIST) {
-                                    ring.push(j.x, in[0]);
-                                    ring.push(j.y, in[1]);
-                                    ring.push(j.z, in[2]);
-                                    ring.push(j.w, in[3]);
-                                } else if (COUNT) {
+                                for (uint32_t e = 0; e < 2u; e++) {
+                                    const float4 x = sm.x[k + e], y = sm.y[k + e], z = sm.z[k + e];
+                                    const uint4 j = LIST ? sm.j[k + e] : make_uint4(0u, 0u, 0u, 0u);
+                                    bool in[4];
+                                    acc.term2(fg_pack(x.x, x.y), fg_pack(y.x, y.y), fg_pack(z.x, z.y), px2, py2, pz2,
+                                              ns2, hh2, h2, in[0], in[1]);
+                                    acc.term2(fg_pack(x.z, x.w), fg_pack(y.z, y.w), fg_pack(z.z, z.w), px2, py2, pz2,
+                                              ns2, hh2, h2, in[2], in[3]);
+                                    if (LIST) {
+                                        ring.push(j.x, in[0]);
+                                        ring.push(j.y, in[1]);
+                                        ring.push(j.z, in[2]);
+                                        ring.push(j.w, in[3]);
+                                    } else if (COUNT) {
 #pragma unroll
-                                    for (int u = 0; u < 4; u++) count += in[u] ? 1u : 0u;
+                                        for (int u = 0; u < 4; u++) count += in[u] ? 1u : 0u;
+                                    }
                                 }
+                                if (LIST) ring.spill(lp, cap);
                             }
-                            if (LIST) ring.spill(lp, cap);
-                        }
-                    });
+                        });
+                }
+                if (LIST && active) ring.finish(lp, cap, i);
+                acc.cnt = LIST ? ring.count() : count;
+            } else if (active) {
+                const uint2 r = density_walk_aside<LIST, COUNT>(S, i, spos, start, end, lp, cap);
+                acc.s = __uint_as_float(r.x);
+                acc.cnt = r.y;
             }
-            if (LIST && active) ring.finish(lp, cap, i);
-            acc.cnt = LIST ? ring.count() : count;
-        } else if (active) {
-            fg_walk27(
-                p.x, p.y, p.z, S, start, end,
-                [&](uint32_t j) { acc.visit<LIST, COUNT>(__ldg(spos + j), j, px, py, pz, scale, h2, lp, cap); });
-            if (LIST) acc.flush(lp, cap, i);
-        }
-        if (active) {
-            const float mass = use_o ? mass_o : S->mass;
-            const float gas = use_o ? gas_o : S->gas;
-            const float rest = use_o ? rest_o : S->rest;
-            const float2 d = fg_density_out(mass, S->kpoly6, gas, rest, acc.sum());
-            dp[i] = d;
-            if (LIST) {
-                const float4 v = __ldg(svel + i);
-                list.rec[2 * i] = make_float4(p.x, p.y, p.z, d.x);
-                list.rec[2 * i + 1] = make_float4(v.x, v.y, v.z, d.y);
-            }
-        } else if (LIST && valid) {
-            /* inactive particles stay neighbours with their stale density */
-            const float2 d = dp[i];
-            const float4 v = __ldg(svel + i);
-            list.rec[2 * i] = make_float4(p.x, p.y, p.z, d.x);
-            list.rec[2 * i + 1] = make_float4(v.x, v.y, v.z, d.y);
-        }
-        if (LIST && valid) list.cnt[i] = acc.cnt;
-        pc += acc.cnt;
-        mx = max(mx, acc.cnt);
-        ovf += (LIST && acc.cnt > cap) ? 1u : 0u;
+            if (valid) density_store<LIST>(acc, S, i, p, active, svel, dp, C, list);
+            tally.add<LIST>(acc.cnt, cap);
         }
     }
-    /* once per warp: in-range pair visits (self included) for reporting, and
-     * the largest list count for the capacity check */
-    if (COUNT && pairs) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) pc += __shfl_xor_sync(0xffffffffu, pc, o);
-        if (lane == 0 && pc) atomicAdd(pairs, pc);
+    tally.flush<LIST, COUNT>(list, pairs);
+}
+
+/* The dispersed ranges, a thread a target.  Bound by the L1's and L2's sectors
+ * (54 bucket words a target) and their latency, for which it wants the L1 and
+ * the warps that the staging kernel's shared memory takes: the same walk there
+ * takes 270 us where this takes 226, at 1,048,576 targets 1.2 h apart (staged:
+ * 477).  Eight CTAs an SM, 62 registers, without lists (sixteen of 32, which
+ * spill: 262 us), ten with them.  A wave of CTAs; the next range's positions
+ * are on their way while one walks or is passed over. */
+#define FG_WALK_CTAS(LIST) ((LIST) ? 10 : 8)
+template <bool LIST, bool COUNT>
+__global__ void __launch_bounds__(FG_CHUNK, FG_WALK_CTAS(LIST)) k_density_dispersed(
+    const FgWork *__restrict__ work, uint32_t nwork, uint32_t n_single, const FgScene *__restrict__ table,
+    const __grid_constant__ FgScene single, uint32_t most, const float4 *__restrict__ spos,
+    const float4 *__restrict__ svel, const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+    float2 *__restrict__ dp, const __grid_constant__ DensityConst C, const __grid_constant__ NbrList list,
+    unsigned long long *__restrict__ pairs)
+{
+    const uint32_t cap = LIST ? __ldg(list.cap) : 0u;
+    DensityTally tally;
+    auto load = [&](uint32_t w) {
+        const FgWork it = fg_work(work, w, n_single);
+        const FgScene *S = fg_scene(table, &single, it.scene);
+        return __ldg(spos + min(it.first + threadIdx.x, (table ? S->pbase + S->n : n_single) - 1u));
+    };
+    uint32_t w = blockIdx.x;
+    float4 ahead = w < nwork ? load(w) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (; w < nwork; w += gridDim.x) {
+        const FgWork it = fg_work(work, w, n_single);
+        const FgScene *S = fg_scene(table, &single, it.scene);
+        const float4 p = ahead;
+        if (w + gridDim.x < nwork) ahead = load(w + gridDim.x);
+        if ((threadIdx.x & ~31u) >= it.count) continue; /* uniform over the warp */
+        const StageGrid G(S);
+        if (!fg_stage_dispersed(fg_stage_cell(p, G), G, 32u, most)) continue;
+        if (threadIdx.x < it.count) {
+            const uint32_t i = it.first + threadIdx.x;
+            const bool active = p.w > 0.0f;
+            DensityAcc acc;
+            acc.init();
+            if (active)
+                density_walk<LIST, COUNT>(acc, S, i, p, spos, start, end,
+                                          LIST ? list.idx + (size_t)i * list.stride : nullptr, cap);
+            density_store<LIST>(acc, S, i, LIST ? __ldg(spos + i) : p, active, svel, dp, C, list);
+            tally.add<LIST>(acc.cnt, cap);
+        }
+        __syncwarp();
     }
-    if (LIST && list.max_count) {
-        mx = __reduce_max_sync(0xffffffffu, mx);
-        if (lane == 0 && mx) atomicMax(list.max_count, mx);
-    }
-    if (LIST && list.overflow) {
-        ovf = __reduce_add_sync(0xffffffffu, ovf);
-        if (lane == 0 && ovf) atomicAdd(list.overflow, (unsigned long long)ovf);
-    }
+    tally.flush<LIST, COUNT>(list, pairs);
 }
 
 /* Targets of a warp: 32, or fewer where that leaves the SMs short of warps
@@ -265,6 +377,50 @@ static uint32_t stage_range(uint32_t nwork)
     return range;
 }
 
+/* What becomes of a pass's dispersed ranges, and beyond how many buckets a
+ * range is one (32: none is).  Density without lists, 1,048,576 random targets,
+ * staged -> walked: 0.5 h apart (four or five cells a range) 312 -> 315 us, 0.8
+ * h (14) 362 -> 235, 1.2 h 477 -> 226, 3 h 543 -> 241; 262,144, 1.7 h: 147 ->
+ * 67.  Nine parts the first two: with eight, the few ranges of the first that
+ * walk take it to 326; with twelve, the second stays at 326.  With L.side the
+ * walk is a kernel beside the staging one (3 us where no range walks); warps
+ * of fewer targets, of which the GPU is not full, walk themselves. */
+static int dispersed_ranges(const Launch &L, uint32_t range, bool count, uint32_t &most)
+{
+    most = range == 32u ? 9u : range - range / 4u;
+    if (!L.side.stream) {
+        if (!count || range < 32u) most = 32u;
+        return DISPERSED_STAGED;
+    }
+    return range == 32u ? DISPERSED_ASIDE : DISPERSED_WALKED;
+}
+
+bool density_ranges_wide(uint32_t nwork) { return stage_range(nwork) == 32u; }
+
+uint32_t density_launches(const Launch &L)
+{
+    uint32_t most;
+    return dispersed_ranges(L, stage_range(L.nwork), false, most) == DISPERSED_ASIDE ? 2u : 1u;
+}
+
+/* L.side's stream, if it is used: forked from L's until the end of the scope. */
+struct SideLaunch {
+    const Launch &L;
+    const bool use;
+    SideLaunch(const Launch &launch, bool fork) : L(launch), use(fork)
+    {
+        if (!use) return;
+        cudaEventRecord(L.side.fork, L.stream);
+        cudaStreamWaitEvent(L.side.stream, L.side.fork, 0);
+    }
+    ~SideLaunch()
+    {
+        if (!use) return;
+        cudaEventRecord(L.side.join, L.side.stream);
+        cudaStreamWaitEvent(L.stream, L.side.join, 0);
+    }
+};
+
 void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, const uint32_t *end, float2 *dp,
                     float gas_o, float rest_o, float mass_o, int use_o, const float4 *svel, const NbrList *list,
                     unsigned long long *pairs)
@@ -273,14 +429,23 @@ void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, 
     NbrList none;
     memset(&none, 0, sizeof(none));
     const NbrList &nl = list ? *list : none;
+    const DensityConst C = {gas_o, rest_o, mass_o, use_o};
     const uint32_t range = stage_range(L.nwork);
+    uint32_t most;
+    const int dispersed = dispersed_ranges(L, range, nl.dispersed != nullptr, most);
     /* ctas_per_sm counts CTAs of FG_CHUNK threads for 32 targets a warp */
     const uint32_t per = FG_CHUNK / range * 32u / FG_DENSITY_THREADS;
     const uint32_t g = grid_for(L.nwork * per, (int)((L.ctas_per_sm ? L.ctas_per_sm : 64u) * per));
-#define FG_DENSITY(LI, CO)                                                                                         \
-    k_density<LI, CO><<<g, FG_DENSITY_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, range, spos, \
-                                                              svel, start, end, dp, gas_o, rest_o, mass_o, use_o,  \
-                                                              nl, pairs)
+#define FG_DENSITY(LI, CO)                                                                                          \
+    do {                                                                                                            \
+        const SideLaunch side(L, dispersed == DISPERSED_ASIDE);                                                     \
+        if (side.use)                                                                                               \
+            k_density_dispersed<LI, CO><<<grid_for(L.nwork, FG_WALK_CTAS(LI)), FG_CHUNK, 0, L.side.stream>>>(            \
+                L.work, L.nwork, L.n, L.table, *L.single, most, spos, svel, start, end, dp, C, nl, pairs);          \
+        k_density<LI, CO><<<g, FG_DENSITY_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, range,  \
+                                                                  most, dispersed, spos, svel, start, end, dp, C,   \
+                                                                  nl, pairs);                                       \
+    } while (0)
     if (list) FG_DENSITY(true, true);
     else if (pairs) FG_DENSITY(false, true);
     else FG_DENSITY(false, false);
@@ -570,7 +735,7 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
     for (uint32_t b0 = (blockIdx.x * (FG_FORCE_THREADS / 32u) + (threadIdx.x >> 5)) * range; b0 < n_all;
          b0 += gridDim.x * (FG_FORCE_THREADS / 32u) * range) {
         uint32_t next, stop;
-        fg_stage_range(b0, range, 0u, n_all, G, spos, next, stop);
+        fg_stage_range(b0, range, 0u, n_all, 32u, false, G, spos, next, stop);
         while (next < stop) {
             const uint32_t i0 = next, i = next + lane; /* sorted index */
             uint32_t n = min(32u, stop - next);

@@ -54,6 +54,49 @@ __device__ __forceinline__ void fg_walk27(float px, float py, float pz, const Fg
     fg_walk27(px, py, pz, S, start, end, fn, [] {});
 }
 
+/* The same walk with a row's three buckets as one run of candidates and the
+ * next row's ranges on their way meanwhile: lanes whose buckets hold a few
+ * particles each wait for the longest of 9 runs, not of 27. */
+template <typename Fn>
+__device__ __forceinline__ void fg_walk27_rows(float px, float py, float pz, const FgScene *S,
+                                               const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
+                                               Fn &&fn)
+{
+    uint32_t hx[3], hy[3], hz[3];
+    fg_neighbour_hashes(px, py, pz, S->cell, hx, hy, hz);
+    const uint32_t hx0 = hx[0], hx1 = hx[1], hx2 = hx[2], hy0 = hy[0], hy1 = hy[1], hy2 = hy[2];
+    const uint32_t hz0 = hz[0], hz1 = hz[1], hz2 = hz[2];
+    const uint32_t nb = S->nb, mask = S->nb_mask, bb = S->bucket_base;
+    uint32_t s[3], e[3];
+    auto row = [&](int r) {
+        const uint32_t yh = fg_sel3(hy0, hy1, hy2, r % 3), zh = fg_sel3(hz0, hz1, hz2, r / 3);
+        const uint32_t b0 = bb + fg_bucket(hx0, yh, zh, nb, mask);
+        const uint32_t b1 = bb + fg_bucket(hx1, yh, zh, nb, mask);
+        const uint32_t b2 = bb + fg_bucket(hx2, yh, zh, nb, mask);
+        s[0] = __ldg(start + b0);
+        s[1] = __ldg(start + b1);
+        s[2] = __ldg(start + b2);
+        e[0] = __ldg(end + b0);
+        e[1] = __ldg(end + b1);
+        e[2] = __ldg(end + b2);
+    };
+    row(0);
+#pragma unroll 1
+    for (int r = 0; r < 9; r++) {
+        uint32_t st[3], c[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+            st[x] = s[x];
+            c[x] = s[x] != FG_EMPTY && e[x] > s[x] ? e[x] - s[x] : 0u; /* end of an empty bucket is stale */
+        }
+        if (r < 8) row(r + 1);
+        const uint32_t c01 = c[0] + c[1], all = c01 + c[2];
+        const uint32_t o1 = st[1] - c[0], o2 = st[2] - c01;
+#pragma unroll 2
+        for (uint32_t k = 0; k < all; k++) fn(k + (k < c[0] ? st[0] : (k < c01 ? o1 : o2)));
+    }
+}
+
 /* Two floats in a register pair, an instruction for both. */
 typedef unsigned long long F2;
 __device__ __forceinline__ F2 fg_pack(float a, float b)
@@ -108,18 +151,9 @@ struct DensityAcc {
         s = u;
     }
 
-    /* add a candidate's (h^2 - l^2)^3, 0 beyond h; whether it is in range */
-    __device__ __forceinline__ bool term(float4 q, float px, float py, float pz, float scale, float h2)
-    {
-        const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
-        const float t = fmaxf(__fsub_rn(h2, r2), 0.0f); /* 0 for a NaN too */
-        add(__fmul_rn(__fmul_rn(t, t), t));
-        return r2 <= h2;
-    }
-
-    /* term() for two candidates, first and second of the pairs: the same
-     * operations, all but the sums two to an instruction */
+    /* add two candidates' (h^2 - l^2)^3, 0 beyond h and for a NaN, and whether
+     * each is in range: visit()'s operations, all but the sums two to an
+     * instruction */
     __device__ __forceinline__ void term2(F2 x, F2 y, F2 z, F2 px, F2 py, F2 pz, F2 nscale, F2 h2, float h2s, bool &in0,
                                           bool &in1)
     {
@@ -140,7 +174,11 @@ struct DensityAcc {
     __device__ __forceinline__ void visit(float4 q, uint32_t j, float px, float py, float pz, float scale, float h2,
                                           uint32_t *lp, uint32_t cap)
     {
-        if (term(q, px, py, pz, scale, h2)) {
+        const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
+        if (r2 <= h2) {
+            const float t = __fsub_rn(h2, r2);
+            add(__fmul_rn(__fmul_rn(t, t), t));
             if (COUNT) cnt++;
             if (LIST) {
                 q2 = q3;

@@ -109,48 +109,69 @@ __device__ __forceinline__ float fg_redux_max(float v)
 #define FG_STAGE_FLIGHT 4u /* chunks of 32 candidates whose loads are in flight together */
 #endif
 
+struct StageCell {
+    int x, y, z;
+    bool active;
+};
+__device__ __forceinline__ StageCell fg_stage_cell(float4 p, const StageGrid &G)
+{
+    StageCell c = {fg_axis_index(p.x, G.cell[0]), fg_axis_index(p.y, G.cell[1]), fg_axis_index(p.z, G.cell[2]),
+                   p.w > 0.0f};
+    return c;
+}
+
+/* Whether the targets of a range, a lane each (past the scene's end its last
+ * one's), are more than `most` and lie in more buckets: a function of the range
+ * alone, so that two kernels that share the ranges agree on it.  (Buckets, not
+ * cells: where many cells share a bucket, the candidates are many too.) */
+__device__ __forceinline__ bool fg_stage_dispersed(const StageCell &c, const StageGrid &G, uint32_t len, uint32_t most)
+{
+    const uint32_t b = fg_bucket((uint32_t)c.x * FG_PX, (uint32_t)c.y * FG_PY, (uint32_t)c.z * FG_PZ, G.nb, G.mask);
+    const uint32_t lane = threadIdx.x & 31u, before = __shfl_up_sync(FG_FULL, b, 1);
+    return (uint32_t)__popc(__ballot_sync(FG_FULL, lane < len && (lane == 0u || b != before))) > most &&
+           (uint32_t)__popc(__ballot_sync(FG_FULL, lane < len && c.active)) > most;
+}
+
 /* The targets [first, stop) of the warp whose nominal range is [b, b + len) of
  * a scene's [lo, hi), len <= 32: a cell that straddles two ranges goes to the
- * first one's warp as a whole, unless it fills a range.  A cut cell would be
- * staged twice, and cells are two to four to a warp. */
-__device__ __forceinline__ void fg_stage_range(uint32_t b, uint32_t len, uint32_t lo, uint32_t hi, const StageGrid &G,
-                                               const float4 *__restrict__ spos, uint32_t &first, uint32_t &stop)
+ * first one's warp as a whole, unless it fills a range.  (A cut cell would be
+ * staged twice, and cells are two to four to a warp.)  Returns whether the
+ * range is dispersed; with `apart` such ranges, which are not staged, stay as
+ * they are. */
+__device__ __forceinline__ bool fg_stage_range(uint32_t b, uint32_t len, uint32_t lo, uint32_t hi, uint32_t most,
+                                               bool apart, const StageGrid &G, const float4 *__restrict__ spos,
+                                               uint32_t &first, uint32_t &stop)
 {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t own = min(len, hi - b);
-    struct Cell {
-        int x, y, z;
-    };
-    auto cell = [&](uint32_t i) {
-        const float4 p = __ldg(spos + min(i, hi - 1u));
-        Cell c = {fg_axis_index(p.x, G.cell[0]), fg_axis_index(p.y, G.cell[1]), fg_axis_index(p.z, G.cell[2])};
-        return c;
-    };
-    auto pick = [&](const Cell &c, uint32_t l) {
-        Cell r = {__shfl_sync(FG_FULL, c.x, (int)l), __shfl_sync(FG_FULL, c.y, (int)l),
-                  __shfl_sync(FG_FULL, c.z, (int)l)};
+    auto cell = [&](uint32_t i) { return fg_stage_cell(__ldg(spos + min(i, hi - 1u)), G); };
+    auto pick = [&](const StageCell &c, uint32_t l) {
+        StageCell r = {__shfl_sync(FG_FULL, c.x, (int)l), __shfl_sync(FG_FULL, c.y, (int)l),
+                       __shfl_sync(FG_FULL, c.z, (int)l), true};
         return r;
     };
-    auto same = [](const Cell &a, const Cell &c) { return a.x == c.x && a.y == c.y && a.z == c.z; };
+    auto same = [](const StageCell &a, const StageCell &c) { return a.x == c.x && a.y == c.y && a.z == c.z; };
     /* how many targets of a range begin by continuing the cell of the target before it */
-    auto leading = [&](const Cell &before, const Cell &mine, uint32_t n) {
-        return (uint32_t)__ffs((int)~(__ballot_sync(FG_FULL, lane < n && same(before, mine)))) - 1u; /* ~0: 32 by wrap */
+    auto leading = [&](const StageCell &before, const StageCell &mine, uint32_t n) {
+        return (uint32_t)__ffs((int)~(__ballot_sync(FG_FULL, lane < n && same(before, mine)))) - 1u; /* all 32: wraps */
     };
-    const Cell mine = cell(b + lane);
+    const StageCell mine = cell(b + lane);
     first = b;
     stop = b + own;
+    const bool dispersed = most < 32u && fg_stage_dispersed(mine, G, len, most);
+    if (dispersed && apart) return true;
     if (b > lo) {
-        /* lane 0: the target before; lane 1: the first of the range before */
-        const Cell e = cell(lane == 0u ? b - 1u : b - len);
-        const Cell before = pick(e, 0u), head = pick(e, 1u);
+        const StageCell e = cell(b - len + lane);
+        const StageCell before = pick(e, len - 1u), head = pick(e, 0u);
         const uint32_t m = leading(before, mine, own);
-        if (m < len && !same(before, head)) first += m;
+        if (m < len && !same(before, head) && !(apart && fg_stage_dispersed(e, G, len, most))) first += m;
     }
     if (b + len < hi) {
-        const Cell last = pick(mine, len - 1u), head = pick(mine, 0u);
-        const uint32_t m = leading(last, cell(b + len + lane), min(len, hi - b - len));
-        if (m < len && !same(last, head)) stop += m;
+        const StageCell last = pick(mine, len - 1u), head = pick(mine, 0u), after = cell(b + len + lane);
+        const uint32_t m = leading(last, after, min(len, hi - b - len));
+        if (m < len && !same(last, head) && !(apart && fg_stage_dispersed(after, G, len, most))) stop += m;
     }
+    return dispersed;
 }
 
 /* Of 32 targets, those before the last cell if the target after them, at

@@ -1,0 +1,129 @@
+"""Targets that share few cells (sprays, sparse clouds): the passes leave their
+ranges to a walk by thread.  The same density bits whichever kernel finds the
+candidates, in the launcher and in a world, and a sparse cloud no slower than a
+dense one."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from fluidgrid_gb300 import World, _ffi, build
+from fluidgrid_gb300.scenes import H, SceneSpec
+from oracle import oracle as O
+import helpers as T
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+WIDE = 77_953  # the fewest work items whose warps take 32 targets, and a remainder of one
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    build.build()
+
+
+def p(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def cloud(n, parts, seed, buckets=(1 << 18, 1, 1), active=1.0, cell=None):
+    """n particles in cubes side by side, each at its own mean distance (kernel radii)."""
+    rng = np.random.default_rng(seed)
+    pos, x = np.ones((n, 4), np.float32), 0.3
+    for part, spacing in zip(np.array_split(np.arange(n), len(parts)), parts):
+        side = spacing * H * len(part) ** (1.0 / 3.0)
+        pos[part, :3] = rng.uniform(0, side, (len(part), 3)) + (x, 0.3, 0.3)
+        x += side + 0.2
+    pos[rng.uniform(size=n) > active, 3] = 0.0
+    vel = np.zeros((n, 4), np.float32)
+    vel[:, :3] = rng.normal(0, 0.1, (n, 3))
+    return SceneSpec(pos=rng.permutation(pos), vel=vel, box_min=(-1,) * 3, box_max=(x + 9, 30, 30), buckets=buckets,
+                     cell=cell)
+
+
+SCENES = {
+    "mixed": cloud(WIDE, (0.5, 1.7), 1), "spray": cloud(WIDE + 30, (1.7,), 2),
+    "near_the_line": cloud(WIDE + 127, (0.6, 0.7, 0.8), 3), "half_active": cloud(WIDE, (0.5, 1.2), 4, active=0.5),
+    "odd_table": cloud(WIDE + 1, (0.5, 1.2), 5, (61, 61, 61)), "few_buckets": cloud(WIDE, (1.2,), 6, (4099, 1, 1)),
+    "small": cloud(9001, (0.5, 1.7), 7), "tiny": cloud(61, (1.7,), 8),
+}
+
+
+def launcher_density(spec):
+    L = _ffi.load()
+    ref = T.oracle_grid(spec, spec.pos, spec.vel)
+    kc = O.kernels_cache(spec.h)
+    L.gInitializeCommonFluidParams(spec.common_params())
+    L.gInitializeKernelParams(_ffi.fgr_kernels_cache(kc.kPoly6, kc.kSpikyGradient, kc.kViscosityLaplacian))
+    opos, dp = dev(ref["spos"]), torch.zeros((spec.n, 2), device="cuda")
+    start, end, key = (dev(ref[k].view(np.int32)) for k in ("start", "end", "skeys"))
+    L.gCalcMassDensity(p(opos), p(dp), p(key), p(start), p(end), spec.n, spec.gas, spec.rest, spec.mass)
+    assert L.fgc_last_status() == 0
+    return dp.cpu().numpy(), ref, kc
+
+
+@pytest.mark.parametrize("name", list(SCENES))
+def test_density_bits_do_not_depend_on_the_kernel(name):
+    spec = SCENES[name]
+    dp, ref, kc = launcher_density(spec)
+    d64, _ = O.density(ref["spos"], ref["start"], ref["end"], ref["p"], kc, spec.gas, spec.rest, spec.mass, f64=True)
+    on = ref["spos"][:, 3] > 0
+    assert (np.abs(dp[on, 0] - d64[on, 0]) / d64[on, 0]).max() <= 1e-5
+    for kernel in (1, 0):
+        w = World([spec])
+        w.set_option("autotune_period", 0)
+        w.set_option("kernel", kernel)
+        w.step(1)
+        assert np.array_equal(w.read("DP").view(np.uint32)[on], dp.view(np.uint32)[on]), kernel
+        w.close()
+
+
+@pytest.mark.parametrize("names", [("spray",), ("mixed", "tiny", "half_active"), ("odd_table",)])
+def test_world_steps_with_and_without_the_walk(names):
+    specs = [SCENES[k] for k in names]
+    out = []
+    for check in (1, 0):  # without capacity checks no world learns that it is dispersed
+        w = World(specs)
+        w.set_option("autotune_period", 0)
+        w.set_option("list_autogrow", check)
+        first = w.launches_per_step()
+        w.step(4)
+        assert w.launches_per_step() == first + check
+        out.append(w.download() + (w.read("DP"), w.counters()))
+        w.close()
+    for a, b in zip(out[0][:3], out[1][:3]):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    assert out[0][3] == out[1][3]
+
+
+def milliseconds(fn):
+    best = 1e9
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(4):
+            fn()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+def test_a_sparse_cloud_is_no_slower_than_a_dense_one():
+    """Its density pass finds a hundredth of the neighbours (staged, it took 1.6
+    times as long; walked, 0.7)."""
+    L = _ffi.load()
+    t = {}
+    for spacing in (0.5, 3.0):
+        spec = cloud(262_144, (spacing,), 9, (1 << 19, 1, 1))
+        _, ref, _ = launcher_density(spec)
+        opos, dp = dev(ref["spos"]), torch.zeros((spec.n, 2), device="cuda")
+        start, end, key = (dev(ref[k].view(np.int32)) for k in ("start", "end", "skeys"))
+        t[spacing] = milliseconds(lambda: L.gCalcMassDensity(p(opos), p(dp), p(key), p(start), p(end), spec.n,
+                                                             spec.gas, spec.rest, spec.mass))
+    assert t[3.0] <= 1.1 * t[0.5]
