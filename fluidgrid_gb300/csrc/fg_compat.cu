@@ -284,7 +284,7 @@ void gSPHCalculateForces(float4 *orderedPositions, float4 *orderedVelocity, floa
     fg::ForceOut o;
     o.vel = vel;
     o.pos = nullptr;
-    fg::launch_forces(single_launch(&S, numParticles), orderedPositions, orderedVelocity, density_pressure, gridStart,
+    fg::launch_forces(staged_launch(&S, numParticles), orderedPositions, orderedVelocity, density_pressure, gridStart,
                       gridEnd, particleId, o, nullptr, nullptr, mass, viscosity, 1);
     finish();
 }
@@ -351,13 +351,13 @@ void gSPHCalculateForcesWithSRB(float4 *oldPositions, float4 *oldVelocity, float
     fg::ForceOut o;
     o.vel = newVel;
     o.pos = nullptr;
+    const fg::Launch L = staged_launch(&S, numParticles);
     std::lock_guard<std::mutex> lk(g_mu);
     int r = useDynamicRB ? mark_near(dyn, 0u, S) : FG_OK;
     if (r == FG_OK && useStaticRB) r = mark_near(sta, 1u, S);
     if (r != FG_OK) { g_status = r; return; }
-    fg::launch_forces(single_launch(&S, numParticles), oldPositions, oldVelocity, density_pressure, gridStart,
-                      gridEnd, particleId, o, useDynamicRB ? &dyn : nullptr, useStaticRB ? &sta : nullptr, mass,
-                      kViscosity, 1);
+    fg::launch_forces(L, oldPositions, oldVelocity, density_pressure, gridStart, gridEnd, particleId, o,
+                      useDynamicRB ? &dyn : nullptr, useStaticRB ? &sta : nullptr, mass, kViscosity, 1);
     finish();
 }
 

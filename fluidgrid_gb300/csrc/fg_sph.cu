@@ -440,7 +440,7 @@ void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, 
     do {                                                                                                            \
         const SideLaunch side(L, dispersed == DISPERSED_ASIDE);                                                     \
         if (side.use)                                                                                               \
-            k_density_dispersed<LI, CO><<<grid_for(L.nwork, FG_WALK_CTAS(LI)), FG_CHUNK, 0, L.side.stream>>>(            \
+            k_density_dispersed<LI, CO><<<grid_for(L.nwork, FG_WALK_CTAS(LI)), FG_CHUNK, 0, L.side.stream>>>(       \
                 L.work, L.nwork, L.n, L.table, *L.single, most, spos, svel, start, end, dp, C, nl, pairs);          \
         k_density<LI, CO><<<g, FG_DENSITY_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, range,  \
                                                                   most, dispersed, spos, svel, start, end, dp, C,   \
@@ -506,7 +506,7 @@ __device__ __forceinline__ void walk_terms(const FgScene *S, uint32_t i, float4 
     const float scale = S->scale, h = S->h, h2 = S->h2, kspiky = S->kspiky;
     const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
     const float2 di = dp[i];
-    fg_walk27(p.x, p.y, p.z, S, start, end, [&](uint32_t j) {
+    fg_walk27_rows(p.x, p.y, p.z, S, start, end, [&](uint32_t j) {
         if (j == i) return;
         const float4 q = __ldg(spos + j);
         const float dx = fmaf(-q.x, scale, px), dy = fmaf(-q.y, scale, py), dz = fmaf(-q.z, scale, pz);
@@ -699,7 +699,8 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces_walk(
  * spacing, 1381 us at 1,048,576 of 0.4 h; here 30 and 917.  Hits queued per
  * thread and drained together, 1923: lanes of a cell lose the loads that they
  * share while they walk in step.  Hits taken by a lane per target, 1268: their
- * numbers differ by lane and round.)  192 staged candidates leave twelve CTAs
+ * numbers differ by lane and round.)  Dispersed ranges walk by thread: in
+ * k_forces_dispersed, or here where a warp has fewer than 32 targets.  192 staged candidates leave twelve CTAs
  * an SM: 256, 991 us; 128, 1073.  The rigid contact follows by warp, for the
  * particles in cells marked near a sphere; walked by every particle, it was
  * three quarters of the 660 us at 262,144 particles (215 now). */
@@ -719,8 +720,8 @@ struct ForceShared {
 };
 
 __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_search(
-    uint32_t n_all, const __grid_constant__ FgScene scene, uint32_t range, const float4 *__restrict__ spos,
-    const float4 *__restrict__ svel, const float2 *__restrict__ dp, const uint32_t *__restrict__ start,
+    uint32_t n_all, const __grid_constant__ FgScene scene, uint32_t range, uint32_t most, int dispersed,
+    const float4 *__restrict__ spos, const float4 *__restrict__ svel, const float2 *__restrict__ dp, const uint32_t *__restrict__ start,
     const uint32_t *__restrict__ end, const uint32_t *__restrict__ ids, float4 *__restrict__ vel_out,
     float4 *__restrict__ pos_out, const __grid_constant__ RigidArgs R, float mass, float visc)
 {
@@ -735,7 +736,9 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
     for (uint32_t b0 = (blockIdx.x * (FG_FORCE_THREADS / 32u) + (threadIdx.x >> 5)) * range; b0 < n_all;
          b0 += gridDim.x * (FG_FORCE_THREADS / 32u) * range) {
         uint32_t next, stop;
-        fg_stage_range(b0, range, 0u, n_all, 32u, false, G, spos, next, stop);
+        const bool walk = fg_stage_range(b0, range, 0u, n_all, most, dispersed == DISPERSED_ASIDE, G, spos, next,
+                                         stop);
+        if (walk && dispersed == DISPERSED_ASIDE) continue;
         while (next < stop) {
             const uint32_t i0 = next, i = next + lane; /* sorted index */
             uint32_t n = min(32u, stop - next);
@@ -750,7 +753,7 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
             const float px = p.x * scale, py = p.y * scale, pz = p.z * scale;
             float fx = 0.f, fy = 0.f, fz = 0.f;
             uint32_t lead, leads;
-            fg_stage_groups(sig, __ballot_sync(FG_FULL, active && !sig.odd), lead, leads);
+            fg_stage_groups(sig, __ballot_sync(FG_FULL, active && !sig.odd && !walk), lead, leads);
             for (; leads; leads &= leads - 1u) {
                 const uint32_t l = (uint32_t)__ffs((int)leads) - 1u;
                 const uint32_t group = __ballot_sync(FG_FULL, lead == l);
@@ -845,13 +848,47 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
                         }
                     });
             }
-            if (active && sig.odd) walk_terms(S, i, p, v, kv, spos, svel, dp, start, end, fx, fy, fz);
+            if (active && (sig.odd || walk)) walk_terms(S, i, p, v, kv, spos, svel, dp, start, end, fx, fy, fz);
             __syncwarp();
             float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
             if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false);
             if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true);
             if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, __ldg(ids + i), vel_out, pos_out);
         }
+    }
+}
+
+/* The dispersed ranges of the launchers' force pass, a thread a target, as
+ * k_density_dispersed: 1,048,576 random targets 0.8 h apart 610 us staged -> 527,
+ * 1.2 h 749 -> 366, 3 h 799 -> 307; 262,144, 1.7 h 241 -> 75; 0.5 h, where no
+ * range is dispersed, 584 -> 589.  Seven CTAs an SM: with six, 262,144 take 98. */
+#define FG_WALK_FORCE_CTAS 7
+__global__ void __launch_bounds__(FG_CHUNK, FG_WALK_FORCE_CTAS) k_forces_dispersed(
+    uint32_t n_all, const __grid_constant__ FgScene scene, uint32_t most, const float4 *__restrict__ spos,
+    const float4 *__restrict__ svel, const float2 *__restrict__ dp, const uint32_t *__restrict__ start,
+    const uint32_t *__restrict__ end, const uint32_t *__restrict__ ids, float4 *__restrict__ vel_out,
+    float4 *__restrict__ pos_out, const __grid_constant__ RigidArgs R, float mass, float visc)
+{
+    const FgScene *S = &scene;
+    const StageGrid G(S);
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t i0 = blockIdx.x * FG_CHUNK + (threadIdx.x & ~31u);
+    float4 ahead = __ldg(spos + min(i0 + lane, n_all - 1u));
+    for (; i0 < n_all; i0 += gridDim.x * FG_CHUNK) {
+        const uint32_t i = i0 + lane;
+        const float4 p = ahead;
+        ahead = __ldg(spos + min(i + gridDim.x * FG_CHUNK, n_all - 1u));
+        if (!fg_stage_dispersed(fg_stage_cell(p, G), G, 32u, most)) continue;
+        const bool valid = i < n_all, active = valid && p.w > 0.0f;
+        const float4 v = valid ? __ldg(svel + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float fx = 0.f, fy = 0.f, fz = 0.f;
+        if (active) walk_terms(S, i, p, v, S->kvisc * visc, spos, svel, dp, start, end, fx, fy, fz);
+        __syncwarp();
+        float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
+        if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false);
+        if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true);
+        if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, __ldg(ids + i), vel_out, pos_out);
+        __syncwarp();
     }
 }
 
@@ -867,9 +904,16 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
     if (statics) { R.sta = *statics; R.use_sta = 1; }
     if (!list && use_o) {
         const uint32_t range = stage_range(L.nwork), warps = (L.n + range - 1u) / range;
-        const uint32_t per_cta = FG_FORCE_THREADS / 32u;
-        k_forces_search<<<grid_for((warps + per_cta - 1u) / per_cta, 128), FG_FORCE_THREADS, 0, L.stream>>>(
-            L.n, *L.single, range, spos, svel, dp, start, end, ids, out.vel, out.pos, R, mass_o, visc_o);
+        const uint32_t ctas = grid_for((warps + FG_FORCE_THREADS / 32u - 1u) / (FG_FORCE_THREADS / 32u), 128);
+        uint32_t most;
+        const int dispersed = dispersed_ranges(L, range, false, most);
+        const SideLaunch side(L, dispersed == DISPERSED_ASIDE);
+        if (side.use)
+            k_forces_dispersed<<<grid_for(L.nwork, FG_WALK_FORCE_CTAS), FG_CHUNK, 0, L.side.stream>>>(
+                L.n, *L.single, most, spos, svel, dp, start, end, ids, out.vel, out.pos, R, mass_o, visc_o);
+        k_forces_search<<<ctas, FG_FORCE_THREADS, 0, L.stream>>>(L.n, *L.single, range, most, dispersed, spos, svel,
+                                                                dp, start, end, ids, out.vel, out.pos, R, mass_o,
+                                                                visc_o);
         return;
     }
     const uint32_t B = L.block ? L.block : FG_CHUNK;
