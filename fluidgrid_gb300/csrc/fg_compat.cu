@@ -356,6 +356,12 @@ void gSPHCalculateForcesWithSRB(float4 *oldPositions, float4 *oldVelocity, float
     int r = useDynamicRB ? mark_near(dyn, 0u, S) : FG_OK;
     if (r == FG_OK && useStaticRB) r = mark_near(sta, 1u, S);
     if (r != FG_OK) { g_status = r; return; }
+    /* one grid's contact ahead, each particle's in its place of the output */
+    if (useDynamicRB || useStaticRB) {
+        fg::RigidGrid &grid = useDynamicRB ? dyn : sta;
+        fg::launch_fluid_contact(L, oldPositions, oldVelocity, grid, newVel, particleId);
+        grid.pre = newVel;
+    }
     fg::launch_forces(L, oldPositions, oldVelocity, density_pressure, gridStart, gridEnd, particleId, o,
                       useDynamicRB ? &dyn : nullptr, useStaticRB ? &sta : nullptr, mass, kViscosity, 1);
     finish();

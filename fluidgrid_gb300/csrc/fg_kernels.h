@@ -188,7 +188,8 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * cell marked near a sphere (G.near), out[id] = its contact with grid G
  * (ProcessCollisionForcesD).  The force pass then
  * reads it (G.pre). */
-void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out);
+void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out,
+                          const uint32_t *ids = nullptr);
 
 void launch_integrate(const Launch &L, float4 *pos, const float4 *vel);
 

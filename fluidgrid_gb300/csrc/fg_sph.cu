@@ -479,11 +479,19 @@ __device__ __forceinline__ float3 force_contact(const FgScene *S, uint32_t scene
 }
 
 /* The contact of a warp's particles (whole warp, converged) with a grid whose
- * near cells are marked, one particle after another by the whole warp. */
+ * near cells are marked: read from particle oi's place where the contact pass
+ * stored it, else one particle after another by the whole warp. */
 __device__ __forceinline__ float3 force_contact_warp(const FgScene *S, bool active, float4 p, float4 v,
-                                                     const RigidGrid &G, bool dynamic)
+                                                     const RigidGrid &G, bool dynamic, uint32_t oi)
 {
     float3 c = make_float3(0.f, 0.f, 0.f);
+    if (G.pre) {
+        if (active && fg_contact_marked(S, 0u, p, G)) {
+            const float4 q = __ldcg(G.pre + oi);
+            c = make_float3(q.x, q.y, q.z);
+        }
+        return c;
+    }
     const ContactShape C(S);
     for (uint32_t m = __ballot_sync(FG_FULL, active && fg_contact_marked(S, 0u, p, G)); m; m &= m - 1u) {
         const int b = __ffs((int)m) - 1;
@@ -702,8 +710,8 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces_walk(
  * numbers differ by lane and round.)  Dispersed ranges walk by thread: in
  * k_forces_dispersed, or here where a warp has fewer than 32 targets.  192 staged candidates leave twelve CTAs
  * an SM: 256, 991 us; 128, 1073.  The rigid contact follows by warp, for the
- * particles in cells marked near a sphere; walked by every particle, it was
- * three quarters of the 660 us at 262,144 particles (215 now). */
+ * particles in cells marked near a sphere, where both grids are given: else it
+ * is read from the contact pass. */
 #ifndef FG_FORCE_STAGE
 #define FG_FORCE_STAGE 192u
 #endif
@@ -850,10 +858,11 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
             }
             if (active && (sig.odd || walk)) walk_terms(S, i, p, v, kv, spos, svel, dp, start, end, fx, fy, fz);
             __syncwarp();
+            const uint32_t oi = valid ? __ldg(ids + i) : 0u;
             float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
-            if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false);
-            if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true);
-            if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, __ldg(ids + i), vel_out, pos_out);
+            if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false, oi);
+            if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true, oi);
+            if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, oi, vel_out, pos_out);
         }
     }
 }
@@ -884,10 +893,11 @@ __global__ void __launch_bounds__(FG_CHUNK, FG_WALK_FORCE_CTAS) k_forces_dispers
         float fx = 0.f, fy = 0.f, fz = 0.f;
         if (active) walk_terms(S, i, p, v, S->kvisc * visc, spos, svel, dp, start, end, fx, fy, fz);
         __syncwarp();
+        const uint32_t oi = valid ? __ldg(ids + i) : 0u;
         float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
-        if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false);
-        if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true);
-        if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, __ldg(ids + i), vel_out, pos_out);
+        if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false, oi);
+        if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true, oi);
+        if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, oi, vel_out, pos_out);
         __syncwarp();
     }
 }
@@ -949,7 +959,13 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * ids along a surface may all need.  4M particles, eight bodies whose AABB is
  * the whole scene: 1007 -> 151 us (a lane each inside the AABB -> here; a lane
  * each in marked cells only: 399; a warp per eight particles: 235).  The force
- * pass adds the stored sum where it would add the walked one: the same bits. */
+ * pass adds the stored sum where it would add the walked one: the same bits.
+ * The launchers' pass goes over sorted particles and stores by id; within the
+ * force search, whose shared memory leaves the bucket tables no L1, the same
+ * searches took twice the time and more (262,144 particles: 4,096 spheres all
+ * among them 652 -> 376 us for contact and forces; 32,768 and a half-width of
+ * 4, half as many particles, 2584 -> 987; four bodies' surfaces, the whole
+ * two-way pass, 488 -> 439). */
 #define FG_CONTACT_THREADS 256u
 __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWork *__restrict__ work, uint32_t nwork,
                                                            uint32_t n_single, const FgScene *__restrict__ table,
@@ -957,6 +973,7 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
                                                            const float4 *__restrict__ pos,
                                                            const float4 *__restrict__ vel,
                                                            const __grid_constant__ RigidGrid G,
+                                                           const uint32_t *__restrict__ ids,
                                                            float4 *__restrict__ out)
 {
     __shared__ uint32_t s_id[FG_CHUNK], s_n;
@@ -982,23 +999,25 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
         }
         __syncthreads();
         const ContactShape C(S);
+        const bool dynamic = G.body_vel != nullptr;
         for (uint32_t k = threadIdx.x >> 5; k < s_n; k += FG_CONTACT_THREADS / 32u) {
             const uint32_t id = s_id[k];
-            const float3 c = fg_contact_warp(S, C, __ldg(pos + id), __ldg(vel + id), G, true);
-            if (lane == 0u) out[id] = make_float4(c.x, c.y, c.z, 0.0f);
+            const float3 c = fg_contact_warp(S, C, __ldg(pos + id), __ldg(vel + id), G, dynamic);
+            if (lane == 0u) out[ids ? __ldg(ids + id) : id] = make_float4(c.x, c.y, c.z, 0.0f);
         }
         __syncthreads();
     }
 }
 
-void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out)
+void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out,
+                          const uint32_t *ids)
 {
     if (!L.nwork) return;
     /* an SM's worth of CTAs: a CTA per item queues ahead of the grid kernels
      * beside this one (64 worlds after 400 steps 896 us a step, here 883; 4M
      * particles 2163, here 2135) */
     k_fluid_contact<<<grid_for(L.nwork, 8), FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos, vel,
-                                                                  G, out);
+                                                                  G, ids, out);
 }
 
 /* SPHIntegrateK (K_FluidSim.cu:418-438): pos += vel*(dt/scale) for active
