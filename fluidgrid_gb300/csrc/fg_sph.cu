@@ -967,6 +967,12 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * 4, half as many particles, 2584 -> 987; four bodies' surfaces, the whole
  * two-way pass, 488 -> 439). */
 #define FG_CONTACT_THREADS 256u
+/* Searches of a CTA beyond which the 27 buckets of a half-width of 1, which
+ * leave most of a warp's lanes idle, are walked by thread: a step of 131,072
+ * particles with 4,096 spheres among all of them 209 -> 170 us, 32,768 spheres
+ * 272 -> 240; surfaces stay below it.  (Half-widths of 2 and more: 257 us walked
+ * and 245 searched with 1,024 spheres, 437 and 353 with 32,768.) */
+#define FG_CONTACT_SEARCHES 80u
 __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWork *__restrict__ work, uint32_t nwork,
                                                            uint32_t n_single, const FgScene *__restrict__ table,
                                                            const __grid_constant__ FgScene single,
@@ -1000,6 +1006,15 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
         __syncthreads();
         const ContactShape C(S);
         const bool dynamic = G.body_vel != nullptr;
+        if (C.total <= 27u && s_n > FG_CONTACT_SEARCHES) {
+            if (threadIdx.x < s_n) {
+                const uint32_t id = s_id[threadIdx.x];
+                const float3 c = fg_fluid_rigid_contact(S, it.scene, __ldg(pos + id), __ldg(vel + id), G, dynamic);
+                out[ids ? __ldg(ids + id) : id] = make_float4(c.x, c.y, c.z, 0.0f);
+            }
+            __syncthreads();
+            continue;
+        }
         for (uint32_t k = threadIdx.x >> 5; k < s_n; k += FG_CONTACT_THREADS / 32u) {
             const uint32_t id = s_id[k];
             const float3 c = fg_contact_warp(S, C, __ldg(pos + id), __ldg(vel + id), G, dynamic);
