@@ -971,7 +971,6 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_pass(const uint32_t *__restri
 
     uint32_t key[RS_ITEMS], val[RS_ITEMS], rank[RS_ITEMS];
     const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t bits = (uint32_t)__popc(mask);
 #pragma unroll
     for (int k = 0; k < RS_ITEMS; k++) {
         const size_t i = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane;
@@ -982,7 +981,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_pass(const uint32_t *__restri
     for (int k = 0; k < RS_ITEMS; k++) {
         const bool valid = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane < n;
         const uint32_t d = (key[k] >> shift) & mask;
-        const uint32_t peers = rs_peers(d, bits) & __ballot_sync(0xffffffffu, valid);
+        /* not a ballot a bit, as k_rs_downsweep: this pass is bound by issue
+         * beside its look-back (1M particles of a lattice, three passes: 65 us
+         * so, 51.5 with match_any; random ones 66 and 60) */
+        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : 0xffffffffu);
         const uint32_t leader = valid ? (uint32_t)__ffs((int)peers) - 1u : lane;
         uint32_t b = 0;
         if (valid && lane == leader) {
