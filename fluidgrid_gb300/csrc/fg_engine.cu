@@ -750,6 +750,10 @@ uint32_t World::sort_launches() const
     return (one_pass_sort && n && P <= 6) ? 2 + P : (P ? radix_launches(n, key_bits, digit_bits) : 0u);
 }
 
+/* Whether a sort of this world goes by digit_bits: one launch of the whole sort
+ * does not, so that a trial of its widths would time the same kernels. */
+bool World::digit_bits_count() const { return one_pass_sort || !radix_one_launch(n); }
+
 /* The hash pass; when the counting sort follows, it counts the keys too. */
 void World::enqueue_hash(const Launch &L, bool sort_follows)
 {
@@ -1054,7 +1058,7 @@ void World::tune_begin()
     int dims[6], nd = 0;
     if (__builtin_popcount(tune_kernels & 0x7u) >= 2) dims[nd++] = 0;
     if ((tune_tiles & 1u) && !use_cc) dims[nd++] = 1;
-    if (tune_tiles & 2u) dims[nd++] = 2;
+    if ((tune_tiles & 2u) && digit_bits_count()) dims[nd++] = 2;
     if (tune_tiles & 4u) dims[nd++] = 3;
     if ((tune_tiles & 8u) && !use_cc) dims[nd++] = 4;
     if ((tune_tiles & 16u) && use_cc) dims[nd++] = 5;

@@ -100,6 +100,7 @@ struct World {
         return total_buckets && tiles <= radix_hist_words((uint32_t)std::max<uint64_t>(cap.particles, 1));
     }
     uint32_t sort_launches() const;
+    bool digit_bits_count() const;
     NbrList nbr{nullptr, nullptr, nullptr, 0, nullptr, nullptr}; /* density -> forces neighbour lists */
     uint32_t list_cap_alloc = 0; /* list slots per particle allocated (the stride) */
     uint32_t list_cap = 0;       /* entries a particle may store (<= list_cap_alloc) */

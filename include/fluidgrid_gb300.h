@@ -193,7 +193,8 @@ int fg_world_set_graphs(fg_world *w, int on);
  *                         density pass takes its targets in bucket order,
  *                         where they stand cell by cell
  *   FG_OPT_ORDER_PERIOD   steps between refreshes of the Morton order (16)
- *   FG_OPT_DIGIT_BITS     radix digit width 1..8
+ *   FG_OPT_DIGIT_BITS     radix digit width 1..8 (the sorts of up to 65,536
+ *                         pairs that take one launch always use 8)
  *   FG_OPT_AUTOTUNE_PERIOD  every this many steps the autotuner runs one
  *                         (real) step per candidate value of one tunable
  *                         under CUDA events and keeps the fastest (0 = off;

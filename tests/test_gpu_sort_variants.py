@@ -62,3 +62,17 @@ def test_keys_and_ids_are_the_stable_order(form, variant, bits):
 def test_the_target_order_changes_no_bit(bits):
     a, b = stepped("random", 2, bits, order=0), stepped("random", 2, bits, order=2)
     assert np.array_equal(a["VEL"].view(np.uint32), b["VEL"].view(np.uint32))
+
+
+@pytest.mark.parametrize("n,tuned", [(20_011, False), (N, True)])
+def test_the_tuner_tries_digit_widths_where_a_sort_goes_by_them(n, tuned):
+    spec = scene("lattice")
+    spec.pos, spec.vel = spec.pos[:n].copy(), spec.vel[:n].copy()
+    w = World([spec])
+    w.set_option("one_pass_sort", 0)
+    w.set_option("digit_bits", 5)
+    w.set_option("autotune_tiles", 2)  # the digit width only: 6 to 8
+    w.set_option("autotune_period", 4)
+    w.step(12)
+    assert (w.get_option("digit_bits") != 5) == tuned
+    w.close()
