@@ -554,7 +554,9 @@ void World::stale_graphs()
 
 int World::init_stream(cudaStream_t st)
 {
-    (void)sm_count(); /* cache the device query outside any graph capture */
+    /* cache the device queries outside any graph capture */
+    (void)sm_count();
+    (void)cluster_ctas();
     if (st) {
         stream = st;
         own_stream = false;
@@ -2160,6 +2162,20 @@ int fg_probe_fp32_peak(float *tflops)
 }
 
 const char *fg_last_error(void) { return fg::g_err.c_str(); }
+
+int fg_selftest_cluster_sort(unsigned int ctas, unsigned int *keys, unsigned int *values, unsigned int keyBits,
+                             unsigned int n, fg_stream_t stream)
+{
+    if (!keys || !values || !ctas || ctas > 16u || (ctas & (ctas - 1u)) || !keyBits || keyBits > 32u || !n ||
+        n > 65536u || n > 8192u * ctas)
+        return FG_E_INVALID;
+    const cudaError_t e = fg::one_launch_sort(keys, values, keys, values, n, keyBits, ctas, (cudaStream_t)stream);
+    if (e != cudaSuccess) {
+        fg::set_error("fg_selftest_cluster_sort", e);
+        return FG_E_CUDA;
+    }
+    return FG_OK;
+}
 
 int fg_selftest_bounded_wait(unsigned int spin_limit, unsigned int *flags)
 {

@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 #include <stdint.h>
 #include <algorithm>
+#include <atomic>
 #include "fg_device.cuh"
 #include "fg_kernels.h"
 
@@ -567,20 +568,27 @@ static cudaError_t cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &
     return cudaFuncSetAttribute(k_sort_cluster<ITEMS>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
 
-/* CTAs of the largest cluster that the GPU places: sixteen, or the portable
- * eight where no part of it has sixteen SMs together (a partition). */
-static uint32_t cluster_ctas()
+/* CTAs of the largest cluster that the current device places: sixteen, or the
+ * portable eight where no part of it has sixteen SMs together (a partition).
+ * Asked once a device; two threads that ask at once get the same answer. */
+uint32_t cluster_ctas()
 {
-    static uint32_t ctas = 0u;
+    constexpr int kDevices = 32;
+    static std::atomic<uint32_t> known[kDevices];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 8u;
+    uint32_t ctas = known[dev].load(std::memory_order_relaxed);
     if (!ctas) {
+        const bool clean = cudaPeekAtLastError() == cudaSuccess;
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute at[1];
         int active = 0;
         if (cluster_config<4>(cfg, at[0], CS_CTAS, 0) != cudaSuccess ||
             cudaOccupancyMaxActiveClusters(&active, k_sort_cluster<4>, &cfg) != cudaSuccess)
             active = 0;
-        if (!active) cudaGetLastError();
+        if (!active && clean) cudaGetLastError(); /* the query's own error */
         ctas = active > 0 ? CS_CTAS : 8u;
+        known[dev].store(ctas, std::memory_order_relaxed);
     }
     return ctas;
 }
@@ -596,6 +604,17 @@ static cudaError_t cluster_sort(const uint32_t *kin, const uint32_t *vin, uint32
     const cudaError_t e = cluster_config<ITEMS>(cfg, at[0], ctas, st);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, k_sort_cluster<ITEMS>, kin, vin, kout, vout, n, bits);
+}
+
+/* As many CTAs as give each thread one pair, up to `most`, then more pairs. */
+cudaError_t one_launch_sort(const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, uint32_t n,
+                            uint32_t bits, uint32_t most, cudaStream_t st)
+{
+    const uint32_t per = most * CS_THREADS;
+    if (n <= per) return cluster_sort<1>(kin, vin, kout, vout, n, bits, st);
+    if (n <= 2u * per) return cluster_sort<2>(kin, vin, kout, vout, n, bits, st);
+    if (n <= 4u * per) return cluster_sort<4>(kin, vin, kout, vout, n, bits, st);
+    return cluster_sort<8>(kin, vin, kout, vout, n, bits, st);
 }
 
 /* Pairs that one launch sorts.  The three kernels a pass, over the whole chip,
@@ -623,14 +642,7 @@ cudaError_t radix_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_
             k_iota_copy<<<grid_for((n + 255) / 256, 8), 256, 0, st>>>(keys_in, vals_in, keys_out, vals_out, n);
         return cudaSuccess;
     }
-    if (radix_one_launch(n)) {
-        /* as many CTAs as give each thread one pair, up to the largest cluster */
-        const uint32_t per = cluster_ctas() * CS_THREADS;
-        if (n <= per) return cluster_sort<1>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
-        if (n <= 2u * per) return cluster_sort<2>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
-        if (n <= 4u * per) return cluster_sort<4>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
-        return cluster_sort<8>(keys_in, vals_in, keys_out, vals_out, n, bits, st);
-    }
+    if (radix_one_launch(n)) return one_launch_sort(keys_in, vals_in, keys_out, vals_out, n, bits, cluster_ctas(), st);
     const uint32_t T = (n + RS_TILE - 1) / RS_TILE;
     uint32_t *totals = s.hist + (size_t)RS_RADIX * T;
     /* the last pass lands in *_out: an odd number of passes starts towards it,

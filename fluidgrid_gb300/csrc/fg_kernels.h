@@ -56,6 +56,11 @@ int radix_passes(uint32_t bits, uint32_t digit_bits);
 uint32_t radix_launches(uint32_t n, uint32_t bits, uint32_t digit_bits);
 /* whether a radix_sort of n pairs is one launch, which leaves the scratch alone */
 bool radix_one_launch(uint32_t n);
+/* CTAs of the cluster that sorts so (asked of the current device once) */
+uint32_t cluster_ctas();
+/* that launch with clusters of at most `most` CTAs (a power of two); n <= 8192 most */
+cudaError_t one_launch_sort(const uint32_t *keys_in, const uint32_t *vals_in, uint32_t *keys_out, uint32_t *vals_out,
+                            uint32_t n, uint32_t bits, uint32_t most, cudaStream_t st);
 /* One-kernel-per-pass variant (decoupled look-back) for the world's fluid
  * sort: same result as radix_sort with vals_in = 0..n-1.  os is
  * onesweep_words(n) words of scratch; err receives FG_DEV_SORT_TIMEOUT if a

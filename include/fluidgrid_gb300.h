@@ -333,6 +333,11 @@ int fg_sort_pairs_noalloc(unsigned int *keys, unsigned int *values, unsigned int
  * spin_limit rounds; *flags receives the device status bits it set (2 = the
  * sort's wait gave up).  The context stays usable afterwards. */
 int fg_selftest_bounded_wait(unsigned int spin_limit, unsigned int *flags);
+/* The sort that takes one launch, in place, with clusters of at most `ctas`
+ * CTAs (1, 2, 4, 8 or 16; n up to 8,192 for each, at most 65,536): 8 is what a
+ * part of a GPU that places no sixteen uses. */
+int fg_selftest_cluster_sort(unsigned int ctas, unsigned int *keys, unsigned int *values, unsigned int keyBits,
+                             unsigned int n, fg_stream_t stream);
 
 /* ---- served form: continuous batching of scenes (no reference
  * counterpart; each scene's step is HeterogeneousSimulator::doTimeStep) ----
