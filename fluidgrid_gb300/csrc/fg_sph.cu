@@ -50,12 +50,8 @@ namespace fg {
  * 90 (60-100 candidates kept of a cell's 216).  384 and ten CTAs an SM leave
  * the L1 60 KB: nine CTAs with 448, whose shared memory is no more, take 1395
  * us at 4M, ten with 320, more rounds, 1265, eleven 1480. */
-#ifndef FG_DENSITY_STAGE
 #define FG_DENSITY_STAGE 384u
-#endif
-#ifndef FG_DENSITY_CTAS
 #define FG_DENSITY_CTAS 10
-#endif
 #define FG_STAGE_GROUPS 9u /* staged together; a warp of more takes them nine by nine */
 #define FG_DENSITY_THREADS 64u
 
@@ -268,7 +264,7 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
                     for (uint32_t k = 0u; k < FG_STAGE_GROUPS; k++) later &= later - 1u;
                     const uint32_t batch = leads ^ later;
                     leads = later;
-                    fg_stage_rounds<FG_DENSITY_STAGE>(
+                    fg_stage_rounds<FG_DENSITY_STAGE, FG_STAGE_GROUPS>(
                         sig, lead, batch, px, py, pz, G, spos, start, end, sm.idx,
                         [&](uint32_t slot, uint32_t j, float4 c) {
                             ((float *)sm.x)[slot] = c.x;
@@ -712,12 +708,8 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces_walk(
  * an SM: 256, 991 us; 128, 1073.  The rigid contact follows by warp, for the
  * particles in cells marked near a sphere, where both grids are given: else it
  * is read from the contact pass. */
-#ifndef FG_FORCE_STAGE
 #define FG_FORCE_STAGE 192u
-#endif
-#ifndef FG_FORCE_CTAS
 #define FG_FORCE_CTAS 12
-#endif
 #define FG_FORCE_THREADS 64u
 struct ForceShared {
     float4 a[FG_FORCE_STAGE];         /* x, y, z, rho */
@@ -765,7 +757,7 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
             for (; leads; leads &= leads - 1u) {
                 const uint32_t l = (uint32_t)__ffs((int)leads) - 1u;
                 const uint32_t group = __ballot_sync(FG_FULL, lead == l);
-                fg_stage_rounds<FG_FORCE_STAGE>(
+                fg_stage_rounds<FG_FORCE_STAGE, 1u>(
                     sig, lead, 1u << l, px, py, pz, G, spos, start, end, sm.idx,
                     [&](uint32_t slot, uint32_t j, float4 c) {
                         sm.a[slot] = c;

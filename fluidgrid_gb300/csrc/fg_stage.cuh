@@ -101,13 +101,8 @@ __device__ __forceinline__ float fg_redux_max(float v)
     return r;
 }
 
-#ifndef FG_STAGE_WINDOW
 #define FG_STAGE_WINDOW 256u /* candidate positions expanded at a time */
-#endif
-
-#ifndef FG_STAGE_FLIGHT
-#define FG_STAGE_FLIGHT 4u /* chunks of 32 candidates whose loads are in flight together */
-#endif
+#define FG_STAGE_FLIGHT 4u   /* chunks of 32 candidates whose loads are in flight together */
 
 struct StageCell {
     int x, y, z;
@@ -184,17 +179,19 @@ __device__ __forceinline__ uint32_t fg_stage_trim(const StageSig &s, float4 afte
     return m ? 32u - (uint32_t)__clz((int)m) : 32u;
 }
 
-/* Stages the groups' candidates round after round (CAP slots) and calls
+/* Stages the candidates of up to GROUPS groups round after round (CAP slots) and calls
  * run(first, end, used) once a round, the whole warp: this lane's candidates
  * are slots [first, end) of [0, used), in visit order and a multiple of eight
  * of them, filled up with x = +inf, which is out of every range.  keep(slot, j, c) stores
- * candidate j at c; up to CAP / 40 groups, so that each has room for a chunk. */
-template <uint32_t CAP, class Keep, class Run>
+ * candidate j at c.  Every round gets on: its first group's share of the slots
+ * holds a chunk. */
+template <uint32_t CAP, uint32_t GROUPS, class Keep, class Run>
 __device__ __forceinline__ void fg_stage_rounds(const StageSig &sig, uint32_t lead, uint32_t leads, float px, float py,
                                                 float pz, const StageGrid &G, const float4 *__restrict__ spos,
                                                 const uint32_t *__restrict__ start, const uint32_t *__restrict__ end,
                                                 uint32_t *idx /* FG_STAGE_WINDOW, shared */, Keep &&keep, Run &&run)
 {
+    static_assert(CAP % 8u == 0u && ((CAP / GROUPS) & ~7u) >= 32u, "a round in which no chunk fits would never end");
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
     const float scale = G.scale, h2 = G.h2;
