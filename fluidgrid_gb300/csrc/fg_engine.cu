@@ -1238,6 +1238,7 @@ int World::step_loop(uint32_t nsteps)
             int r = graph_for_current(&ge, span);
             if (r != FG_OK) return r;
             CK(cudaGraphLaunch(ge, stream));
+            graph_launches++;
             kernels_enqueued += (uint64_t)span * launches_per_step();
             tune_count[current_kernel()] += span;
             counted_steps += span;
@@ -1264,6 +1265,7 @@ int World::step_loop(uint32_t nsteps)
         if (tr.active) CK(cudaEventRecord(tr.ev[2 * tr.idx], stream));
         if (!use_graphs) enqueue_step();
         else CK(cudaGraphLaunch(ge, stream));
+        graph_launches += use_graphs ? 1u : 0u;
         kernels_enqueued += launches_per_step();
         if (tr.active) {
             CK(cudaEventRecord(tr.ev[2 * tr.idx + 1], stream));
@@ -2072,6 +2074,13 @@ int fg_world_kernel_launches(const fg_world *w, uint64_t *count)
 {
     if (!w || !count) return FG_E_INVALID;
     *count = ((const World *)w)->kernels_enqueued;
+    return FG_OK;
+}
+
+int fg_world_graph_launches(const fg_world *w, uint64_t *count)
+{
+    if (!w || !count) return FG_E_INVALID;
+    *count = ((const World *)w)->graph_launches;
     return FG_OK;
 }
 

@@ -156,6 +156,12 @@ class World:
         check(self.L.fg_world_kernel_launches(self.h, ctypes.byref(c)), "fg_world_kernel_launches")
         return int(c.value)
 
+    def graph_launches(self):
+        """Graph launches so far, of one step or of several."""
+        c = ctypes.c_uint64(0)
+        check(self.L.fg_world_graph_launches(self.h, ctypes.byref(c)), "fg_world_graph_launches")
+        return int(c.value)
+
     # ---------------------------------------------------------------- timing
     STAGES = ["hash", "sort", "ranges", "density", "rb_grid", "rb_contact", "forces", "bodies"]
 
