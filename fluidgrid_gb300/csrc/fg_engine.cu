@@ -312,7 +312,7 @@ int World::reserve(const Capacity &c)
     k_set_u32<<<1, 1, 0, stream>>>(list_cap_d, list_cap);
     nbr.max_count = max_count;
     nbr.overflow = overflow_counter;
-    nbr.dispersed = max_count + 2;
+    nbr.spread = max_count + 2;
     CK(cudaMemsetAsync(dp, 0, 8 * N, stream));
     CK(cudaMemsetAsync(vel, 0, 16 * N, stream));
     CK(cudaMemsetAsync(end, 0, 4 * NB, stream));
@@ -618,7 +618,8 @@ Launch World::fluid_launch() const
     L.stream = stream;
     L.ctas_per_sm = ctas_per_sm;
     L.block = block;
-    if (dispersed || !use_list) L.side = SideStream{stream3, ev_walk, ev_walk_done};
+    if (!use_list) L.side = SideStream{stream3, ev_walk, ev_walk_done};
+    L.walk = density_walks;
     return L;
 }
 
@@ -964,7 +965,7 @@ uint64_t World::graph_signature() const
            ((ordered && order_forces_only) ? 1ull << 19 : 0ull) | ((uint64_t)(ctas_per_sm & 0x7fu) << 20) |
            (one_pass_sort ? 1ull << 27 : 0ull) | (bucket_sort_on ? 1ull << 28 : 0ull) |
            ((uint64_t)((block >> 6) & 0x7u) << 29) | ((uint64_t)(cc_warps & 0x7u) << 32) |
-           (dispersed ? 1ull << 35 : 0ull) |
+           (density_walks ? 1ull << 35 : 0ull) |
            ((uint64_t)nbr.stride << 40);
 }
 
@@ -1145,18 +1146,20 @@ int World::tune_finish()
 /* Every FG_LIST_CHECK_PERIOD steps (kernel 1): grow the neighbour-list
  * capacity to 1.125x the largest in-range count seen since the last check,
  * so the force pass walks lists instead of buckets as a scene compresses; and
- * give the density pass's dispersed ranges a kernel of their own while they
- * are an eighth of all or more. */
+ * choose between the density pass's forms for the steps to come: staged, or
+ * walked by thread where the ranges of 32 targets lie in more than 7.5 buckets
+ * in the mean.  Steps, staged and walked: 1,000 scenes of 100 particles (12.6)
+ * 91 and 51 us, 100 of 3,000 splashed (7.7) 177 and 179, 50 of 10,000 (6.6) 296
+ * and 281, 30 uneven ones (6.3) 298 and 322, 1M of a lattice (5.2) 603 and 690;
+ * 1,048,576 random particles 0.65 h apart 562 and 494, 1.2 h 550 and 367. */
 int World::check_list_cap()
 {
     const bool grow = step_count % FG_LIST_CHECK_PERIOD == 0;
-    uint32_t seen[3]; /* largest count, the capacity, dispersed ranges */
+    uint32_t seen[4]; /* largest count, the capacity, buckets and number of the ranges counted */
     CK(cudaMemcpyAsync(seen, max_count, sizeof(seen), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    CK(cudaMemsetAsync(nbr.dispersed, 0, 4, stream));
-    /* an eighth of the ranges is counted, four to a work item */
-    dispersed = seen[2] && 16ull * seen[2] >= (step_count - checked_at) * nwork;
-    checked_at = step_count;
+    CK(cudaMemsetAsync(nbr.spread, 0, 8, stream));
+    density_walks = density_ranges_wide(nwork) && 2ull * seen[2] > 15ull * seen[3];
     if (!grow) return FG_OK;
     CK(cudaMemsetAsync(max_count, 0, 4, stream));
     const uint32_t mx = seen[0];

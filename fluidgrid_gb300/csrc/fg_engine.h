@@ -151,10 +151,9 @@ struct World {
     bool own_stream = false;
     cudaStream_t stream2 = nullptr; /* rigid-body branch of a full step */
     cudaEvent_t ev_fork = nullptr, ev_fluid_ready = nullptr, ev_rb_done = nullptr, ev_bodies_done = nullptr;
-    cudaStream_t stream3 = nullptr; /* velocity upload of an end-to-end step; the density pass's dispersed ranges */
+    cudaStream_t stream3 = nullptr; /* velocity upload of an end-to-end step; the dispersed ranges of a pass without lists */
     cudaEvent_t ev_walk = nullptr, ev_walk_done = nullptr;
-    bool dispersed = false; /* those ranges are many: a kernel of their own (check_list_cap) */
-    uint64_t checked_at = 0; /* step of the last check */
+    bool density_walks = false; /* the density pass with lists walks by thread (check_list_cap) */
     cudaEvent_t ev_io_fork = nullptr, ev_vel_in = nullptr, ev_pos_in = nullptr;
     void enqueue_rb_grid(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches);
     void enqueue_rb_contact(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches, bool with_fluid);

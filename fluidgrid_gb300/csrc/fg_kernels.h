@@ -26,7 +26,8 @@ struct Launch {
     cudaStream_t stream;
     uint32_t ctas_per_sm;  /* density/force grids: CTAs of FG_CHUNK threads per SM (0 = 64) */
     uint32_t block;        /* density/force grids: threads per CTA, 64, 128 or 256 (0 = FG_CHUNK) */
-    SideStream side;       /* the staged passes' dispersed ranges go to kernels of their own beside them, or {} */
+    SideStream side;       /* a pass without lists: its dispersed ranges go to a kernel of their own there, or {} */
+    bool walk;             /* density with lists: every target walks by thread */
 };
 
 int sm_count();
@@ -147,7 +148,7 @@ struct NbrList {
     const uint32_t *cap;          /* device word: entries a target may store (<= stride) */
     uint32_t *max_count;          /* optional: atomicMax of cnt */
     unsigned long long *overflow; /* optional: targets with cnt > cap */
-    uint32_t *dispersed;          /* += an eighth of the dispersed ranges of 32 */
+    uint32_t *spread;             /* optional: += the buckets of every sixteenth range of 32, and 1 */
 };
 
 /* whether a density pass over nwork items takes ranges of 32 targets, whose

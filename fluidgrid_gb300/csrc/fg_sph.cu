@@ -202,6 +202,16 @@ __device__ __noinline__ uint2 density_walk_aside(const FgScene *S, uint32_t i, c
     return make_uint2(__float_as_uint(acc.sum()), acc.cnt);
 }
 
+/* A range's buckets, for the host (every sixteenth range of 32). */
+__device__ __forceinline__ void count_buckets(const NbrList &list, const StageCell &c, const StageGrid &G)
+{
+    const uint32_t b = fg_stage_buckets(c, G, 32u);
+    if (list.spread && (threadIdx.x & 31u) == 0u) {
+        atomicAdd(list.spread, b);
+        atomicAdd(list.spread + 1, 1u);
+    }
+}
+
 /* What a pass does with its dispersed ranges: those of more than `most`
  * buckets, whose targets share too little for a lookup and a cull a cell. */
 enum { DISPERSED_STAGED, DISPERSED_WALKED, DISPERSED_ASIDE /* another kernel has them */ };
@@ -231,14 +241,11 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
         const float scale = S->scale, h2 = S->h2;
         const StageGrid G(S);
         uint32_t next, stop;
-        bool walk = fg_stage_range(it.first + q0, range, lo, hi, most, dispersed == DISPERSED_ASIDE, G, spos, next,
-                                   stop);
-        if (walk) {
-            /* an eighth of them, for the host */
-            if (LIST && list.dispersed && lane == 0u && (warp & 7u) == 0u) atomicAdd(list.dispersed, 1u);
-            if (dispersed == DISPERSED_ASIDE) continue;
-            walk = dispersed == DISPERSED_WALKED;
-        }
+        const bool walk = fg_stage_range(it.first + q0, range, lo, hi, most, dispersed == DISPERSED_ASIDE, G, spos,
+                                         next, stop);
+        if (walk && dispersed == DISPERSED_ASIDE) continue;
+        if (LIST && range == 32u && (warp & 15u) == 0u)
+            count_buckets(list, fg_stage_cell(__ldg(spos + min(it.first + q0 + lane, hi - 1u)), G), G);
         while (next < stop) {
             const uint32_t i = next + lane; /* sorted index */
             uint32_t n = min(32u, stop - next);
@@ -313,13 +320,14 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
     tally.flush<LIST, COUNT>(list, pairs);
 }
 
-/* The dispersed ranges, a thread a target.  Bound by the L1's and L2's sectors
- * (54 bucket words a target) and their latency, for which it wants the L1 and
- * the warps that the staging kernel's shared memory takes: the same walk there
- * takes 270 us where this takes 226, at 1,048,576 targets 1.2 h apart (staged:
- * 477).  Eight CTAs an SM, 62 registers, without lists (sixteen of 32, which
- * spill: 262 us), ten with them.  A wave of CTAs; the next range's positions
- * are on their way while one walks or is passed over. */
+/* The dispersed ranges (most = 0: every range), a thread a target.  Bound by
+ * the L1's and L2's sectors (54 bucket words a target) and their latency, for
+ * which it wants the L1 and the warps that the staging kernel's shared memory
+ * takes: the same walk there takes 270 us where this takes 226, at 1,048,576
+ * targets 1.2 h apart (staged: 477).  Eight CTAs an SM, 62 registers, without
+ * lists (sixteen of 32, which spill: 262 us), ten with them.  A wave of CTAs;
+ * the next range's positions are on their way while one walks or is passed
+ * over. */
 #define FG_WALK_CTAS(LIST) ((LIST) ? 10 : 8)
 template <bool LIST, bool COUNT>
 __global__ void __launch_bounds__(FG_CHUNK, FG_WALK_CTAS(LIST)) k_density_dispersed(
@@ -344,8 +352,13 @@ __global__ void __launch_bounds__(FG_CHUNK, FG_WALK_CTAS(LIST)) k_density_disper
         const float4 p = ahead;
         if (w + gridDim.x < nwork) ahead = load(w + gridDim.x);
         if ((threadIdx.x & ~31u) >= it.count) continue; /* uniform over the warp */
-        const StageGrid G(S);
-        if (!fg_stage_dispersed(fg_stage_cell(p, G), G, 32u, most)) continue;
+        if (most) {
+            const StageGrid G(S);
+            if (!fg_stage_dispersed(fg_stage_cell(p, G), G, 32u, most)) continue;
+        } else if (LIST && threadIdx.x < 32u && (w & 3u) == 0u) {
+            const StageGrid G(S);
+            count_buckets(list, fg_stage_cell(p, G), G);
+        }
         if (threadIdx.x < it.count) {
             const uint32_t i = it.first + threadIdx.x;
             const bool active = p.w > 0.0f;
@@ -380,14 +393,16 @@ static uint32_t stage_range(uint32_t nwork)
  * 67.  Nine parts the first two: with eight, the few ranges of the first that
  * walk take it to 326; with twelve, the second stays at 326.  With L.side the
  * walk is a kernel beside the staging one (3 us where no range walks); warps
- * of fewer targets, of which the GPU is not full, walk themselves. */
-static int dispersed_ranges(const Launch &L, uint32_t range, bool count, uint32_t &most)
+ * of fewer targets, of which the GPU is not full, walk themselves.  A world with
+ * lists chooses for all its ranges at once (World::check_list_cap): there the
+ * walk of a few ranges, 27 rows and a list one after another, lasts as long as
+ * the whole pass (32 uneven splashed scenes, an eighth of the ranges dispersed:
+ * 298 us a step staged, 354 with those walked). */
+static int dispersed_ranges(const Launch &L, uint32_t range, uint32_t &most)
 {
+    most = 32u;
+    if (!L.side.stream) return DISPERSED_STAGED;
     most = range == 32u ? 9u : range - range / 4u;
-    if (!L.side.stream) {
-        if (!count || range < 32u) most = 32u;
-        return DISPERSED_STAGED;
-    }
     return range == 32u ? DISPERSED_ASIDE : DISPERSED_WALKED;
 }
 
@@ -396,7 +411,7 @@ bool density_ranges_wide(uint32_t nwork) { return stage_range(nwork) == 32u; }
 uint32_t density_launches(const Launch &L)
 {
     uint32_t most;
-    return dispersed_ranges(L, stage_range(L.nwork), false, most) == DISPERSED_ASIDE ? 2u : 1u;
+    return dispersed_ranges(L, stage_range(L.nwork), most) == DISPERSED_ASIDE ? 2u : 1u;
 }
 
 /* L.side's stream, if it is used: forked from L's until the end of the scope. */
@@ -426,25 +441,36 @@ void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, 
     memset(&none, 0, sizeof(none));
     const NbrList &nl = list ? *list : none;
     const DensityConst C = {gas_o, rest_o, mass_o, use_o};
+    if (list && L.walk) {
+        k_density_dispersed<true, true><<<grid_for(L.nwork, FG_WALK_CTAS(true)), FG_CHUNK, 0, L.stream>>>(
+            L.work, L.nwork, L.n, L.table, *L.single, 0u, spos, svel, start, end, dp, C, nl, pairs);
+        return;
+    }
     const uint32_t range = stage_range(L.nwork);
     uint32_t most;
-    const int dispersed = dispersed_ranges(L, range, nl.dispersed != nullptr, most);
+    const int dispersed = dispersed_ranges(L, range, most);
     /* ctas_per_sm counts CTAs of FG_CHUNK threads for 32 targets a warp */
     const uint32_t per = FG_CHUNK / range * 32u / FG_DENSITY_THREADS;
     const uint32_t g = grid_for(L.nwork * per, (int)((L.ctas_per_sm ? L.ctas_per_sm : 64u) * per));
 #define FG_DENSITY(LI, CO)                                                                                          \
-    do {                                                                                                            \
-        const SideLaunch side(L, dispersed == DISPERSED_ASIDE);                                                     \
-        if (side.use)                                                                                               \
-            k_density_dispersed<LI, CO><<<grid_for(L.nwork, FG_WALK_CTAS(LI)), FG_CHUNK, 0, L.side.stream>>>(       \
-                L.work, L.nwork, L.n, L.table, *L.single, most, spos, svel, start, end, dp, C, nl, pairs);          \
-        k_density<LI, CO><<<g, FG_DENSITY_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, range,  \
-                                                                  most, dispersed, spos, svel, start, end, dp, C,   \
-                                                                  nl, pairs);                                       \
-    } while (0)
-    if (list) FG_DENSITY(true, true);
-    else if (pairs) FG_DENSITY(false, true);
-    else FG_DENSITY(false, false);
+    k_density<LI, CO><<<g, FG_DENSITY_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, range, most, \
+                                                              dispersed, spos, svel, start, end, dp, C, nl, pairs)
+    if (list) {
+        FG_DENSITY(true, true);
+        return;
+    }
+    const SideLaunch side(L, dispersed == DISPERSED_ASIDE);
+#define FG_DISPERSED(CO)                                                                                            \
+    k_density_dispersed<false, CO><<<grid_for(L.nwork, FG_WALK_CTAS(false)), FG_CHUNK, 0, L.side.stream>>>(         \
+        L.work, L.nwork, L.n, L.table, *L.single, most, spos, svel, start, end, dp, C, nl, pairs)
+    if (pairs) {
+        if (side.use) FG_DISPERSED(true);
+        FG_DENSITY(false, true);
+    } else {
+        if (side.use) FG_DISPERSED(false);
+        FG_DENSITY(false, false);
+    }
+#undef FG_DISPERSED
 #undef FG_DENSITY
 }
 
@@ -908,7 +934,7 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
         const uint32_t range = stage_range(L.nwork), warps = (L.n + range - 1u) / range;
         const uint32_t ctas = grid_for((warps + FG_FORCE_THREADS / 32u - 1u) / (FG_FORCE_THREADS / 32u), 128);
         uint32_t most;
-        const int dispersed = dispersed_ranges(L, range, false, most);
+        const int dispersed = dispersed_ranges(L, range, most);
         const SideLaunch side(L, dispersed == DISPERSED_ASIDE);
         if (side.use)
             k_forces_dispersed<<<grid_for(L.nwork, FG_WALK_FORCE_CTAS), FG_CHUNK, 0, L.side.stream>>>(

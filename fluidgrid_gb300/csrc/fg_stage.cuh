@@ -115,15 +115,23 @@ __device__ __forceinline__ StageCell fg_stage_cell(float4 p, const StageGrid &G)
     return c;
 }
 
-/* Whether the targets of a range, a lane each (past the scene's end its last
- * one's), are more than `most` and lie in more buckets: a function of the range
- * alone, so that two kernels that share the ranges agree on it.  (Buckets, not
- * cells: where many cells share a bucket, the candidates are many too.) */
-__device__ __forceinline__ bool fg_stage_dispersed(const StageCell &c, const StageGrid &G, uint32_t len, uint32_t most)
+/* Buckets of a range of len targets, a lane each (past the scene's end its
+ * last one's).  Buckets, not cells: where many cells share a bucket, the
+ * candidates are many too. */
+__device__ __forceinline__ uint32_t fg_stage_buckets(const StageCell &c, const StageGrid &G, uint32_t len)
 {
     const uint32_t b = fg_bucket((uint32_t)c.x * FG_PX, (uint32_t)c.y * FG_PY, (uint32_t)c.z * FG_PZ, G.nb, G.mask);
     const uint32_t lane = threadIdx.x & 31u, before = __shfl_up_sync(FG_FULL, b, 1);
-    return (uint32_t)__popc(__ballot_sync(FG_FULL, lane < len && (lane == 0u || b != before))) > most &&
+    return (uint32_t)__popc(__ballot_sync(FG_FULL, lane < len && (lane == 0u || b != before)));
+}
+
+/* Whether its active targets are more than `most` and its buckets too: a
+ * function of the range alone, so that two kernels that share the ranges agree
+ * on it. */
+__device__ __forceinline__ bool fg_stage_dispersed(const StageCell &c, const StageGrid &G, uint32_t len, uint32_t most)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    return most < 32u && fg_stage_buckets(c, G, len) > most &&
            (uint32_t)__popc(__ballot_sync(FG_FULL, lane < len && c.active)) > most;
 }
 
@@ -153,7 +161,7 @@ __device__ __forceinline__ bool fg_stage_range(uint32_t b, uint32_t len, uint32_
     const StageCell mine = cell(b + lane);
     first = b;
     stop = b + own;
-    const bool dispersed = most < 32u && fg_stage_dispersed(mine, G, len, most);
+    const bool dispersed = fg_stage_dispersed(mine, G, len, most);
     if (dispersed && apart) return true;
     if (b > lo) {
         const StageCell e = cell(b - len + lane);
