@@ -197,9 +197,10 @@ int radix_passes(uint32_t bits, uint32_t digit_bits)
 /* The lanes of the warp whose digit (of `bits` bits) is the same: a ballot a
  * bit.  match_any takes a round for each distinct value of the warp: with it
  * the downsweep of 700,000 random pairs took 11.4 us, with the ballots 9.2; but
- * of keys in runs, as those of a fluid are, a sort of 1,000,000 (32 bits) took
- * 98 us with match_any, 106 with the ballots, and takes 97 choosing by the
- * warp's runs (a lattice's keys 102, 106, 99; random ones 123, 115, 115). */
+ * of keys in runs, as those of a fluid are, a sort of 4,000,000 (21 bits) took
+ * 187 us with match_any, 173 with the ballots, and takes 156 choosing by the
+ * runs of a warp's first keys (a lattice's keys 198, 174, 169; random ones 228,
+ * 178, 180; 700,000 of these, chosen key by key, 83 instead of 82). */
 __device__ __forceinline__ uint32_t rs_peers(uint32_t d, uint32_t bits)
 {
     uint32_t peers = 0xffffffffu;
@@ -324,25 +325,28 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_downsweep(const uint32_t *__r
         key[k] = i < n ? __ldg(kin + i) : 0xffffffffu;
         val[k] = i < n ? (vin ? __ldg(vin + i) : (uint32_t)i) : 0u;
     }
+    /* up to nine runs of equal digits in the warp's first 32: match_any, a round a digit */
+    const uint32_t d0 = (key[0] >> shift) & mask;
+    const bool few = (uint32_t)__popc(__ballot_sync(0xffffffffu, d0 != __shfl_up_sync(0xffffffffu, d0, 1))) < 9u;
+    auto rank_all = [&](auto &&peers_of) {
 #pragma unroll
-    for (int k = 0; k < RS_ITEMS; k++) {
-        const bool valid = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane < n;
-        const uint32_t d = (key[k] >> shift) & mask;
-        const uint32_t act = __ballot_sync(0xffffffffu, valid);
-        /* up to nine runs of equal digits: match_any, a round a digit */
-        const uint32_t before = __shfl_up_sync(0xffffffffu, d, 1);
-        const bool few = (uint32_t)__popc(__ballot_sync(0xffffffffu, d != before)) < 9u;
-        const uint32_t peers = (few ? __match_any_sync(0xffffffffu, d) : rs_peers(d, bits)) & act;
-        const uint32_t leader = valid ? (uint32_t)__ffs((int)peers) - 1u : lane;
-        uint32_t b = 0;
-        if (valid && lane == leader) {
-            b = s_whist[wid][d];
-            s_whist[wid][d] = b + __popc(peers);
+        for (int k = 0; k < RS_ITEMS; k++) {
+            const bool valid = base + (size_t)wid * (32 * RS_ITEMS) + (size_t)k * 32 + lane < n;
+            const uint32_t d = (key[k] >> shift) & mask;
+            const uint32_t peers = peers_of(d) & __ballot_sync(0xffffffffu, valid);
+            const uint32_t leader = valid ? (uint32_t)__ffs((int)peers) - 1u : lane;
+            uint32_t b = 0;
+            if (valid && lane == leader) {
+                b = s_whist[wid][d];
+                s_whist[wid][d] = b + __popc(peers);
+            }
+            b = __shfl_sync(0xffffffffu, b, (int)leader);
+            rank[k] = b + __popc(peers & lt);
+            __syncwarp();
         }
-        b = __shfl_sync(0xffffffffu, b, (int)leader);
-        rank[k] = b + __popc(peers & lt);
-        __syncwarp();
-    }
+    };
+    if (few) rank_all([](uint32_t d) { return __match_any_sync(0xffffffffu, d); });
+    else rank_all([bits](uint32_t d) { return rs_peers(d, bits); });
     __syncthreads();
     /* per digit: exclusive over warps, tile count */
     uint32_t run = 0;
