@@ -312,7 +312,6 @@ int World::reserve(const Capacity &c)
     k_set_u32<<<1, 1, 0, stream>>>(list_cap_d, list_cap);
     nbr.max_count = max_count;
     nbr.overflow = overflow_counter;
-    nbr.spread = max_count + 2;
     CK(cudaMemsetAsync(dp, 0, 8 * N, stream));
     CK(cudaMemsetAsync(vel, 0, 16 * N, stream));
     CK(cudaMemsetAsync(end, 0, 4 * NB, stream));
@@ -717,7 +716,9 @@ void World::enqueue_fluid_contact(cudaStream_t st, uint32_t &launches)
     if (!fluid_contact_pass()) return;
     Launch Lf = fluid_launch();
     Lf.stream = st;
-    launch_fluid_contact(Lf, pos, vel, body_grid(), fcontact);
+    bool narrow = false; /* some scene's search */
+    for (const FgScene &S : scenes_h) narrow |= S.nbodies && contact_narrow(S.f2r_rel);
+    launch_fluid_contact(Lf, pos, vel, body_grid(), fcontact, narrow);
     launches++;
 }
 
@@ -1156,10 +1157,11 @@ int World::check_list_cap()
 {
     const bool grow = step_count % FG_LIST_CHECK_PERIOD == 0;
     uint32_t seen[4]; /* largest count, the capacity, buckets and number of the ranges counted */
+    CK(cudaMemsetAsync(max_count + 2, 0, 8, stream));
+    if (density_ranges_wide(nwork)) launch_spread(fluid_launch(), spos, max_count + 2);
     CK(cudaMemcpyAsync(seen, max_count, sizeof(seen), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    CK(cudaMemsetAsync(nbr.spread, 0, 8, stream));
-    density_walks = density_ranges_wide(nwork) && 2ull * seen[2] > 15ull * seen[3];
+    density_walks = 2ull * seen[2] > 15ull * seen[3];
     if (!grow) return FG_OK;
     CK(cudaMemsetAsync(max_count, 0, 4, stream));
     const uint32_t mx = seen[0];

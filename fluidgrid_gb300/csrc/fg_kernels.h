@@ -148,9 +148,11 @@ struct NbrList {
     const uint32_t *cap;          /* device word: entries a target may store (<= stride) */
     uint32_t *max_count;          /* optional: atomicMax of cnt */
     unsigned long long *overflow; /* optional: targets with cnt > cap */
-    uint32_t *spread;             /* optional: += the buckets of every sixteenth range of 32, and 1 */
 };
 
+/* adds the buckets that every sixteenth range of 32 sorted targets lies in, and
+ * the number of those ranges, to out[0] and out[1] */
+void launch_spread(const Launch &L, const float4 *spos, uint32_t *out);
 /* whether a density pass over nwork items takes ranges of 32 targets, whose
  * dispersed ones can go to a kernel of their own */
 bool density_ranges_wide(uint32_t nwork);
@@ -195,7 +197,9 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * (ProcessCollisionForcesD).  The force pass then
  * reads it (G.pre). */
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out,
-                          const uint32_t *ids = nullptr);
+                          bool narrow, const uint32_t *ids = nullptr);
+/* whether a search half-width is one of up to 27 buckets */
+bool contact_narrow(const int rel[3]);
 
 void launch_integrate(const Launch &L, float4 *pos, const float4 *vel);
 

@@ -202,16 +202,6 @@ __device__ __noinline__ uint2 density_walk_aside(const FgScene *S, uint32_t i, c
     return make_uint2(__float_as_uint(acc.sum()), acc.cnt);
 }
 
-/* A range's buckets, for the host (every sixteenth range of 32). */
-__device__ __forceinline__ void count_buckets(const NbrList &list, const StageCell &c, const StageGrid &G)
-{
-    const uint32_t b = fg_stage_buckets(c, G, 32u);
-    if (list.spread && (threadIdx.x & 31u) == 0u) {
-        atomicAdd(list.spread, b);
-        atomicAdd(list.spread + 1, 1u);
-    }
-}
-
 /* What a pass does with its dispersed ranges: those of more than `most`
  * buckets, whose targets share too little for a lookup and a cull a cell. */
 enum { DISPERSED_STAGED, DISPERSED_WALKED, DISPERSED_ASIDE /* another kernel has them */ };
@@ -244,8 +234,6 @@ __global__ void __launch_bounds__(FG_DENSITY_THREADS, FG_DENSITY_CTAS) k_density
         const bool walk = fg_stage_range(it.first + q0, range, lo, hi, most, dispersed == DISPERSED_ASIDE, G, spos,
                                          next, stop);
         if (walk && dispersed == DISPERSED_ASIDE) continue;
-        if (LIST && range == 32u && (warp & 15u) == 0u)
-            count_buckets(list, fg_stage_cell(__ldg(spos + min(it.first + q0 + lane, hi - 1u)), G), G);
         while (next < stop) {
             const uint32_t i = next + lane; /* sorted index */
             uint32_t n = min(32u, stop - next);
@@ -355,9 +343,6 @@ __global__ void __launch_bounds__(FG_CHUNK, FG_WALK_CTAS(LIST)) k_density_disper
         if (most) {
             const StageGrid G(S);
             if (!fg_stage_dispersed(fg_stage_cell(p, G), G, 32u, most)) continue;
-        } else if (LIST && threadIdx.x < 32u && (w & 3u) == 0u) {
-            const StageGrid G(S);
-            count_buckets(list, fg_stage_cell(p, G), G);
         }
         if (threadIdx.x < it.count) {
             const uint32_t i = it.first + threadIdx.x;
@@ -373,6 +358,33 @@ __global__ void __launch_bounds__(FG_CHUNK, FG_WALK_CTAS(LIST)) k_density_disper
         __syncwarp();
     }
     tally.flush<LIST, COUNT>(list, pairs);
+}
+
+/* out[0] += the buckets of every sixteenth range of 32, out[1] += 1 for each. */
+__global__ void __launch_bounds__(FG_CHUNK) k_spread(const FgWork *__restrict__ work, uint32_t nwork, uint32_t n_single,
+                                                     const FgScene *__restrict__ table,
+                                                     const __grid_constant__ FgScene single,
+                                                     const float4 *__restrict__ spos, uint32_t *out)
+{
+    for (uint32_t w = 4u * (blockIdx.x * (FG_CHUNK / 32u) + (threadIdx.x >> 5)); w < nwork;
+         w += 4u * gridDim.x * (FG_CHUNK / 32u)) {
+        const FgWork it = fg_work(work, w, n_single);
+        const FgScene *S = fg_scene(table, &single, it.scene);
+        const uint32_t hi = table ? S->pbase + S->n : n_single, lane = threadIdx.x & 31u;
+        const StageGrid G(S);
+        const uint32_t b = fg_stage_buckets(fg_stage_cell(__ldg(spos + min(it.first + lane, hi - 1u)), G), G, 32u);
+        if (lane == 0u) {
+            atomicAdd(out, b);
+            atomicAdd(out + 1, 1u);
+        }
+    }
+}
+
+void launch_spread(const Launch &L, const float4 *spos, uint32_t *out)
+{
+    if (!L.nwork) return;
+    k_spread<<<grid_for((L.nwork + 15u) / 16u, 16), FG_CHUNK, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single,
+                                                                             spos, out);
 }
 
 /* Targets of a warp: 32, or fewer where that leaves the SMs short of warps
@@ -500,20 +512,21 @@ __device__ __forceinline__ float3 force_contact(const FgScene *S, uint32_t scene
     return make_float3(q.x, q.y, q.z);
 }
 
+/* The contact that the contact pass stored for particle oi, if it is marked. */
+__device__ __forceinline__ float3 force_contact_stored(const FgScene *S, bool active, float4 p, const RigidGrid &G,
+                                                       uint32_t oi)
+{
+    if (!active || !fg_contact_marked(S, 0u, p, G)) return make_float3(0.f, 0.f, 0.f);
+    const float4 q = __ldcg(G.pre + oi); /* the output's memory */
+    return make_float3(q.x, q.y, q.z);
+}
+
 /* The contact of a warp's particles (whole warp, converged) with a grid whose
- * near cells are marked: read from particle oi's place where the contact pass
- * stored it, else one particle after another by the whole warp. */
+ * near cells are marked, one particle after another by the whole warp. */
 __device__ __forceinline__ float3 force_contact_warp(const FgScene *S, bool active, float4 p, float4 v,
-                                                     const RigidGrid &G, bool dynamic, uint32_t oi)
+                                                     const RigidGrid &G, bool dynamic)
 {
     float3 c = make_float3(0.f, 0.f, 0.f);
-    if (G.pre) {
-        if (active && fg_contact_marked(S, 0u, p, G)) {
-            const float4 q = __ldcg(G.pre + oi);
-            c = make_float3(q.x, q.y, q.z);
-        }
-        return c;
-    }
     const ContactShape C(S);
     for (uint32_t m = __ballot_sync(FG_FULL, active && fg_contact_marked(S, 0u, p, G)); m; m &= m - 1u) {
         const int b = __ffs((int)m) - 1;
@@ -525,6 +538,18 @@ __device__ __forceinline__ float3 force_contact_warp(const FgScene *S, bool acti
         if ((int)(threadIdx.x & 31u) == b) c = r;
     }
     return c;
+}
+
+/* The launchers' contact: one grid's from the contact pass, and the static
+ * one's searched here where that was the dynamic's. */
+__device__ __forceinline__ void force_contacts(const FgScene *S, bool active, float4 p, float4 v, uint32_t oi,
+                                               const RigidArgs &R, float3 &sta, float3 &dyn)
+{
+    sta = dyn = make_float3(0.f, 0.f, 0.f);
+    if (R.use_dyn) dyn = force_contact_stored(S, active, p, R.dyn, oi);
+    if (R.use_sta)
+        sta = R.use_dyn ? force_contact_warp(S, active, p, v, R.sta, false)
+                        : force_contact_stored(S, active, p, R.sta, oi);
 }
 
 /* Pair terms of one target by a walk over its 27 buckets. */
@@ -547,6 +572,16 @@ __device__ __forceinline__ void walk_terms(const FgScene *S, uint32_t i, float4 
             fg_pair(fx, fy, fz, dx, dy, dz, r2, h, kspiky, kv, di.x, di.y, v, dj.x, dj.y, vj);
         }
     });
+}
+
+/* The same out of line, for the search kernel's few. */
+__device__ __noinline__ float3 walk_terms_aside(const FgScene *S, uint32_t i, float kv, const float4 *spos,
+                                                const float4 *svel, const float2 *dp, const uint32_t *start,
+                                                const uint32_t *end)
+{
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    walk_terms(S, i, __ldg(spos + i), __ldg(svel + i), kv, spos, svel, dp, start, end, f.x, f.y, f.z);
+    return f;
 }
 
 /* From the summed pair terms to the particle's new velocity (and, fused, its
@@ -874,12 +909,14 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
                         }
                     });
             }
-            if (active && (sig.odd || walk)) walk_terms(S, i, p, v, kv, spos, svel, dp, start, end, fx, fy, fz);
+            if (active && (sig.odd || walk)) {
+                const float3 f = walk_terms_aside(S, i, kv, spos, svel, dp, start, end);
+                fx = f.x; fy = f.y; fz = f.z;
+            }
             __syncwarp();
             const uint32_t oi = valid ? __ldg(ids + i) : 0u;
-            float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
-            if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false, oi);
-            if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true, oi);
+            float3 sta, dyn;
+            force_contacts(S, active, p, v, oi, R, sta, dyn);
             if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, oi, vel_out, pos_out);
         }
     }
@@ -912,9 +949,8 @@ __global__ void __launch_bounds__(FG_CHUNK, FG_WALK_FORCE_CTAS) k_forces_dispers
         if (active) walk_terms(S, i, p, v, S->kvisc * visc, spos, svel, dp, start, end, fx, fy, fz);
         __syncwarp();
         const uint32_t oi = valid ? __ldg(ids + i) : 0u;
-        float3 sta = make_float3(0.f, 0.f, 0.f), dyn = sta;
-        if (R.use_sta) sta = force_contact_warp(S, active, p, v, R.sta, false, oi);
-        if (R.use_dyn) dyn = force_contact_warp(S, active, p, v, R.dyn, true, oi);
+        float3 sta, dyn;
+        force_contacts(S, active, p, v, oi, R, sta, dyn);
         if (valid) force_finish(S, p, v, fx, fy, fz, mass, sta, dyn, oi, vel_out, pos_out);
         __syncwarp();
     }
@@ -989,8 +1025,10 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * leave most of a warp's lanes idle, are walked by thread: a step of 131,072
  * particles with 4,096 spheres among all of them 209 -> 170 us, 32,768 spheres
  * 272 -> 240; surfaces stay below it.  (Half-widths of 2 and more: 257 us walked
- * and 245 searched with 1,024 spheres, 437 and 353 with 32,768.) */
+ * and 245 searched with 1,024 spheres, 437 and 353 with 32,768.)  Its registers
+ * cost the other half-widths 3%, so they have a kernel without it. */
 #define FG_CONTACT_SEARCHES 80u
+template <bool WALK27>
 __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWork *__restrict__ work, uint32_t nwork,
                                                            uint32_t n_single, const FgScene *__restrict__ table,
                                                            const __grid_constant__ FgScene single,
@@ -1024,7 +1062,7 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
         __syncthreads();
         const ContactShape C(S);
         const bool dynamic = G.body_vel != nullptr;
-        if (C.total <= 27u && s_n > FG_CONTACT_SEARCHES) {
+        if (WALK27 && C.total <= 27u && s_n > FG_CONTACT_SEARCHES) {
             if (threadIdx.x < s_n) {
                 const uint32_t id = s_id[threadIdx.x];
                 const float3 c = fg_fluid_rigid_contact(S, it.scene, __ldg(pos + id), __ldg(vel + id), G, dynamic);
@@ -1043,14 +1081,24 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
 }
 
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out,
-                          const uint32_t *ids)
+                          bool narrow, const uint32_t *ids)
 {
     if (!L.nwork) return;
     /* an SM's worth of CTAs: a CTA per item queues ahead of the grid kernels
      * beside this one (64 worlds after 400 steps 896 us a step, here 883; 4M
      * particles 2163, here 2135) */
-    k_fluid_contact<<<grid_for(L.nwork, 8), FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos, vel,
-                                                                  G, ids, out);
+    const uint32_t g = grid_for(L.nwork, 8);
+    if (narrow)
+        k_fluid_contact<true><<<g, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos,
+                                                                      vel, G, ids, out);
+    else
+        k_fluid_contact<false><<<g, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos,
+                                                                       vel, G, ids, out);
+}
+
+bool contact_narrow(const int rel[3])
+{
+    return (2 * rel[0] + 1) * (2 * rel[1] + 1) * (2 * rel[2] + 1) <= 27;
 }
 
 /* SPHIntegrateK (K_FluidSim.cu:418-438): pos += vel*(dt/scale) for active
