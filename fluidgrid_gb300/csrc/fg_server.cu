@@ -53,16 +53,23 @@ namespace fg {
 /* Host memory of particle states, kept for the next requests: fresh pages cost
  * more to touch than to copy into (16 MB: 1.0 ms against 0.6).  Shared by a
  * server and the results handed out, so any thread may give an array back; at
- * most FG_SERVER_SPARE_BYTES are kept, and they go with the last owner. */
+ * most FG_SERVER_SPARE_BYTES are kept, and they go with the server: a result
+ * that outlives it holds its own array only. */
 #define FG_SERVER_SPARE_BYTES ((size_t)256 << 20)
 struct HostPool {
     std::mutex mu;
     std::vector<std::pair<size_t, float *>> spare; /* floats, array */
     size_t bytes = 0;
+    bool open = true;
 
-    ~HostPool()
+    ~HostPool() { close(); }
+    void close()
     {
+        std::lock_guard<std::mutex> lock(mu);
+        open = false;
         for (auto &s : spare) free(s.second);
+        spare.clear();
+        bytes = 0;
     }
     /* an array of at least n floats, not initialised (nullptr: no memory) */
     float *take(size_t n, size_t &cap)
@@ -90,7 +97,7 @@ struct HostPool {
     {
         {
             std::lock_guard<std::mutex> lock(mu);
-            if (bytes + sizeof(float) * cap <= FG_SERVER_SPARE_BYTES && spare.size() < spare.capacity()) {
+            if (open && bytes + sizeof(float) * cap <= FG_SERVER_SPARE_BYTES && spare.size() < spare.capacity()) {
                 bytes += sizeof(float) * cap;
                 spare.push_back({cap, p});
                 return;
@@ -186,6 +193,7 @@ struct Server {
     }
     ~Server()
     {
+        pool->close();
         w.reset();
         for (int k = 0; k < FG_SERVER_RING; k++) {
             if (ev0[k]) cudaEventDestroy(ev0[k]);
