@@ -25,7 +25,7 @@ struct Launch {
     uint32_t n;            /* particles (single-scene mode) */
     cudaStream_t stream;
     uint32_t ctas_per_sm;  /* density/force grids: CTAs of FG_CHUNK threads per SM (0 = 64) */
-    uint32_t block;        /* density/force grids: threads per CTA, 64, 128 or 256 (0 = FG_CHUNK) */
+    uint32_t block;        /* force grid: threads per CTA, 64, 128 or 256 (0 = FG_CHUNK) */
     SideStream side;       /* a pass without lists: its dispersed ranges go to a kernel of their own there, or {} */
     bool walk;             /* density with lists: every target walks by thread */
 };
@@ -119,9 +119,8 @@ void launch_rb_sort_ranges(const FgScene *table, const FgScene *single, uint32_t
 void launch_morton_keys(const Launch &L, const float4 *pos, uint32_t *keys, uint32_t bits, uint32_t scene_shift);
 
 
-/* Target order of the density/force passes: target slot t processes the
- * particle tord[t] (a particle id, scene-contiguous), found in sorted order
- * at inv[tord[t]].  tord == nullptr: slot t is sorted index t. */
+/* Target order of the force pass: target slot t processes the particle tord[t]
+ * (a particle id, scene-contiguous), found in sorted order at inv[tord[t]].  tord == nullptr: slot t is sorted index t. */
 struct TargetOrder {
     const uint32_t *tord;
     const uint32_t *inv;
@@ -134,9 +133,9 @@ struct TargetOrder {
  * duplicate bucket visits kept) in the bucket walk's order; the force pass
  * skips j == i.  Target slot t owns idx[t * stride, (t + 1) * stride) and
  * stores at most cap entries there; cap lives in device memory, so the host
- * changes it between steps without touching a captured graph.  The density pass writes two entries (8 bytes) at a time,
- * so a 32-byte sector is completed by four stores of one thread rather than
- * eight scattered 4-byte ones; the force pass reads four at a time.
+ * changes it between steps without touching a captured graph.  The density pass
+ * writes a sector of eight entries at a time (its walk two entries); the force
+ * pass reads four at a time.
  * cnt[t] may exceed cap; then the force pass re-walks the buckets.
  * rec[2i] = (x, y, z, rho_i), rec[2i+1] = (vx, vy, vz, P_i): one 32-byte
  * sector per neighbour gather. */

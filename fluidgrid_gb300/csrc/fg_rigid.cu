@@ -318,7 +318,8 @@ __device__ __forceinline__ void body_integrate(const FgScene *S, uint32_t b, dou
     if (lane < 9u) W.Tm[e] = W.R[3u * r] * I[k] + W.R[3u * r + 1u] * I[3u + k] + W.R[3u * r + 2u] * I[6u + k];
     __syncwarp();
     if (lane < 9u)
-        W.G[e] = W.Tm[3u * r] * W.R[3u * k] + W.Tm[3u * r + 1u] * W.R[3u * k + 1u] + W.Tm[3u * r + 2u] * W.R[3u * k + 2u];
+        W.G[e] = W.Tm[3u * r] * W.R[3u * k] + W.Tm[3u * r + 1u] * W.R[3u * k + 1u] +
+                 W.Tm[3u * r + 2u] * W.R[3u * k + 2u];
     __syncwarp();
     if (lane < 4u)
         W.om[c] = c < 3u ? W.G[3u * c] * W.L[0] + W.G[3u * c + 1u] * W.L[1] + W.G[3u * c + 2u] * W.L[2] : 0.0;
@@ -376,7 +377,8 @@ __global__ void __launch_bounds__(BODY_THREADS) k_body_update(const FgScene *__r
             v = body_sum_cta(body_first[b], 0u, body_count[b], force, torque, s_red);
         }
         if (threadIdx.x < 32) {
-            if (threadIdx.x < 8) ((double *)((threadIdx.x < 4 ? st.force_sum : st.torque_sum) + b))[threadIdx.x & 3] = v;
+            FgD4 *const sum = threadIdx.x < 4 ? st.force_sum : st.torque_sum;
+            if (threadIdx.x < 8) ((double *)(sum + b))[threadIdx.x & 3] = v;
             const double T = __shfl_sync(0xffffffffu, v, (threadIdx.x & 3) + 4);
             const double F = __shfl_sync(0xffffffffu, v, threadIdx.x & 3);
             /* mass 0: a static body (the reference's "static" rigid-body
@@ -398,7 +400,8 @@ void launch_body_update(const FgScene *table, const FgScene *single, const uint3
                                                                             st.partial);
     else
         st.partial = nullptr;
-    k_body_update<<<grid_for(nbodies, st.partial ? 16 : 4), st.partial ? 32 : BODY_THREADS, 0, s>>>(table, *single, body_scene, body_first, body_count,
+    const int per_sm = st.partial ? 16 : 4, threads = st.partial ? 32 : BODY_THREADS;
+    k_body_update<<<grid_for(nbodies, per_sm), threads, 0, s>>>(table, *single, body_scene, body_first, body_count,
                                                                 nbodies, force, torque, st, integrate);
 }
 

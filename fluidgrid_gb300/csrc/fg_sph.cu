@@ -426,15 +426,20 @@ uint32_t density_launches(const Launch &L)
     return dispersed_ranges(L, stage_range(L.nwork), most) == DISPERSED_ASIDE ? 2u : 1u;
 }
 
-/* L.side's stream, if it is used: forked from L's until the end of the scope. */
+/* L.side's stream, if it is used: forked from L's until the end of the scope.
+ * Where that fails (a context made anew under the process) one kernel takes
+ * every range. */
 struct SideLaunch {
     const Launch &L;
-    const bool use;
-    SideLaunch(const Launch &launch, bool fork) : L(launch), use(fork)
+    bool use;
+    SideLaunch(const Launch &launch, int &dispersed) : L(launch), use(dispersed == DISPERSED_ASIDE)
     {
-        if (!use) return;
-        cudaEventRecord(L.side.fork, L.stream);
-        cudaStreamWaitEvent(L.side.stream, L.side.fork, 0);
+        if (!use || (cudaEventRecord(L.side.fork, L.stream) == cudaSuccess &&
+                     cudaStreamWaitEvent(L.side.stream, L.side.fork, 0) == cudaSuccess))
+            return;
+        cudaGetLastError();
+        use = false;
+        dispersed = DISPERSED_WALKED;
     }
     ~SideLaunch()
     {
@@ -460,7 +465,7 @@ void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, 
     }
     const uint32_t range = stage_range(L.nwork);
     uint32_t most;
-    const int dispersed = dispersed_ranges(L, range, most);
+    int dispersed = dispersed_ranges(L, range, most);
     /* ctas_per_sm counts CTAs of FG_CHUNK threads for 32 targets a warp */
     const uint32_t per = FG_CHUNK / range * 32u / FG_DENSITY_THREADS;
     const uint32_t g = grid_for(L.nwork * per, (int)((L.ctas_per_sm ? L.ctas_per_sm : 64u) * per));
@@ -471,7 +476,7 @@ void launch_density(const Launch &L, const float4 *spos, const uint32_t *start, 
         FG_DENSITY(true, true);
         return;
     }
-    const SideLaunch side(L, dispersed == DISPERSED_ASIDE);
+    const SideLaunch side(L, dispersed);
 #define FG_DISPERSED(CO)                                                                                            \
     k_density_dispersed<false, CO><<<grid_for(L.nwork, FG_WALK_CTAS(false)), FG_CHUNK, 0, L.side.stream>>>(         \
         L.work, L.nwork, L.n, L.table, *L.single, most, spos, svel, start, end, dp, C, nl, pairs)
@@ -782,9 +787,10 @@ struct ForceShared {
 
 __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_search(
     uint32_t n_all, const __grid_constant__ FgScene scene, uint32_t range, uint32_t most, int dispersed,
-    const float4 *__restrict__ spos, const float4 *__restrict__ svel, const float2 *__restrict__ dp, const uint32_t *__restrict__ start,
-    const uint32_t *__restrict__ end, const uint32_t *__restrict__ ids, float4 *__restrict__ vel_out,
-    float4 *__restrict__ pos_out, const __grid_constant__ RigidArgs R, float mass, float visc)
+    const float4 *__restrict__ spos, const float4 *__restrict__ svel, const float2 *__restrict__ dp,
+    const uint32_t *__restrict__ start, const uint32_t *__restrict__ end, const uint32_t *__restrict__ ids,
+    float4 *__restrict__ vel_out, float4 *__restrict__ pos_out, const __grid_constant__ RigidArgs R, float mass,
+    float visc)
 {
     __shared__ ForceShared shared[FG_FORCE_THREADS / 32];
     ForceShared &sm = shared[threadIdx.x >> 5];
@@ -898,8 +904,9 @@ __global__ void __launch_bounds__(FG_FORCE_THREADS, FG_FORCE_CTAS) k_forces_sear
                             }
 #pragma unroll
                             for (int u = 0; u < 2; u++) {
-                                const float x = __shfl_sync(FG_FULL, r[0], 16 * u), y = __shfl_sync(FG_FULL, r[1], 16 * u),
-                                            z = __shfl_sync(FG_FULL, r[2], 16 * u);
+                                const float x = __shfl_sync(FG_FULL, r[0], 16 * u);
+                                const float y = __shfl_sync(FG_FULL, r[1], 16 * u);
+                                const float z = __shfl_sync(FG_FULL, r[2], 16 * u);
                                 if ((int)lane == t[u] && (u == 0 || two)) {
                                     fx = __fadd_rn(fx, x);
                                     fy = __fadd_rn(fy, y);
@@ -970,8 +977,8 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
         const uint32_t range = stage_range(L.nwork), warps = (L.n + range - 1u) / range;
         const uint32_t ctas = grid_for((warps + FG_FORCE_THREADS / 32u - 1u) / (FG_FORCE_THREADS / 32u), 128);
         uint32_t most;
-        const int dispersed = dispersed_ranges(L, range, most);
-        const SideLaunch side(L, dispersed == DISPERSED_ASIDE);
+        int dispersed = dispersed_ranges(L, range, most);
+        const SideLaunch side(L, dispersed);
         if (side.use)
             k_forces_dispersed<<<grid_for(L.nwork, FG_WALK_FORCE_CTAS), FG_CHUNK, 0, L.side.stream>>>(
                 L.n, *L.single, most, spos, svel, dp, start, end, ids, out.vel, out.pos, R, mass_o, visc_o);
