@@ -93,6 +93,8 @@ World::~World()
     if (ev_io_fork) cudaEventDestroy(ev_io_fork);
     if (ev_vel_in) cudaEventDestroy(ev_vel_in);
     if (ev_pos_in) cudaEventDestroy(ev_pos_in);
+    if (ev_spread) cudaEventDestroy(ev_spread);
+    cudaFreeHost(spread_h);
     if (ev_walk) cudaEventDestroy(ev_walk);
     if (ev_walk_done) cudaEventDestroy(ev_walk_done);
     if (stream2) cudaStreamDestroy(stream2);
@@ -573,6 +575,8 @@ int World::init_stream(cudaStream_t st)
     CK(cudaEventCreateWithFlags(&ev_vel_in, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_pos_in, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_walk, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ev_spread, cudaEventDisableTiming));
+    CK(cudaHostAlloc((void **)&spread_h, 8, cudaHostAllocDefault));
     CK(cudaEventCreateWithFlags(&ev_walk_done, cudaEventDisableTiming));
     return FG_OK;
 }
@@ -963,7 +967,7 @@ uint64_t World::graph_signature() const
     const bool ordered = use_order && order_valid;
     return (uint64_t)(stages & 0xffu) | (fused_integrate ? 0x100ull : 0ull) | ((uint64_t)(digit_bits & 0xfu) << 9) |
            (use_list ? 1ull << 16 : 0ull) | (ordered ? 1ull << 17 : 0ull) | (use_cc ? 1ull << 18 : 0ull) |
-           ((ordered && order_forces_only) ? 1ull << 19 : 0ull) | ((uint64_t)(ctas_per_sm & 0x7fu) << 20) |
+           ((uint64_t)(ctas_per_sm & 0x7fu) << 20) |
            (one_pass_sort ? 1ull << 27 : 0ull) | (bucket_sort_on ? 1ull << 28 : 0ull) |
            ((uint64_t)((block >> 6) & 0x7u) << 29) | ((uint64_t)(cc_warps & 0x7u) << 32) |
            (density_walks ? 1ull << 35 : 0ull) |
@@ -1073,7 +1077,7 @@ void World::tune_begin()
         for (int k = 0; k < 3; k++)
             if (tune_kernels & (1u << k)) tr.cand[tr.ncand++] = k;
     } else if (tr.dim == 1) {
-        /* CTAs per SM of the 128-thread density/force grids */
+        /* CTAs per SM of the density/force grids, in CTAs of 128 threads */
         const int v[3] = {16, 32, 64};
         for (int k = 0; k < 3; k++) tr.cand[tr.ncand++] = v[k];
     } else if (tr.dim == 2) {
@@ -1085,7 +1089,7 @@ void World::tune_begin()
         tr.cand[tr.ncand++] = 1;
         if (bucket_sort_fits()) tr.cand[tr.ncand++] = 2;
     } else if (tr.dim == 4) {
-        /* threads per CTA of the density/force grids */
+        /* threads per CTA of the force grid */
         const int v[3] = {64, 128, 256};
         for (int k = 0; k < 3; k++) tr.cand[tr.ncand++] = v[k];
     } else {
@@ -1153,6 +1157,8 @@ int World::tune_finish()
  * 91 and 51 us, 100 of 3,000 splashed (7.7) 177 and 179, 50 of 10,000 (6.6) 296
  * and 281, 30 uneven ones (6.3) 298 and 322, 1M of a lattice (5.2) 603 and 690;
  * 1,048,576 random particles 0.65 h apart 562 and 494, 1.2 h 550 and 367. */
+static bool walks_pay(const uint32_t spread[2]) { return 2ull * spread[0] > 15ull * spread[1]; }
+
 int World::check_list_cap()
 {
     const bool grow = step_count % FG_LIST_CHECK_PERIOD == 0;
@@ -1161,7 +1167,7 @@ int World::check_list_cap()
     if (density_ranges_wide(nwork)) launch_spread(fluid_launch(), spos, max_count + 2);
     CK(cudaMemcpyAsync(seen, max_count, sizeof(seen), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    density_walks = 2ull * seen[2] > 15ull * seen[3];
+    density_walks = walks_pay(seen + 2);
     if (!grow) return FG_OK;
     CK(cudaMemsetAsync(max_count, 0, 4, stream));
     const uint32_t mx = seen[0];
@@ -1169,6 +1175,26 @@ int World::check_list_cap()
     const uint32_t want = std::min<uint32_t>(((mx + mx / 8u) + 31u) & ~31u, FG_LIST_CAP_MAX);
     if (want <= list_cap) return FG_OK;
     return set_list_cap(want);
+}
+
+/* The same choice for a world without those checks (a capacity that was set, a
+ * server's): the count comes back while the steps go on, and takes effect at
+ * the first step that finds it. */
+int World::watch_spread()
+{
+    if (!use_list || list_autogrow || !density_ranges_wide(nwork)) return FG_OK;
+    if (spread_pending && cudaEventQuery(ev_spread) == cudaSuccess) {
+        spread_pending = false;
+        density_walks = walks_pay(spread_h);
+    }
+    if (spread_pending || step_count < spread_next) return FG_OK;
+    CK(cudaMemsetAsync(max_count + 2, 0, 8, stream));
+    launch_spread(fluid_launch(), spos, max_count + 2);
+    CK(cudaMemcpyAsync(spread_h, max_count + 2, 8, cudaMemcpyDeviceToHost, stream));
+    CK(cudaEventRecord(ev_spread, stream));
+    spread_pending = true;
+    spread_next = step_count + FG_LIST_CHECK_PERIOD;
+    return FG_OK;
 }
 
 /* Whether step s starts by that check, the one for dispersed ranges also after
@@ -1236,6 +1262,7 @@ int World::step(uint32_t nsteps, const StepIO *io)
 int World::step_loop(uint32_t nsteps)
 {
     for (uint32_t k = 0; k < nsteps; k++) {
+        if (const int r = watch_spread(); r != FG_OK) return r;
         const uint32_t span = graph_span(nsteps - k);
         if (span > 1) {
             /* several steps in one captured graph */
@@ -1953,7 +1980,7 @@ int fg_world_set_option(fg_world *w, int option, int value)
     case FG_OPT_TARGET_ORDER:
         if (value < 0 || value > 2) return FG_E_INVALID;
         W->use_order = value != 0;
-        W->order_forces_only = value == 2;
+        if (value) W->order_option = value;
         return FG_OK;
     case FG_OPT_ORDER_PERIOD:
         if (value < 0) return FG_E_INVALID;
@@ -2057,7 +2084,7 @@ int fg_world_get_option(const fg_world *w, int option, int *value)
     const World *W = (const World *)w;
     switch (option) {
     case FG_OPT_NEIGHBOR_LIST: *value = W->use_list ? 1 : 0; return FG_OK;
-    case FG_OPT_TARGET_ORDER: *value = W->use_order ? (W->order_forces_only ? 2 : 1) : 0; return FG_OK;
+    case FG_OPT_TARGET_ORDER: *value = W->use_order ? W->order_option : 0; return FG_OK;
     case FG_OPT_ORDER_PERIOD: *value = (int)W->order_period; return FG_OK;
     case FG_OPT_DIGIT_BITS: *value = (int)W->digit_bits; return FG_OK;
     case FG_OPT_KERNEL: *value = W->current_kernel(); return FG_OK;

@@ -107,12 +107,12 @@ struct World {
     uint32_t *list_cap_d = nullptr; /* the same, in device memory for the kernels */
     uint32_t *inv = nullptr;  /* particle -> sorted index (written by the ranges pass) */
     uint32_t *tord = nullptr; /* spatial target order (particle ids, scene-contiguous) */
-    /* default: Morton target order in the force pass only (FG_OPT_TARGET_ORDER 2) */
+    /* default: Morton target order in the force pass */
     bool use_list = true, use_order = true;
-    bool order_forces_only = true;
+    int order_option = 2; /* FG_OPT_TARGET_ORDER as set: 1 and 2 are the same now */
     bool use_cc = false;       /* kernel 2: warp per bucket run, candidates staged in shared memory */
     uint32_t ctas_per_sm = 0;  /* CTAs per SM of the density/force grids (0 = 64) */
-    uint32_t block = 128;      /* kernels 0/1: threads per CTA of the density/force grids (64, 128, 256) */
+    uint32_t block = 128;      /* kernels 0/1: threads per CTA of the force grid (64, 128, 256) */
     uint32_t cc_warps = 4;     /* kernel 2: bucket runs (warps) per CTA (1, 2, 4) */
     int set_list_cap(uint32_t cap);
     uint32_t *runs = nullptr;  /* occupied-bucket run heads */
@@ -154,6 +154,11 @@ struct World {
     cudaStream_t stream3 = nullptr; /* velocity upload of an end-to-end step; the dispersed ranges of a pass without lists */
     cudaEvent_t ev_walk = nullptr, ev_walk_done = nullptr;
     bool density_walks = false; /* the density pass with lists walks by thread (check_list_cap) */
+    cudaEvent_t ev_spread = nullptr;
+    uint32_t *spread_h = nullptr; /* what a world without those checks counted, on its way */
+    bool spread_pending = false;
+    uint64_t spread_next = 1;
+    int watch_spread();
     cudaEvent_t ev_io_fork = nullptr, ev_vel_in = nullptr, ev_pos_in = nullptr;
     void enqueue_rb_grid(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches);
     void enqueue_rb_contact(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches, bool with_fluid);

@@ -211,14 +211,18 @@ int fg_world_set_graphs(fg_world *w, int on);
  *                         nothing but the limit; setting it turns
  *                         FG_OPT_LIST_AUTOGROW off)
  *   FG_OPT_LIST_AUTOGROW  kernel 1: 1 = every 25 steps grow the capacity to
- *                         1.125x the largest in-range count seen (default)
+ *                         1.125x the largest in-range count seen (default).
+ *                         The same check, and one after the first step, sees
+ *                         whether the particles share cells, and chooses the
+ *                         density pass's form by it (without the option, as
+ *                         soon as a count of its own has come back)
  *   FG_OPT_GRAPH_STEPS    steps captured in one CUDA graph launch (1..64,
  *                         default 1; until it is set, small worlds join up
  *                         to four steps of one call once their step has been
  *                         replayed a while); such a launch never spans an
  *                         autotuning round or a list capacity check
- *   FG_OPT_CTAS_PER_SM    kernels 0/1: CTAs per SM of the persistent
- *                         128-thread density/force grids (0 = 64; the
+ *   FG_OPT_CTAS_PER_SM    kernels 0/1: CTAs per SM of the density/force
+ *                         grids, in CTAs of 128 threads (0 = 64; the
  *                         autotuner tries 16, 32 and 64)
  *   FG_OPT_AUTOTUNE_TILES bit mask of the tunables the autotuner varies:
  *                         1 = CTAs per SM, 2 = radix digit width, 4 = the
