@@ -76,6 +76,40 @@ int World::alloc(void **p, size_t bytes)
     return FG_OK;
 }
 
+/* Eight-byte slots of one page-locked page, which any world may take: locking
+ * memory takes 0.8 ms, which a process with a world pays once.  The page goes
+ * with the last slot. */
+struct HostSlots {
+    std::mutex mu;
+    uint32_t *page = nullptr;
+    uint64_t used[8] = {}; /* a bit a slot */
+    uint32_t *take()
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!page && cudaHostAlloc((void **)&page, 4096, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            page = nullptr;
+        }
+        for (int k = 0; page && k < 512; k++)
+            if (!(used[k / 64] >> (k % 64) & 1u)) {
+                used[k / 64] |= 1ull << (k % 64);
+                return page + 2 * k;
+            }
+        return nullptr;
+    }
+    void give(uint32_t *slot)
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const size_t k = (size_t)(slot - page) / 2;
+        used[k / 64] &= ~(1ull << (k % 64));
+        for (uint64_t u : used)
+            if (u) return;
+        cudaFreeHost(page);
+        page = nullptr;
+    }
+};
+static HostSlots host_slots;
+
 World::~World()
 {
     if (flush_buf) cudaFree(flush_buf);
@@ -94,7 +128,7 @@ World::~World()
     if (ev_vel_in) cudaEventDestroy(ev_vel_in);
     if (ev_pos_in) cudaEventDestroy(ev_pos_in);
     if (ev_spread) cudaEventDestroy(ev_spread);
-    cudaFreeHost(spread_h);
+    if (spread_h) host_slots.give(spread_h); /* no copy under way: freeing the arrays waited for the device */
     if (ev_walk) cudaEventDestroy(ev_walk);
     if (ev_walk_done) cudaEventDestroy(ev_walk_done);
     if (stream2) cudaStreamDestroy(stream2);
@@ -576,7 +610,6 @@ int World::init_stream(cudaStream_t st)
     CK(cudaEventCreateWithFlags(&ev_pos_in, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_walk, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_spread, cudaEventDisableTiming));
-    CK(cudaHostAlloc((void **)&spread_h, 8, cudaHostAllocDefault));
     CK(cudaEventCreateWithFlags(&ev_walk_done, cudaEventDisableTiming));
     return FG_OK;
 }
@@ -1152,23 +1185,26 @@ int World::tune_finish()
  * capacity to 1.125x the largest in-range count seen since the last check,
  * so the force pass walks lists instead of buckets as a scene compresses; and
  * choose between the density pass's forms for the steps to come: staged, or
- * walked by thread where the ranges of 32 targets lie in more than 7.5 buckets
- * in the mean.  Steps, staged and walked: 1,000 scenes of 100 particles (12.6)
- * 91 and 51 us, 100 of 3,000 splashed (7.7) 177 and 179, 50 of 10,000 (6.6) 296
- * and 281, 30 uneven ones (6.3) 298 and 322, 1M of a lattice (5.2) 603 and 690;
- * 1,048,576 random particles 0.65 h apart 562 and 494, 1.2 h 550 and 367. */
-static bool walks_pay(const uint32_t spread[2]) { return 2ull * spread[0] > 15ull * spread[1]; }
+ * walked by thread where the ranges of 32 targets lie in more than nine buckets
+ * in the mean.  Steps, staged and walked: 1,000 scenes of 100 particles (12) 74
+ * and 48 us, 300 of 1,000 (9.5) 146 and 133, 100 of 3,000 that splash (10.7) 173
+ * and 180, 50 of 10,000 (8.5) 292 and 300, 20 of 30,000 (7.5) 365 and 425, 1M
+ * of a dam break (5.4) 947 and 1362; 1,048,576 random particles 0.8 h apart (14)
+ * 532 and 427, 1.7 h 609 and 372. */
+static bool walks_pay(const uint32_t spread[2]) { return spread[0] > 9ull * spread[1]; }
 
 int World::check_list_cap()
 {
-    const bool grow = step_count % FG_LIST_CHECK_PERIOD == 0;
     uint32_t seen[4]; /* largest count, the capacity, buckets and number of the ranges counted */
     CK(cudaMemsetAsync(max_count + 2, 0, 8, stream));
-    if (density_ranges_wide(nwork)) launch_spread(fluid_launch(), spos, max_count + 2);
+    if (density_ranges_wide(nwork)) {
+        launch_spread(fluid_launch(), spos, max_count + 2);
+        kernels_enqueued++;
+    }
     CK(cudaMemcpyAsync(seen, max_count, sizeof(seen), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     density_walks = walks_pay(seen + 2);
-    if (!grow) return FG_OK;
+    spread_pending = false; /* an older count */
     CK(cudaMemsetAsync(max_count, 0, 4, stream));
     const uint32_t mx = seen[0];
     if (mx <= list_cap) return FG_OK;
@@ -1177,31 +1213,57 @@ int World::check_list_cap()
     return set_list_cap(want);
 }
 
-/* The same choice for a world without those checks (a capacity that was set, a
- * server's): the count comes back while the steps go on, and takes effect at
- * the first step that finds it. */
-int World::watch_spread()
+/* The same choice after the first step, and for a world without those checks (a
+ * capacity that was set, a server's) every FG_LIST_CHECK_PERIOD steps: the
+ * ranges of a step just enqueued are counted, the count comes back while the
+ * steps go on, and the first step that finds it takes it up.  Both forms give
+ * the same bits, so it need not be the same step each time.  (A capture, of the
+ * caller's on this stream or another, is left alone: nothing is counted into
+ * it, and it doesn't bar the query.) */
+void World::poll_spread()
 {
-    if (!use_list || list_autogrow || !density_ranges_wide(nwork)) return FG_OK;
-    if (spread_pending && cudaEventQuery(ev_spread) == cudaSuccess) {
-        spread_pending = false;
-        density_walks = walks_pay(spread_h);
+    if (!spread_pending) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaEventQuery(ev_spread);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaErrorNotReady) cudaGetLastError(); /* no error */
+    if (e != cudaSuccess) return;
+    spread_pending = false;
+    density_walks = walks_pay(spread_h);
+}
+
+int World::count_spread()
+{
+    if (spread_pending || step_count < spread_next || !use_list || !density_ranges_wide(nwork)) return FG_OK;
+    if (list_autogrow && spread_next > 1u) return FG_OK; /* the checks count from here on */
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        return FG_OK;
     }
-    if (spread_pending || step_count < spread_next) return FG_OK;
+    if (cs != cudaStreamCaptureStatusNone) return FG_OK;
+    spread_next = step_count + FG_LIST_CHECK_PERIOD;
+    if (!spread_h) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        spread_h = host_slots.take();
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!spread_h) return FG_OK;
+    }
     CK(cudaMemsetAsync(max_count + 2, 0, 8, stream));
     launch_spread(fluid_launch(), spos, max_count + 2);
+    kernels_enqueued++;
     CK(cudaMemcpyAsync(spread_h, max_count + 2, 8, cudaMemcpyDeviceToHost, stream));
     CK(cudaEventRecord(ev_spread, stream));
     spread_pending = true;
-    spread_next = step_count + FG_LIST_CHECK_PERIOD;
     return FG_OK;
 }
 
-/* Whether step s starts by that check, the one for dispersed ranges also after
- * the first step. */
+/* Whether step s starts by that check. */
 bool World::list_check_due(uint64_t s) const
 {
-    return use_list && list_autogrow && s && (s % FG_LIST_CHECK_PERIOD == 0 || (s == 1 && density_ranges_wide(nwork)));
+    return use_list && list_autogrow && s && s % FG_LIST_CHECK_PERIOD == 0;
 }
 
 /* Whether step s starts by refreshing the Morton target order. */
@@ -1262,7 +1324,7 @@ int World::step(uint32_t nsteps, const StepIO *io)
 int World::step_loop(uint32_t nsteps)
 {
     for (uint32_t k = 0; k < nsteps; k++) {
-        if (const int r = watch_spread(); r != FG_OK) return r;
+        poll_spread();
         const uint32_t span = graph_span(nsteps - k);
         if (span > 1) {
             /* several steps in one captured graph */
@@ -1275,6 +1337,7 @@ int World::step_loop(uint32_t nsteps)
             tune_count[current_kernel()] += span;
             counted_steps += span;
             step_count += span;
+            if ((r = count_spread()) != FG_OK) return r;
             k += span - 1;
             continue;
         }
@@ -1309,6 +1372,7 @@ int World::step_loop(uint32_t nsteps)
         tune_count[kused]++;
         counted_steps++;
         step_count++;
+        if (const int r = count_spread(); r != FG_OK) return r;
     }
     cudaError_t e = cudaPeekAtLastError();
     if (e != cudaSuccess) {

@@ -155,10 +155,11 @@ struct World {
     cudaEvent_t ev_walk = nullptr, ev_walk_done = nullptr;
     bool density_walks = false; /* the density pass with lists walks by thread (check_list_cap) */
     cudaEvent_t ev_spread = nullptr;
-    uint32_t *spread_h = nullptr; /* what a world without those checks counted, on its way */
+    uint32_t *spread_h = nullptr; /* what was counted, on its way to the host */
     bool spread_pending = false;
-    uint64_t spread_next = 1;
-    int watch_spread();
+    uint64_t spread_next = 1; /* steps after which to count */
+    void poll_spread();
+    int count_spread();
     cudaEvent_t ev_io_fork = nullptr, ev_vel_in = nullptr, ev_pos_in = nullptr;
     void enqueue_rb_grid(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches);
     void enqueue_rb_contact(cudaStream_t st, cudaEvent_t *ev, uint32_t &launches, bool with_fluid);

@@ -128,10 +128,11 @@ __device__ __forceinline__ F2 fg_mul2(F2 a, F2 b)
  * candidates with l <= h (an exact 0 at l = h, so the sum equals the
  * reference's l < h sum) and the force pass's neighbour list (every visit
  * with l <= h, the target's own entries included, which the force pass
- * skips), stored two entries (8 bytes) at a time.  Every addition's rounding
- * error is collected beside the sum; a candidate out of range adds an exact 0
- * to both.  So the result depends on the in-range candidates and their order
- * alone: however they are found, a target gets the same bits. */
+ * skips), stored two entries (8 bytes) at a time.  An addition's rounding
+ * error is collected beside the sum (all of it while the sum is the larger
+ * operand); a candidate out of range adds an exact 0 to both.  So the result
+ * depends on the in-range candidates and their order alone: however they are
+ * found, a target gets the same bits. */
 struct DensityAcc {
     float s, c;      /* sum and compensation */
     uint32_t cnt;    /* in-range visits, the list's entries */

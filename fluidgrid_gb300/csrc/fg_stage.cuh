@@ -115,13 +115,14 @@ __device__ __forceinline__ StageCell fg_stage_cell(float4 p, const StageGrid &G)
     return c;
 }
 
-/* Buckets of a range of 32 targets, a lane each (past the scene's end its last
- * one's); cells of a shorter one (len < 32), which saves the modulo.  Buckets,
- * not cells: where many cells share a bucket, the candidates are many too. */
+/* Buckets of a range of len targets, a lane each (past the scene's end its last
+ * one's); cells of a shorter one where a bucket takes a modulo.  Buckets, not
+ * cells: where many cells share a bucket, the candidates are many too. */
 __device__ __forceinline__ uint32_t fg_stage_buckets(const StageCell &c, const StageGrid &G, uint32_t len)
 {
     uint32_t b = (uint32_t)c.x * FG_PX ^ (uint32_t)c.y * FG_PY ^ (uint32_t)c.z * FG_PZ;
-    if (len == 32u) b = G.mask ? b & G.mask : b % G.nb;
+    if (G.mask) b &= G.mask;
+    else if (len == 32u) b %= G.nb;
     const uint32_t lane = threadIdx.x & 31u, before = __shfl_up_sync(FG_FULL, b, 1);
     return (uint32_t)__popc(__ballot_sync(FG_FULL, lane < len && (lane == 0u || b != before)));
 }
