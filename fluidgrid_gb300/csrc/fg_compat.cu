@@ -132,8 +132,10 @@ void sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t bits, uint32_t n)
 {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!n) { g_status = FG_OK; return; }
-    int r = ensure_sort(n);
-    if (r != FG_OK) { g_status = r; return; }
+    if (!fg::radix_one_launch((uint32_t)n)) { /* that sorts in shared memory */
+        int r = ensure_sort(n);
+        if (r != FG_OK) { g_status = r; return; }
+    }
     fg::RadixScratch rs{g_sort.k, g_sort.v, g_sort.h};
     fg::radix_sort(keys, vals, keys, vals, n, bits, 8, rs, 0);
     finish();
