@@ -856,7 +856,7 @@ uint32_t World::enqueue_step(cudaEvent_t *ev)
     /* end-to-end step: the positions upload first, then the velocities on a
      * third stream while the hash and sort run; the reorder waits for them
      * (one direction of the link carries one copy at a time: with the
-     * velocities first, the hash waited for both, 372 against 352 us a step
+     * velocities first, the hash waited for both, 368 against 347 us a step
      * at 262,144 particles) */
     const size_t iob = 16 * (size_t)n;
     if (cur_io && iob) {
@@ -981,7 +981,7 @@ uint32_t World::enqueue_step(cudaEvent_t *ev)
     return launches;
 }
 
-/* Spatial target order from the current particle positions: Morton keys of
+/* Target order of the force pass from the current particle positions: Morton keys of
  * the unsorted particles, stable sort by key with particle ids as values.
  * The sorted-key buffers of the step are free here (the step rewrites them
  * before reading), so they serve as key scratch. */
@@ -1090,8 +1090,9 @@ int World::graph_for_current(cudaGraphExec_t *out, uint32_t nsteps)
 }
 
 /* Autotuning round: the candidate values of one tunable (rotating among the
- * kernel, the CTAs per SM of the density/force grids and the radix digit
- * width) each run one real step between CUDA events -- the state advances as
+ * kernel, the CTAs per SM of the density/force grids, the radix digit width
+ * where it counts, the sort variant, the CTA size of the force grid and kernel
+ * 2's runs a CTA) each run one real step between CUDA events -- the state advances as
  * in any step -- and the fastest value is kept.  A round may span several
  * step() calls. */
 void World::tune_begin()

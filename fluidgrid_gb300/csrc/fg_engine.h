@@ -106,7 +106,7 @@ struct World {
     uint32_t list_cap = 0;       /* entries a particle may store (<= list_cap_alloc) */
     uint32_t *list_cap_d = nullptr; /* the same, in device memory for the kernels */
     uint32_t *inv = nullptr;  /* particle -> sorted index (written by the ranges pass) */
-    uint32_t *tord = nullptr; /* spatial target order (particle ids, scene-contiguous) */
+    uint32_t *tord = nullptr; /* the force pass's target order (particle ids, scene-contiguous) */
     /* default: Morton target order in the force pass */
     bool use_list = true, use_order = true;
     int order_option = 2; /* FG_OPT_TARGET_ORDER as set: 1 and 2 are the same now */
@@ -151,7 +151,8 @@ struct World {
     bool own_stream = false;
     cudaStream_t stream2 = nullptr; /* rigid-body branch of a full step */
     cudaEvent_t ev_fork = nullptr, ev_fluid_ready = nullptr, ev_rb_done = nullptr, ev_bodies_done = nullptr;
-    cudaStream_t stream3 = nullptr; /* velocity upload of an end-to-end step; the dispersed ranges of a pass without lists */
+    /* velocity upload of an end-to-end step; the dispersed ranges of a pass without lists */
+    cudaStream_t stream3 = nullptr;
     cudaEvent_t ev_walk = nullptr, ev_walk_done = nullptr;
     bool density_walks = false; /* the density pass with lists walks by thread (check_list_cap) */
     cudaEvent_t ev_spread = nullptr;

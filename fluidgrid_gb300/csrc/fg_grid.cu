@@ -1204,12 +1204,13 @@ void launch_cell_ranges(const uint32_t *keys, const uint32_t *ids, const float4 
 }
 
 /* ------------------------------------------------ spatial target order
- * Density and force kernels process their targets in a spatially coherent
- * order so that a CTA's particles share neighbour cells and the neighbour
- * loads hit L1 (the hashed bucket order scatters a CTA over random cells).
- * The key is the scene id above a Morton code of the particle's cell,
- * counted from the scene's volume_min and clamped to 2^bits cells per axis;
- * a particle outside that range only loses locality, never correctness. */
+ * The force kernels process their targets in a spatially coherent order so
+ * that a CTA's particles share listed neighbours and their loads hit L1 (the
+ * hashed bucket order scatters a CTA over random cells); the density pass
+ * stages by cell, in bucket order.  The key is the scene id above a Morton
+ * code of the particle's cell, counted from that of the scene's volume_min and
+ * clamped to 2^bits cells per axis; a particle outside that range only loses
+ * locality, never correctness. */
 __device__ __forceinline__ uint32_t fg_spread3(uint32_t v)
 {
     v &= 0x3ffu;

@@ -120,7 +120,8 @@ void launch_morton_keys(const Launch &L, const float4 *pos, uint32_t *keys, uint
 
 
 /* Target order of the force pass: target slot t processes the particle tord[t]
- * (a particle id, scene-contiguous), found in sorted order at inv[tord[t]].  tord == nullptr: slot t is sorted index t. */
+ * (a particle id, scene-contiguous), found in sorted order at inv[tord[t]].
+ * tord == nullptr: slot t is sorted index t. */
 struct TargetOrder {
     const uint32_t *tord;
     const uint32_t *inv;

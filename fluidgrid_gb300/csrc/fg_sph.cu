@@ -1018,9 +1018,10 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * diverging from its neighbours', takes as long as dozens of searches by
  * warp.  The CTA's eight warps share the searches of its 128 particles, which
  * ids along a surface may all need.  4M particles, eight bodies whose AABB is
- * the whole scene: 1007 -> 151 us (a lane each inside the AABB -> here; a lane
- * each in marked cells only: 399; a warp per eight particles: 235).  The force
- * pass adds the stored sum where it would add the walked one: the same bits.
+ * the whole scene: 1007 -> 151 us by itself (a lane each inside the AABB ->
+ * here; a lane each in marked cells only: 399; a warp per eight particles:
+ * 235), some 230 beside the density pass.  The force pass adds the stored sum
+ * where it would add the walked one: the same bits.
  * The launchers' pass goes over sorted particles and stores by id; within the
  * force search, whose shared memory leaves the bucket tables no L1, the same
  * searches took twice the time and more (262,144 particles: 4,096 spheres all
