@@ -362,7 +362,8 @@ void gSPHCalculateForcesWithSRB(float4 *oldPositions, float4 *oldVelocity, float
     /* one grid's contact ahead, each particle's in its place of the output */
     if (useDynamicRB || useStaticRB) {
         fg::RigidGrid &grid = useDynamicRB ? dyn : sta;
-        fg::launch_fluid_contact(L, oldPositions, oldVelocity, grid, newVel, fg::contact_narrow(S.f2r_rel), particleId);
+        const bool may_walk = fg::contact_may_walk(S.f2r_rel, 0u, numParticles); /* the spheres' number is not told */
+        fg::launch_fluid_contact(L, oldPositions, oldVelocity, grid, newVel, may_walk, particleId);
         grid.pre = newVel;
     }
     fg::launch_forces(L, oldPositions, oldVelocity, density_pressure, gridStart, gridEnd, particleId, o,

@@ -753,9 +753,9 @@ void World::enqueue_fluid_contact(cudaStream_t st, uint32_t &launches)
     if (!fluid_contact_pass()) return;
     Launch Lf = fluid_launch();
     Lf.stream = st;
-    bool narrow = false; /* some scene's search */
-    for (const FgScene &S : scenes_h) narrow |= S.nbodies && contact_narrow(S.f2r_rel);
-    launch_fluid_contact(Lf, pos, vel, body_grid(), fcontact, narrow);
+    bool may_walk = false; /* some scene's contact */
+    for (const FgScene &S : scenes_h) may_walk |= S.nbodies && contact_may_walk(S.f2r_rel, S.nsph, S.n);
+    launch_fluid_contact(Lf, pos, vel, body_grid(), fcontact, may_walk);
     launches++;
 }
 
@@ -1191,7 +1191,8 @@ int World::tune_finish()
  * and 48 us, 300 of 1,000 (9.5) 146 and 133, 100 of 3,000 that splash (10.7) 173
  * and 180, 50 of 10,000 (8.5) 292 and 300, 20 of 30,000 (7.5) 365 and 425, 1M
  * of a dam break (5.4) 947 and 1362; 1,048,576 random particles 0.8 h apart (14)
- * 532 and 427, 1.7 h 609 and 372. */
+ * 532 and 427, 1.7 h 609 and 372.  With eight buckets, 200,000 random particles
+ * 0.5 h apart took 155 instead of 149. */
 static bool walks_pay(const uint32_t spread[2]) { return spread[0] > 9ull * spread[1]; }
 
 int World::check_list_cap()

@@ -197,9 +197,9 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * (ProcessCollisionForcesD).  The force pass then
  * reads it (G.pre). */
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out,
-                          bool narrow, const uint32_t *ids = nullptr);
-/* whether a search half-width is one of up to 27 buckets */
-bool contact_narrow(const int rel[3]);
+                          bool may_walk, const uint32_t *ids = nullptr);
+/* whether the pass may walk by thread at a search half-width (0 spheres: not known) */
+bool contact_may_walk(const int rel[3], uint32_t spheres, uint32_t particles);
 
 void launch_integrate(const Launch &L, float4 *pos, const float4 *vel);
 

@@ -43,7 +43,7 @@ namespace fg {
  * (cells of 8 to 27 targets fill a warp badly) 138 -> 136 -> 126; 16,384, where
  * a thread's chain of 216 candidate loads was the pass, 37 -> 14.  64 worlds of
  * 1.23M particles that have splashed apart, whose warps lie in more and smaller
- * groups: 379 -> 378 after 20 steps, 504 -> 521 after 400 (a warp of more than
+ * groups: 379 -> 378 after 20 steps, 504 -> 511 after 400 (a warp of more than
  * nine groups walking by thread instead: 415 and 547).
  *
  * Staged candidates of a warp: its targets lie in four or five groups of some
@@ -770,10 +770,10 @@ __global__ void __launch_bounds__(BLOCK, 768 / BLOCK) k_forces_walk(
  * thread and drained together, 1923: lanes of a cell lose the loads that they
  * share while they walk in step.  Hits taken by a lane per target, 1268: their
  * numbers differ by lane and round.)  Dispersed ranges walk by thread: in
- * k_forces_dispersed, or here where a warp has fewer than 32 targets.  192 staged candidates leave twelve CTAs
- * an SM: 256, 991 us; 128, 1073.  The rigid contact follows by warp, for the
- * particles in cells marked near a sphere, where both grids are given: else it
- * is read from the contact pass. */
+ * k_forces_dispersed, or here where a warp has fewer than 32 targets.  192
+ * staged candidates leave twelve CTAs an SM: 256, 991 us; 128, 1073.  The rigid
+ * contact follows by warp, for the particles in cells marked near a sphere,
+ * where both grids are given: else it is read from the contact pass. */
 #define FG_FORCE_STAGE 192u
 #define FG_FORCE_CTAS 12
 #define FG_FORCE_THREADS 64u
@@ -1029,14 +1029,24 @@ void launch_forces(const Launch &L, const float4 *spos, const float4 *svel, cons
  * 4, half as many particles, 2584 -> 987; four bodies' surfaces, the whole
  * two-way pass, 488 -> 439). */
 #define FG_CONTACT_THREADS 256u
-/* Searches of a CTA beyond which the 27 buckets of a half-width of 1, which
- * leave most of a warp's lanes idle, are walked by thread: a step of 131,072
- * particles with 4,096 spheres among all of them 209 -> 170 us, 32,768 spheres
- * 272 -> 240; surfaces stay below it.  (Half-widths of 2 and more: 257 us walked
+/* Searches of a work item beyond which its particles walk by thread instead:
+ * the 27 buckets of a half-width of 1 leave most of a searching warp idle, and
+ * those of 3 and more are searched round by round.  Walking takes as long
+ * however many lanes of a CTA need it, and an SM its 128 threads an item: such a
+ * CTA takes two items, and walks or searches both (an item of each kind took as
+ * long as the two forms one after the other, 556 us).  A step of 131,072
+ * particles with spheres among 0.6, 0.8 and all of the width, searched -> by this
+ * rule: half-width 1, 169, 200, 231 -> 164, 162, 173 us; 3, 287, 455, 612 -> 287,
+ * 450, 454; 5, 836, 1548, 2196 -> 835, 1380, 1342.  (Half-width 2: 257 us walked
  * and 245 searched with 1,024 spheres, 437 and 353 with 32,768.)  Its registers
- * cost the other half-widths 3%, so they have a kernel without it. */
-#define FG_CONTACT_SEARCHES 80u
-template <bool WALK27>
+ * cost the other half-widths 3%, so they have a kernel without it; the choice
+ * of the output's index (IDS) made while it runs cost 3% too. */
+__host__ __device__ __forceinline__ uint32_t contact_searches(const int rel[3])
+{
+    const uint32_t total = (2u * rel[0] + 1u) * (2u * rel[1] + 1u) * (2u * rel[2] + 1u);
+    return total <= 27u ? 44u : total <= 216u ? FG_CHUNK : 72u;
+}
+template <bool WALKS, bool IDS>
 __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWork *__restrict__ work, uint32_t nwork,
                                                            uint32_t n_single, const FgScene *__restrict__ table,
                                                            const __grid_constant__ FgScene single,
@@ -1046,67 +1056,80 @@ __global__ void __launch_bounds__(FG_CONTACT_THREADS) k_fluid_contact(const FgWo
                                                            const uint32_t *__restrict__ ids,
                                                            float4 *__restrict__ out)
 {
-    __shared__ uint32_t s_id[FG_CHUNK], s_n;
+    constexpr uint32_t ITEMS = WALKS ? FG_CONTACT_THREADS / FG_CHUNK : 1u; /* at a time */
+    __shared__ uint32_t s_id[ITEMS][FG_CHUNK], s_n[ITEMS];
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t w = blockIdx.x; w < nwork; w += gridDim.x) {
-        const FgWork it = fg_work(work, w, n_single);
+    const bool dynamic = G.body_vel != nullptr;
+    for (uint32_t w0 = ITEMS * blockIdx.x; w0 < nwork; w0 += ITEMS * gridDim.x) {
+        const uint32_t items = min(ITEMS, nwork - w0), h = threadIdx.x / FG_CHUNK, t = threadIdx.x % FG_CHUNK;
+        const FgWork it = fg_work(work, w0 + min(h, items - 1u), n_single);
         const FgScene *S = fg_scene(table, &single, it.scene);
-        if (!(S->flags & FG_SCENE_HAS_RB)) continue; /* uniform over the CTA */
-        if (threadIdx.x == 0) s_n = 0u;
+        uint32_t some = 0u, bodies = S->flags & FG_SCENE_HAS_RB; /* some: searches beyond which all are walked */
+        for (uint32_t q = 0; WALKS && q < items; q++) {
+            const FgScene *Q = fg_scene(table, &single, fg_work(work, w0 + q, n_single).scene);
+            bodies |= Q->flags & FG_SCENE_HAS_RB;
+            some += contact_searches(Q->f2r_rel);
+        }
+        if (!bodies) continue; /* uniform over the CTA */
+        if (threadIdx.x < ITEMS) s_n[threadIdx.x] = 0u;
         __syncthreads();
-        if (threadIdx.x < FG_CHUNK) {
-            const uint32_t id = it.first + threadIdx.x;
-            bool walk = false;
-            if (threadIdx.x < it.count) {
+        if (h < items) {
+            const uint32_t id = it.first + t;
+            bool near = false;
+            if (t < it.count && (S->flags & FG_SCENE_HAS_RB)) {
                 const float4 p = __ldg(pos + id);
-                walk = p.w > 0.0f && !fg_contact_outside(S, it.scene, p, G) && fg_contact_marked(S, it.scene, p, G);
+                near = p.w > 0.0f && !fg_contact_outside(S, it.scene, p, G) && fg_contact_marked(S, it.scene, p, G);
             }
-            const uint32_t m = __ballot_sync(0xffffffffu, walk);
+            const uint32_t m = __ballot_sync(0xffffffffu, near);
             uint32_t base = 0u;
-            if (lane == 0u && m) base = atomicAdd(&s_n, (uint32_t)__popc(m));
+            if (lane == 0u && m) base = atomicAdd(&s_n[h], (uint32_t)__popc(m));
             base = __shfl_sync(0xffffffffu, base, 0);
-            if (walk) s_id[base + __popc(m & ((1u << lane) - 1u))] = id;
+            if (near) s_id[h][base + __popc(m & ((1u << lane) - 1u))] = id;
         }
         __syncthreads();
-        const ContactShape C(S);
-        const bool dynamic = G.body_vel != nullptr;
-        if (WALK27 && C.total <= 27u && s_n > FG_CONTACT_SEARCHES) {
-            if (threadIdx.x < s_n) {
-                const uint32_t id = s_id[threadIdx.x];
+        if (WALKS && s_n[0] + s_n[ITEMS - 1u] > some) {
+            if (h < items && t < s_n[h]) {
+                const uint32_t id = s_id[h][t];
                 const float3 c = fg_fluid_rigid_contact(S, it.scene, __ldg(pos + id), __ldg(vel + id), G, dynamic);
-                out[ids ? __ldg(ids + id) : id] = make_float4(c.x, c.y, c.z, 0.0f);
+                out[IDS ? __ldg(ids + id) : id] = make_float4(c.x, c.y, c.z, 0.0f);
             }
             __syncthreads();
             continue;
         }
-        for (uint32_t k = threadIdx.x >> 5; k < s_n; k += FG_CONTACT_THREADS / 32u) {
-            const uint32_t id = s_id[k];
-            const float3 c = fg_contact_warp(S, C, __ldg(pos + id), __ldg(vel + id), G, dynamic);
-            if (lane == 0u) out[ids ? __ldg(ids + id) : id] = make_float4(c.x, c.y, c.z, 0.0f);
+        for (uint32_t q = 0; q < items; q++) {
+            const FgScene *Q = WALKS ? fg_scene(table, &single, fg_work(work, w0 + q, n_single).scene) : S;
+            const ContactShape C(Q);
+            for (uint32_t k = threadIdx.x >> 5; k < s_n[q]; k += FG_CONTACT_THREADS / 32u) {
+                const uint32_t id = s_id[q][k];
+                const float3 c = fg_contact_warp(Q, C, __ldg(pos + id), __ldg(vel + id), G, dynamic);
+                if (lane == 0u) out[IDS ? __ldg(ids + id) : id] = make_float4(c.x, c.y, c.z, 0.0f);
+            }
         }
         __syncthreads();
     }
 }
 
 void launch_fluid_contact(const Launch &L, const float4 *pos, const float4 *vel, const RigidGrid &G, float4 *out,
-                          bool narrow, const uint32_t *ids)
+                          bool may_walk, const uint32_t *ids)
 {
     if (!L.nwork) return;
     /* an SM's worth of CTAs: a CTA per item queues ahead of the grid kernels
      * beside this one (64 worlds after 400 steps 896 us a step, here 883; 4M
      * particles 2163, here 2135) */
-    const uint32_t g = grid_for(L.nwork, 8);
-    if (narrow)
-        k_fluid_contact<true><<<g, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos,
-                                                                      vel, G, ids, out);
-    else
-        k_fluid_contact<false><<<g, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos,
-                                                                       vel, G, ids, out);
+    const uint32_t g = grid_for(may_walk ? (L.nwork + 1u) / 2u : L.nwork, 8);
+    auto *k = ids ? (may_walk ? k_fluid_contact<true, true> : k_fluid_contact<false, true>)
+                  : (may_walk ? k_fluid_contact<true, false> : k_fluid_contact<false, false>);
+    k<<<g, FG_CONTACT_THREADS, 0, L.stream>>>(L.work, L.nwork, L.n, L.table, *L.single, pos, vel, G, ids, out);
 }
 
-bool contact_narrow(const int rel[3])
+/* Many spheres favour the search, which takes them a lane each: 65,536
+ * particles and a half-width of 8, a step with half as many spheres 4156 us
+ * searched and 6842 walked, with a sixteenth 6372 and 4406; 131,072 and a
+ * quarter 7381 and 6298. */
+bool contact_may_walk(const int rel[3], uint32_t spheres, uint32_t particles)
 {
-    return (2 * rel[0] + 1) * (2 * rel[1] + 1) * (2 * rel[2] + 1) <= 27;
+    const uint32_t searches = contact_searches(rel);
+    return searches < 64u || (searches < FG_CHUNK && spheres <= particles / 4u);
 }
 
 /* SPHIntegrateK (K_FluidSim.cu:418-438): pos += vel*(dt/scale) for active
